@@ -2,6 +2,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -11,6 +12,7 @@
 
 #include "dgc_gb300.h"
 #include "dgc_internal.hpp"
+#include "eo.hpp"
 #include "rhs_launch.cuh"
 
 namespace {
@@ -151,6 +153,23 @@ int upload_operators(dgc_handle_s* h, int form) {
   if (!h->d_mats32[form]) CK(cudaMalloc(&h->d_mats32[form], m32.size() * sizeof(float)));
   CK(cudaMemcpy(h->d_mats64[form], m64.data(), m64.size() * sizeof(double), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(h->d_mats32[form], m32.data(), m32.size() * sizeof(float), cudaMemcpyHostToDevice));
+  // even / odd form for the FP64 kernels: the weak operators of FP64 handles and
+  // the strong ones of laplace handles.  Operators without the reflection
+  // symmetry run the node-by-node kernels; NaN in its place then, so that a graph
+  // a caller captured with symmetric operators cannot quietly go on with those.
+  if (form == 0 ? h->prec == DGC_F64 : h->desc.physics == DGC_LAPLACE) {
+    const std::vector<double>* M = form == 1 ? &re.M : nullptr;
+    const std::vector<uint8_t> tab = dgc::eo_tables(re.N);
+    std::vector<double> eo = dgc::eo_pack(re.N, Dr, Ds, L, M);
+    h->eo_ok[form] = dgc::eo_symmetric(re.N, Dr, Ds, L, M);
+    if (!h->eo_ok[form]) std::fill(eo.begin(), eo.end(), std::nan(""));
+    const size_t nops = eo.size();
+    eo.resize(nops + tab.size() / sizeof(double));
+    std::memcpy(eo.data() + nops, tab.data(), tab.size());
+    if (!h->d_eo64[form]) CK(cudaMalloc(&h->d_eo64[form], eo.size() * sizeof(double)));
+    CK(cudaMemcpy(h->d_eo64[form], eo.data(), eo.size() * sizeof(double), cudaMemcpyHostToDevice));
+    h->d_eo_tab[form] = reinterpret_cast<const uint8_t*>(h->d_eo64[form] + nops);
+  }
   if (form == 0) {
     // register-blocked kernel operand: rows j of Dr^T, Ds^T (j < Np) and m of
     // LIFT^T (m < 3 Nfp), each padded with zeros to NpP columns
@@ -372,6 +391,7 @@ void device_free(dgc_handle_s* h) {
   for (int f = 0; f < 2; ++f) {
     cudaFree(h->d_mats64[f]);
     cudaFree(h->d_mats32[f]);
+    cudaFree(h->d_eo64[f]);
   }
   cudaFree(h->d_tc_b);
   cudaFree(h->d_blk_b);
@@ -456,6 +476,10 @@ extern "C" int dgc_set_operators(dgc_handle h, int form, const double* Dr, const
   (form == 0 ? re.Lw : re.Ls).assign(L, L + nl);
   CK(cudaDeviceSynchronize());
   const int rc = dgc::upload_operators(h, form);
+  if (h->graph_exec) {  // the kernel it captured depends on the operators' symmetry
+    cudaGraphExecDestroy(h->graph_exec);
+    h->graph_exec = nullptr;
+  }
   if (rc == DGC_OK) dgc::ipdg_operators_changed(h);
   return rc;
 }
@@ -512,6 +536,8 @@ dgk::RhsParams base_params(dgc_handle h) {
   p.nbr = reinterpret_cast<const int4*>(h->d_nbr);
   p.bxy = h->d_bxy;
   p.mats = h->prec == DGC_F64 ? h->d_mats64[0] : h->d_mats32[0];
+  p.mats_eo = h->prec == DGC_F64 && h->eo_ok[0] ? h->d_eo64[0] : nullptr;
+  p.tab_eo = h->d_eo_tab[0];
   p.mats_tc = h->prec == DGC_F32 ? h->d_tc_b : nullptr;
   p.mats_blk = h->prec == DGC_F32 ? h->d_blk_b : (h->prec == DGC_F32C ? h->d_blk_bs : nullptr);
   p.ax = h->desc.ax;

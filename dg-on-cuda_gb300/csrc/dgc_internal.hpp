@@ -31,6 +31,9 @@ struct dgc_handle_s {
   float* d_tau32 = nullptr;     // [K][4] laplace penalty, FP32
   void* d_mats64[2] = {nullptr, nullptr};  // weak, strong (transposed, padded)
   void* d_mats32[2] = {nullptr, nullptr};
+  double* d_eo64[2] = {nullptr, nullptr};  // the same, FP64, in the even / odd basis (eo.hpp), then its pair tables
+  bool eo_ok[2] = {false, false};          // the operators have the symmetry that basis needs
+  const uint8_t* d_eo_tab[2] = {nullptr, nullptr};
   void* d_tc_b = nullptr;     // FP32 tensor-core operand [Dr | Ds | LIFT] (strong form, split TF32)
   void* d_blk_b = nullptr;    // FP32 operand of the register-blocked kernel (weak form, rows padded to NpP)
   void* d_blk_bs = nullptr;   // the same rows in the strong form (compensated-state kernel, DGC_F32C)

@@ -1,0 +1,66 @@
+"""FP64 kernels in the even / odd basis of the reflection r <-> s against the
+oracle (every order, meshes smaller than a tile, with a ragged last tile and with
+many tiles), and the node-by-node kernels that operators without the symmetry
+still run."""
+import numpy as np
+import pytest
+import torch
+
+import dgc_gb300 as dg
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+# rounding: the oracle and the kernels sum the same O(N^2) terms in another order
+TOL = 1e-12
+PHYS = [("advection", oracle.ADVECTION), ("maxwell_tm", oracle.MAXWELL_TM), ("maxwell_te", oracle.MAXWELL_TE)]
+
+
+def rel(a, b):
+    return np.linalg.norm(np.ravel(a) - np.ravel(b)) / np.linalg.norm(np.ravel(b))
+
+
+@pytest.mark.parametrize("n", [1, 5, 23])
+@pytest.mark.parametrize("N", range(1, 9))
+def test_stage(N, n):
+    m = dg.meshes.jittered_square(n, seed=N)
+    o = oracle.Oracle(m.xy, m.cells, N)
+    rng = np.random.default_rng(N)
+    for name, kind in PHYS:
+        D = dg.Discretization(m, name, N, dg.F64, ax=-0.7, ay=0.4)
+        p = oracle.problem(kind, ax=-0.7, ay=0.4)
+        q0 = rng.standard_normal(D.Nf * D.K * D.Np)
+        q = D.upload(q0)
+        ref = o.rhs(p, 0.3, q0)
+        assert rel(D.download(D.rhs(q, 0.3)), ref) < TOL
+        for dt in (1e-3, -1e-3):  # the time step is folded into the face factors, whose sign picks the upwind side
+            qb, res = D.empty_state(), D.empty_state()
+            D.lserk4_stage(0, q, qb, res, 0.3, dt)
+            assert rel(D.download(res), dt * ref) < TOL
+        D.check()
+
+
+def test_operators_without_the_symmetry():
+    """The node-by-node kernels take over, and give the caller's operators."""
+    N = 4
+    m = dg.meshes.jittered_square(6, seed=2)
+    D = dg.Discretization(m, "advection", N, dg.F64, ax=0.8, ay=0.6, bc=dg.BC_ZERO)
+    q = D.upload(np.random.default_rng(0).standard_normal(D.K * D.Np))
+    base = D.download(D.rhs(q, 0.0))
+    Dr, Ds, L = (D.operator(w).copy() for w in (dg.OP_DR_WEAK, dg.OP_DS_WEAK, dg.OP_LIFT))
+    E = np.zeros_like(Dr)
+    E[3, 7] = 0.5
+    qa, qb, res = q.clone(), D.empty_state(), D.empty_state()
+    D.lserk4_run(qa, qb, res, 0.0, 1e-3, 4)  # a cached graph holds the symmetric kernel
+    D.set_operators(0, Dr + E, Ds, L)
+    got = D.download(D.rhs(q, 0.0))
+    # the change of the volume term: (ax rx + ay ry) E q
+    g, _, _ = dg.host_mesh(m, N)
+    qn = D.download(q).reshape(D.K, D.Np)
+    want = base.reshape(D.K, D.Np) + (0.8 * g[:, :1] + 0.6 * g[:, 1:2]) * (qn @ E.T)
+    assert rel(got, want) < TOL
+    a = D.lserk4_run(q.clone(), qb, res, 0.0, 1e-3, 4, graph=False).clone()
+    qa.copy_(q)
+    assert torch.equal(D.lserk4_run(qa, qb, res, 0.0, 1e-3, 4), a)
+    D.set_operators(0, Dr, Ds, L)
+    assert rel(D.download(D.rhs(q, 0.0)), base) < 1e-14
