@@ -15,6 +15,7 @@
 #include "dgc_internal.hpp"
 #include "ipdg.cuh"
 #include "ipdg_blk.cuh"
+#include "ipdg_eo.cuh"
 
 namespace dgk {
 
@@ -57,6 +58,47 @@ cudaError_t ipdg_launch_n(int kind, const IpdgParams& p, int sm, cudaStream_t s)
   if (grid > ntiles) grid = ntiles;
   void* args[] = {const_cast<IpdgParams*>(&p)};
   return cudaLaunchKernel(fn, dim3(grid), dim3(256), args, smem, s);
+}
+
+// The FP64 passes in the even / odd basis (ipdg_eo.cuh): kind IK_GRAD_PLAIN ..
+// IK_DIV_RESID.  Overlapped launch where the grid leaves every SM one CTA, as
+// for the FP64 stage kernel (rhs_f64.cu).
+template <int N>
+cudaError_t ipdg_eo_launch_n(int kind, const IpdgParams& p, int sm, cudaStream_t s) {
+  using C = IpdgEo<N>;
+  using Fn = void (*)(const IpdgParams, int);
+  static const Fn fns[6] = {ipdg_grad_eo_kernel<N, GRAD_PLAIN>, ipdg_grad_eo_kernel<N, GRAD_PCG>,
+                            ipdg_div_eo_kernel<N, DIV_LAPLACE>, ipdg_div_eo_kernel<N, DIV_SPD>,
+                            ipdg_div_eo_kernel<N, DIV_SPD_DOT>, ipdg_div_eo_kernel<N, DIV_RESID>};
+  static std::once_flag once;
+  static cudaError_t st = cudaSuccess;
+  std::call_once(once, [] {
+    for (int k = 0; k < 6 && st == cudaSuccess; ++k)
+      st = cudaFuncSetAttribute(fns[k], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                k <= IK_GRAD_PCG ? C::kSmemGrad : C::kSmemDiv);
+  });
+  if (st != cudaSuccess) return st;
+  const bool grad = kind <= IK_GRAD_PCG;
+  const int te = eo_pick_tile(C::D, p.K, sm, C::TE, grad ? C::kCostGrad : C::kCostDiv);
+  const int ntiles = (p.K + te - 1) / te;
+  const size_t smem = grad ? C::kSmemGrad : C::kSmemDiv;
+  if (ntiles <= sm) return launch_stage(fns[kind], ntiles, 256, smem, s, p, te);
+  fns[kind]<<<ntiles, 256, smem, s>>>(p, te);
+  return cudaGetLastError();
+}
+
+cudaError_t ipdg_eo_launch(int N, int kind, const IpdgParams& p, int sm, cudaStream_t s) {
+  switch (N) {
+    case 1: return ipdg_eo_launch_n<1>(kind, p, sm, s);
+    case 2: return ipdg_eo_launch_n<2>(kind, p, sm, s);
+    case 3: return ipdg_eo_launch_n<3>(kind, p, sm, s);
+    case 4: return ipdg_eo_launch_n<4>(kind, p, sm, s);
+    case 5: return ipdg_eo_launch_n<5>(kind, p, sm, s);
+    case 6: return ipdg_eo_launch_n<6>(kind, p, sm, s);
+    case 7: return ipdg_eo_launch_n<7>(kind, p, sm, s);
+    case 8: return ipdg_eo_launch_n<8>(kind, p, sm, s);
+    default: return cudaErrorInvalidValue;
+  }
 }
 
 // register-blocked FP32 CG kernels
@@ -363,6 +405,8 @@ dgk::IpdgParams base(const dgc_handle_s* h) {
   p.tau = sizeof(R) == 8 ? (const void*)h->d_tau : (const void*)h->d_tau32;
   p.mats = sizeof(R) == 8 ? h->d_mats64[1] : h->d_mats32[1];
   p.mass = sizeof(R) == 8 ? h->ipdg->mass64 : h->ipdg->mass32;
+  p.mats_eo = sizeof(R) == 8 && h->eo_ok[1] ? h->d_eo64[1] : nullptr;
+  p.tab_eo = h->d_eo_tab[1];
   p.binv = sizeof(R) == 8 ? (const void*)h->ipdg->binv64 : (const void*)h->ipdg->binv32;
   p.mats_blk = h->ipdg->ops_blk32;
   p.mass_blk = h->ipdg->mass_blk32;
@@ -375,7 +419,10 @@ dgk::IpdgParams base(const dgc_handle_s* h) {
 
 template <typename R>
 int launch(dgc_handle_s* h, int kind, const dgk::IpdgParams& p, cudaStream_t s) {
-  cudaError_t e = dgk::ipdg_launch<R>(h->N, kind, p, h->sm_count, s);
+  // FP64 passes in the even / odd basis; the node-by-node ones for operators
+  // without the reflection symmetry (dgc_set_operators)
+  cudaError_t e = p.mats_eo && kind <= dgk::IK_DIV_RESID ? dgk::ipdg_eo_launch(h->N, kind, p, h->sm_count, s)
+                                                         : dgk::ipdg_launch<R>(h->N, kind, p, h->sm_count, s);
   if (e != cudaSuccess) return cuda_err(e, "ipdg kernel launch");
   ++h->launches;
   return DGC_OK;
@@ -674,7 +721,9 @@ int ipdg_boundary_cells(const dgc_handle_s* h, const int** cells, int* n) {
 }
 
 void ipdg_operators_changed(dgc_handle_s* h) {
-  if (h->ipdg) upload_ipdg_matrices(h);
+  if (!h->ipdg) return;
+  drop_chunk_graphs(h->ipdg);  // the passes' kernels depend on the operators' symmetry
+  upload_ipdg_matrices(h);
 }
 
 namespace {

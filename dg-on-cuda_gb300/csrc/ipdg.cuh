@@ -47,6 +47,8 @@ struct IpdgParams {
   const void* tau;      // [K][4] penalty per face, in R
   const void* mats;     // strong-form DrT | DsT | LT (R)
   const void* mass;     // M (Np x Np, R), symmetric
+  const void* mats_eo;  // FP64: strong-form operators and M in the even / odd basis (ipdg_eo.cuh), NULL: not symmetric
+  const uint8_t* tab_eo;  // their pair tables
   // grad pass
   const void* u;        // input u (GRAD_PLAIN) or z (GRAD_PCG)
   void* p;              // GRAD_PCG: new search direction p (written); update: p (read)

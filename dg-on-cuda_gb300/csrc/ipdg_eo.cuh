@@ -1,0 +1,416 @@
+// ipdg_eo.cuh -- the two passes of laplace_2d (ipdg.cuh) in the even / odd basis
+// of the reflection r <-> s (eo.hpp): the FP64 path of the operator, of its CG
+// iteration and of the refinement residuals.
+//
+// Bound by the FP64 pipe like the FP64 stage kernel (dg_rhs_eo.cuh): the
+// node-by-node passes kept it over 90 % busy.  FP64 instructions per element at
+// N = 4, grad + div + mass: 1.4k instead of 2.7k --
+//   * D+ and D- of a field take Np^2 products where Dr and Ds took 2 Np^2, and
+//     the divergence is one D+ p + D- m, p and m combined from (qx, qy) with the
+//     element's constant geometry: 2 Np^2 instead of 6 Np^2 for both passes, LIFT
+//     and M half of theirs;
+//   * -1/J (the SPD form: J (1/J) = 1), faceJ, normals and penalties are
+//     multiplied into per-element constants.
+// One tile of `te` elements per CTA (eo_pick_tile); set-up data are fetched
+// before the wait for the previous launch, exterior traces while the tile's own
+// fields arrive.
+#pragma once
+
+#include "eo.hpp"
+#include "ipdg.cuh"
+
+namespace dgk {
+
+template <int N>
+struct IpdgEo {
+  using R = double;
+  using O = Order<N>;
+  static constexpr EoDims D{N};
+  static constexpr int Np = O::Np, NpP = O::NpP, Nfp = O::Nfp;
+  static constexpr int nE = D.nE, nO = D.nO, fE = D.fE, fO = D.fO;
+  static constexpr int TE = 256 / Np;
+  static constexpr int FSTR = 4 * fE;  // grad: x | y, div: one, each [fE sums | fE differences]
+  static constexpr int CSTR = 16;
+  static constexpr uint32_t kOpsG = (D.kK() + D.kL()) * 8, kOpsD = kOpsG + D.kM() * 8, kTab = D.tabBytes();
+  static constexpr uint32_t kF = TE * NpP * 8;  // one field
+  static constexpr uint32_t oBar = 0, oTab = 32, oGeom = oTab + kTab, oNbr = oGeom + TE * 16 * 8, oTau = oNbr + TE * 16,
+                            oC = oTau + TE * 4 * 8, oFld = oC + TE * CSTR * 8, oIn = oFld + 3 * kF,
+                            oF = oIn + TE * 2 * Np * 8, oRed = (oF + TE * FSTR * 8 + 15) / 16 * 16, oOps = oRed + 16 * 8;
+  static constexpr uint32_t kSmemGrad = oOps + kOpsG, kSmemDiv = oOps + kOpsD;
+  static_assert(TE * fE <= 256, "one face-node pair per thread");
+  static_assert(oGeom % 16 == 0 && oFld % 16 == 0 && kF % 16 == 0 && oRed % 16 == 0 && kOpsG % 16 == 0, "alignment");
+  // FP64 instructions per item (eo_pick_tile)
+  static constexpr EoCost kCostGrad{Np + 2 * fE + 6, 12, 2, 8}, kCostDiv{Np + fE + nE + 5, 14, 8, 8};
+};
+
+// per-element constants: (rx +- sx, ry +- sy) s, then per face (cx, cy, ct)
+enum IpdgEoConst : int { IC_P1 = 0, IC_P2 = 1, IC_Q1 = 2, IC_Q2 = 3, IC_F = 4 };
+
+// views of a CTA's shared memory, and the parts both passes share
+template <int N>
+struct IpdgEoTile {
+  using C = IpdgEo<N>;
+  unsigned char* smem;
+  __device__ uint64_t* bar() const { return reinterpret_cast<uint64_t*>(smem + C::oBar); }
+  __device__ const uint8_t* nodes() const { return smem + C::oTab; }
+  __device__ const uint8_t* faces() const { return smem + C::oTab + 2 * C::nE; }
+  __device__ const uint8_t* inverse() const { return smem + C::oTab + 2 * C::nE + 2 * C::fE; }
+  __device__ const double* geom() const { return reinterpret_cast<const double*>(smem + C::oGeom); }
+  __device__ const int4* nbr() const { return reinterpret_cast<const int4*>(smem + C::oNbr); }
+  __device__ const double* tau() const { return reinterpret_cast<const double*>(smem + C::oTau); }
+  __device__ double* consts() const { return reinterpret_cast<double*>(smem + C::oC); }
+  __device__ double* field(int i) const { return reinterpret_cast<double*>(smem + C::oFld + i * C::kF); }
+  __device__ double* in() const { return reinterpret_cast<double*>(smem + C::oIn); }
+  __device__ double* flux() const { return reinterpret_cast<double*>(smem + C::oF); }
+  __device__ double* red() const { return reinterpret_cast<double*>(smem + C::oRed); }
+  __device__ const double* K() const { return reinterpret_cast<const double*>(smem + C::oOps); }
+  __device__ const double* L() const { return K() + C::D.kK(); }
+  __device__ const double* M() const { return L() + C::D.kL(); }
+
+  // set-up data of the elements k0 .. k0 + ne - 1; false if a wait expired
+  __device__ bool setup(const IpdgParams& p, int k0, int ne, uint32_t ops, bool tau) const {
+    if (threadIdx.x == 0) {
+      mbar_init(bar(), 1);
+      mbar_init(bar() + 1, 1);
+      fence_barrier_init();
+      mbar_arrive_expect_tx(bar(), ops + C::kTab + ne * (16 * 8 + 16 + (tau ? 32 : 0)));
+      bulk_g2s(smem + C::oOps, p.mats_eo, ops, bar());
+      bulk_g2s(smem + C::oTab, p.tab_eo, C::kTab, bar());
+      bulk_g2s(smem + C::oGeom, static_cast<const double*>(p.geom) + (size_t)k0 * 16, ne * 16 * 8, bar());
+      bulk_g2s(smem + C::oNbr, p.nbr + k0, ne * 16, bar());
+      if (tau) bulk_g2s(smem + C::oTau, static_cast<const double*>(p.tau) + (size_t)k0 * 4, ne * 32, bar());
+    }
+    __syncthreads();
+    return __syncthreads_and(mbar_wait(bar(), 0, p.status));
+  }
+  // constants: volume factors times sv, face factors h n and 2 tau h, h = faceJ / 2 times sf
+  template <bool TAU>
+  __device__ void constants(int ne, bool spd) const {
+    for (int x = 255 - (int)threadIdx.x; x < ne * 8; x += 256) {
+      const int e = x >> 3, v = x & 7;
+      const double* g = geom() + e * 16;
+      double* c = consts() + e * C::CSTR;
+      const double sv = spd ? g[14] : 1.0, sf = spd ? 1.0 : g[4];  // -J and (-1/J)(-J) = 1 | 1 and -1/J
+      if (v < 2) c[IC_P1 + v] = sv * (v ? g[0] - g[2] : g[0] + g[2]);
+      else if (v < 4) c[IC_Q1 + v - 2] = sv * (v == 3 ? g[1] - g[3] : g[1] + g[3]);
+      else if (v < 7) {
+        const int f = v - 4;
+        const double h = 0.5 * g[5 + f] * sf;
+        c[IC_F + 3 * f] = h * g[8 + f];
+        c[IC_F + 3 * f + 1] = h * g[11 + f];
+        if (TAU) c[IC_F + 3 * f + 2] = 2.0 * tau()[e * 4 + f] * h;
+      }
+    }
+  }
+};
+
+// ---------------------------------------------------------------- grad pass
+template <int N, int MODE>
+__global__ void __launch_bounds__(256) ipdg_grad_eo_kernel(const IpdgParams p, const int te) {
+  using C = IpdgEo<N>;
+  constexpr int Np = C::Np, NpP = C::NpP, Nfp = C::Nfp, nE = C::nE, nO = C::nO, fE = C::fE, fO = C::fO;
+  constexpr bool PCG = MODE == GRAD_PCG;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ double s_beta;
+  const IpdgEoTile<N> t{smem};
+  const int tid = threadIdx.x;
+  const int k0 = blockIdx.x * te, ne = min(te, p.K - k0);
+  if (!t.setup(p, k0, ne, C::kOpsG, false)) return;
+  const double* u_in = static_cast<const double*>(p.u);
+  const double* pold = static_cast<const double*>(p.p_old);
+  grid_dep_wait();
+  grid_dep_launch();
+  if (PCG && p.cg->done) return;
+  if (tid == 0) {
+    mbar_arrive_expect_tx(t.bar() + 1, (PCG ? 2 : 1) * ne * NpP * 8);
+    bulk_g2s(t.field(0), u_in + (size_t)k0 * NpP, ne * NpP * 8, t.bar() + 1);
+    if (PCG) bulk_g2s(t.field(1), pold + (size_t)k0 * NpP, ne * NpP * 8, t.bar() + 1);
+    // beta = rz_new / rz_old, one division per CTA
+    s_beta = PCG && !p.first ? p.cg->rz[p.slot] / p.cg->rz[(p.slot + 2) % 3] : 0.0;
+    if (PCG && blockIdx.x == 0) p.cg->pAp = 0.0;
+  }
+  // exterior values of the face-node pair
+  const int fe = tid / fE, fc = tid - fe * fE;
+  const bool fact = fe < ne, ftwo = fc < fO;
+  double bz[2] = {0.0, 0.0}, bp[2] = {0.0, 0.0};
+  int kind[2] = {0, 0};  // 0 interior, 1 Dirichlet, 2 Neumann
+  if (fact) {
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      if (w && !ftwo) break;
+      const int m = t.faces()[2 * fc + w], f = m / Nfp, d = m - f * Nfp;
+      const int nb = nb_of<double, N>(t.nbr()[fe], f);
+      if (nb >= 0) {
+        const size_t o = (size_t)(nb >> 2) * NpP + fmask<N>(nb & 3, Nfp - 1 - d);
+        bz[w] = __ldg(u_in + o);
+        if (PCG) bp[w] = __ldg(pold + o);
+      } else {
+        kind[w] = bc_dirichlet<N>(p, nb, d) ? 1 : 2;
+      }
+    }
+  }
+  t.template constants<false>(ne, false);
+  if (!__syncthreads_and(mbar_wait(t.bar() + 1, 0, p.status))) return;
+  double* sU = t.field(0);
+  const double beta = s_beta;
+  if (PCG) {
+    // p = z + beta p_old on the tile, written out
+    double* pv = static_cast<double*>(p.p);
+    for (int x = tid; x < ne * NpP; x += 256) {
+      const double v = fma(beta, t.field(1)[x], sU[x]);
+      sU[x] = v;
+      pv[(size_t)k0 * NpP + x] = v;
+    }
+    __syncthreads();
+  }
+  // lifted jumps: sums and differences of the face-node pairs
+  if (fact) {
+    const double* c = t.consts() + fe * C::CSTR + IC_F;
+    double lx[2] = {0.0, 0.0}, ly[2] = {0.0, 0.0};
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      if (w && !ftwo) break;
+      const int m = t.faces()[2 * fc + w], f = m / Nfp, d = m - f * Nfp;
+      const double um = sU[fe * NpP + fmask<N>(f, d)];
+      double up = PCG ? fma(beta, bp[w], bz[w]) : bz[w];
+      if (kind[w]) up = kind[w] == 1 ? -um : um;
+      const double du = um - up;
+      lx[w] = c[3 * f] * du;
+      ly[w] = c[3 * f + 1] * du;
+    }
+    double* fo = t.flux() + fe * C::FSTR + fc;
+    fo[0] = ftwo ? lx[0] + lx[1] : lx[0];
+    fo[fE] = ftwo ? lx[0] - lx[1] : 0.0;
+    fo[2 * fE] = ftwo ? ly[0] + ly[1] : ly[0];
+    fo[3 * fE] = ftwo ? ly[0] - ly[1] : 0.0;
+  }
+  for (int x = 255 - tid; x < ne * nE; x += 256) {
+    const int e = x / nE, c = x - e * nE;
+    double* in = t.in() + e * 2 * Np + c;
+    const double ua = sU[e * NpP + t.nodes()[2 * c]];
+    if (c < nO) {
+      const double ub = sU[e * NpP + t.nodes()[2 * c + 1]];
+      in[0] = ua + ub;
+      in[nE] = ua - ub;
+    } else {
+      in[0] = ua;
+    }
+  }
+  __syncthreads();
+  const int e = tid / Np, r = tid - e * Np;
+  const bool act = e < ne;
+  double qx = 0.0, qy = 0.0;
+  if (act) {
+    const bool sum = r < nE;
+    const double* k = t.K() + r;
+    const double* x = t.in() + e * 2 * Np;
+    const double* c = t.consts() + e * C::CSTR;
+    double s1 = 0.0, s2 = 0.0;
+#pragma unroll 4
+    for (int j = 0; j < nE; ++j) s1 = fma(k[j * Np], x[j], s1);
+    k += nE * Np;
+    x += nE;
+#pragma unroll 4
+    for (int j = 0; j < nO; ++j) s2 = fma(k[j * Np], x[j], s2);
+    const int ia = sum ? 0 : 1;  // D+ u is s1 in a sum row, s2 in a difference row
+    qx = fma(c[IC_P1 + ia], s1, c[IC_P2 - ia] * s2);
+    qy = fma(c[IC_Q1 + ia], s1, c[IC_Q2 - ia] * s2);
+    const double* l = t.L() + r;
+    const double* f = t.flux() + e * C::FSTR + (sum ? 0 : fE);
+#pragma unroll 4
+    for (int m = 0; m < fE; ++m) {
+      const double ll = l[m * Np];
+      qx = fma(ll, f[m], qx);
+      qy = fma(ll, f[2 * fE + m], qy);
+    }
+  }
+  __syncthreads();
+  double* ro = t.in() + e * 2 * Np;
+  if (act) {
+    ro[r] = qx;
+    ro[Np + r] = qy;
+  }
+  __syncthreads();
+  if (act) {
+    const int inv = t.inverse()[r], c = inv & 127;
+    qx = ro[c];
+    qy = ro[Np + c];
+    if (c < nO) {
+      const double ox = ro[nE + c], oy = ro[Np + nE + c];
+      qx = inv & 128 ? qx - ox : qx + ox;
+      qy = inv & 128 ? qy - oy : qy + oy;
+    }
+    const size_t o = (size_t)(k0 + e) * NpP + r;
+    static_cast<double*>(p.qx)[o] = qx;
+    static_cast<double*>(p.qy)[o] = qy;
+  }
+}
+
+// ---------------------------------------------------------------- div pass
+template <int N, int MODE>
+__global__ void __launch_bounds__(256) ipdg_div_eo_kernel(const IpdgParams p, const int te) {
+  using C = IpdgEo<N>;
+  constexpr int Np = C::Np, NpP = C::NpP, Nfp = C::Nfp, nE = C::nE, nO = C::nO, fE = C::fE, fO = C::fO;
+  constexpr bool SPD = MODE != DIV_LAPLACE;
+  extern __shared__ __align__(128) unsigned char smem[];
+  const IpdgEoTile<N> t{smem};
+  const int tid = threadIdx.x;
+  const int k0 = blockIdx.x * te, ne = min(te, p.K - k0);
+  if (!t.setup(p, k0, ne, SPD ? C::kOpsD : C::kOpsG, true)) return;
+  const double* qx = static_cast<const double*>(p.qx);
+  const double* qy = static_cast<const double*>(p.qy);
+  const double* uj = static_cast<const double*>(p.du_src);
+  double* out = static_cast<double*>(p.out);
+  grid_dep_wait();
+  grid_dep_launch();
+  if (MODE == DIV_SPD_DOT && p.cg->done) return;
+  if (tid == 0) {
+    mbar_arrive_expect_tx(t.bar() + 1, 3 * ne * NpP * 8);
+    bulk_g2s(t.field(0), qx + (size_t)k0 * NpP, ne * NpP * 8, t.bar() + 1);
+    bulk_g2s(t.field(1), qy + (size_t)k0 * NpP, ne * NpP * 8, t.bar() + 1);
+    bulk_g2s(t.field(2), uj + (size_t)k0 * NpP, ne * NpP * 8, t.bar() + 1);
+    if (MODE == DIV_SPD_DOT && blockIdx.x == 0) {
+      const int s1 = (p.slot + 1) % 3;
+      p.cg->rz[s1] = 0.0;
+      p.cg->rr[s1] = 0.0;
+    }
+  }
+  // exterior traces of the face-node pair
+  const int fe = tid / fE, fc = tid - fe * fE;
+  const bool fact = fe < ne, ftwo = fc < fO;
+  double bx[2], by[2], bu[2];
+  int kind[2] = {0, 0};
+  if (fact) {
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      if (w && !ftwo) break;
+      const int m = t.faces()[2 * fc + w], f = m / Nfp, d = m - f * Nfp;
+      const int nb = nb_of<double, N>(t.nbr()[fe], f);
+      if (nb >= 0) {
+        const size_t o = (size_t)(nb >> 2) * NpP + fmask<N>(nb & 3, Nfp - 1 - d);
+        bx[w] = __ldg(qx + o);
+        by[w] = __ldg(qy + o);
+        bu[w] = __ldg(uj + o);
+      } else {
+        kind[w] = bc_dirichlet<N>(p, nb, d) ? 1 : 2;
+      }
+    }
+  }
+  const int e = tid / Np, r = tid - e * Np;
+  const bool act = e < ne;
+  const size_t o = (size_t)(k0 + e) * NpP + r;
+  double bv = 0.0;
+  if (MODE == DIV_RESID && act) bv = static_cast<const double*>(p.b)[o];
+  t.template constants<true>(ne, SPD);
+  if (!__syncthreads_and(mbar_wait(t.bar() + 1, 0, p.status))) return;
+  const double *sX = t.field(0), *sY = t.field(1), *sU = t.field(2);
+  if (fact) {
+    const double* c = t.consts() + fe * C::CSTR + IC_F;
+    double fl[2] = {0.0, 0.0};
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      if (w && !ftwo) break;
+      const int m = t.faces()[2 * fc + w], f = m / Nfp, d = m - f * Nfp;
+      const int nd = fe * NpP + fmask<N>(f, d);
+      const double xm = sX[nd], ym = sY[nd], um = sU[nd];
+      if (kind[w]) {  // Dirichlet: [q] = 0, du = 2 u-; Neumann: [q] = 2 q-, du = 0
+        const bool dir = kind[w] == 1;
+        bx[w] = dir ? xm : -xm;
+        by[w] = dir ? ym : -ym;
+        bu[w] = dir ? -um : um;
+      }
+      fl[w] = fma(c[3 * f], xm - bx[w], fma(c[3 * f + 1], ym - by[w], c[3 * f + 2] * (um - bu[w])));
+    }
+    double* fo = t.flux() + fe * C::FSTR + fc;
+    fo[0] = ftwo ? fl[0] + fl[1] : fl[0];
+    fo[fE] = ftwo ? fl[0] - fl[1] : 0.0;
+  }
+  // p | m: the combinations of (qx, qy) that D+ and D- act on
+  for (int x = 255 - tid; x < ne * nE; x += 256) {
+    const int ie = x / nE, c = x - ie * nE;
+    const double* cc = t.consts() + ie * C::CSTR;
+    const double p1 = cc[IC_P1], p2 = cc[IC_P2], q1 = cc[IC_Q1], q2 = cc[IC_Q2];
+    double* in = t.in() + ie * 2 * Np + c;
+    const int na = ie * NpP + t.nodes()[2 * c], nb = ie * NpP + t.nodes()[2 * c + 1];
+    const double xa = sX[na], ya = sY[na];
+    if (c < nO) {
+      const double xb = sX[nb], yb = sY[nb];
+      const double xs = xa + xb, ys = ya + yb, xd = xa - xb, yd = ya - yb;
+      in[0] = fma(p1, xs, q1 * ys);
+      in[Np] = fma(p2, xs, q2 * ys);
+      in[nE] = fma(p1, xd, q1 * yd);
+      in[Np + nE] = fma(p2, xd, q2 * yd);
+    } else {
+      in[0] = fma(p1, xa, q1 * ya);
+      in[Np] = fma(p2, xa, q2 * ya);
+    }
+  }
+  __syncthreads();
+  double au = 0.0;
+  const bool sum = r < nE;
+  if (act) {
+    const double* k = t.K() + r;
+    const double* x = t.in() + e * 2 * Np;
+    // sum rows take p's sums and m's differences, difference rows the others
+    const double* u = x + (sum ? 0 : Np);
+    const double* v = x + (sum ? Np : 0) + nE;
+    double s2 = 0.0;
+#pragma unroll 4
+    for (int j = 0; j < nE; ++j) au = fma(k[j * Np], u[j], au);
+    k += nE * Np;
+#pragma unroll 4
+    for (int j = 0; j < nO; ++j) s2 = fma(k[j * Np], v[j], s2);
+    const double* l = t.L() + r;
+    const double* f = t.flux() + e * C::FSTR + (sum ? 0 : fE);
+#pragma unroll 4
+    for (int m = 0; m < fE; ++m) au = fma(l[m * Np], f[m], au);
+    au += s2;
+    if (SPD && p.shift != 0.0) {  // (A - shift I) u, scaled by -J like the rest
+      const int c = sum ? r : r - nE;
+      const double ua = sU[e * NpP + t.nodes()[2 * c]], ub = sU[e * NpP + t.nodes()[2 * c + 1]];
+      const double uh = sum ? (c < nO ? 0.5 * (ua + ub) : ua) : 0.5 * (ua - ub);
+      au = fma(-p.shift * t.geom()[e * 16 + 14], uh, au);
+    }
+  }
+  __syncthreads();
+  double* ro = t.in() + e * 2 * Np;
+  if (act) ro[r] = au;
+  __syncthreads();
+  if (SPD) {
+    if (act) {
+      // mass rows: half sums from half sums, half differences from half differences
+      const double* m = t.M() + r;
+      const double* w = ro + (sum ? 0 : nE);
+      const int n = sum ? nE : nO;
+      au = 0.0;
+#pragma unroll 4
+      for (int j = 0; j < n; ++j) au = fma(m[j * Np], w[j], au);
+      ro[Np + r] = au;
+    }
+    __syncthreads();
+    ro += Np;
+  }
+  double dot = 0.0;
+  if (act) {
+    const int inv = t.inverse()[r], c = inv & 127;
+    double v = ro[c];
+    if (c < nO) v = inv & 128 ? v - ro[nE + c] : v + ro[nE + c];
+    if (MODE == DIV_RESID) {
+      v = bv - v;
+      dot = v * v;
+    } else if (MODE == DIV_SPD_DOT) {
+      dot = sU[e * NpP + r] * v;
+    }
+    out[o] = v;
+  }
+  // padded output nodes are written as 0 (callers sum over whole vectors)
+  constexpr int kPad = NpP - Np;
+  if constexpr (kPad > 0)
+    for (int q = tid; q < ne * kPad; q += 256) out[(size_t)(k0 + q / kPad) * NpP + Np + q % kPad] = 0.0;
+  if (MODE == DIV_SPD_DOT || MODE == DIV_RESID) {
+    const double s = block_sum(dot, t.red());
+    if (tid == 0) atomicAdd(MODE == DIV_SPD_DOT ? &p.cg->pAp : p.dot_out, s);
+  }
+}
+
+}  // namespace dgk

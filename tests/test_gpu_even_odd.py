@@ -40,6 +40,23 @@ def test_stage(N, n):
         D.check()
 
 
+@pytest.mark.parametrize("n", [1, 4, 19])
+@pytest.mark.parametrize("N", range(1, 9))
+def test_laplace(N, n):
+    m = dg.meshes.jittered_square(n, seed=10 + N)
+    o = oracle.Oracle(m.xy, m.cells, N)
+    D = dg.Discretization(m, "laplace", N, dg.F64, tau=dg.TAU_SCALED, dirichlet=True)
+    u0 = np.random.default_rng(N).standard_normal(D.K * D.Np)
+    u = D.upload(u0)
+    assert rel(D.download(D.laplace(u)), o.laplace(u0, True, 1)) < TOL
+    s = o.spd(u0, 1)
+    assert rel(D.download(D.spd(u)), s) < TOL
+    # shifted form S + shift J M
+    D.set_shift(3.5)
+    assert rel(D.download(D.spd(u)), s + 3.5 * D.download(D.mass(u))) < TOL
+    D.check()
+
+
 def test_operators_without_the_symmetry():
     """The node-by-node kernels take over, and give the caller's operators."""
     N = 4
