@@ -43,6 +43,10 @@ struct IpdgEo {
   static constexpr EoCost kCostGrad{Np + 2 * fE + 6, 12, 2, 8}, kCostDiv{Np + fE + nE + 5, 14, 8, 8};
 };
 
+// volume + lift / J as the strong form has them (1, -1/J), the strong form times
+// -J, or the weak form's signs (-1, 1/J)
+enum IpdgEoForm : int { EO_STRONG = 0, EO_SPD = 1, EO_WEAK = 2 };
+
 // per-element constants: (rx +- sx, ry +- sy) s, then per face (cx, cy, ct)
 enum IpdgEoConst : int { IC_P1 = 0, IC_P2 = 1, IC_Q1 = 2, IC_Q2 = 3, IC_F = 4 };
 
@@ -84,13 +88,14 @@ struct IpdgEoTile {
     return __syncthreads_and(mbar_wait(bar(), 0, p.status));
   }
   // constants: volume factors times sv, face factors h n and 2 tau h, h = faceJ / 2 times sf
-  template <bool TAU>
-  __device__ void constants(int ne, bool spd) const {
+  template <IpdgEoForm FORM, bool TAU = false>
+  __device__ void constants(int ne) const {
     for (int x = 255 - (int)threadIdx.x; x < ne * 8; x += 256) {
       const int e = x >> 3, v = x & 7;
       const double* g = geom() + e * 16;
       double* c = consts() + e * C::CSTR;
-      const double sv = spd ? g[14] : 1.0, sf = spd ? 1.0 : g[4];  // -J and (-1/J)(-J) = 1 | 1 and -1/J
+      const double sv = FORM == EO_SPD ? g[14] : (FORM == EO_WEAK ? -1.0 : 1.0);      // g[14] = -J
+      const double sf = FORM == EO_SPD ? 1.0 : (FORM == EO_WEAK ? -g[4] : g[4]);      // g[4] = -1/J
       if (v < 2) c[IC_P1 + v] = sv * (v ? g[0] - g[2] : g[0] + g[2]);
       else if (v < 4) c[IC_Q1 + v - 2] = sv * (v == 3 ? g[1] - g[3] : g[1] + g[3]);
       else if (v < 7) {
@@ -101,6 +106,120 @@ struct IpdgEoTile {
         if (TAU) c[IC_F + 3 * f + 2] = 2.0 * tau()[e * 4 + f] * h;
       }
     }
+  }
+
+  // inputs of the gradient rows: sums and differences of the field u
+  __device__ void sum_diff(const double* u, int ne) const {
+    constexpr int nE = C::nE;
+    for (int x = 255 - (int)threadIdx.x; x < ne * nE; x += 256) {
+      const int e = x / nE, c = x - e * nE;
+      double* i = in() + e * 2 * C::Np + c;
+      const double ua = u[e * C::NpP + nodes()[2 * c]];
+      if (c < C::nO) {
+        const double ub = u[e * C::NpP + nodes()[2 * c + 1]];
+        i[0] = ua + ub;
+        i[nE] = ua - ub;
+      } else {
+        i[0] = ua;
+      }
+    }
+  }
+  // inputs of the divergence rows: p | m, the combinations of the fields (x, y)
+  // that D+ and D- act on
+  __device__ void combine(const double* fx, const double* fy, int ne) const {
+    constexpr int nE = C::nE, Np = C::Np;
+    for (int x = 255 - (int)threadIdx.x; x < ne * nE; x += 256) {
+      const int e = x / nE, c = x - e * nE;
+      const double* cc = consts() + e * C::CSTR;
+      const double p1 = cc[IC_P1], p2 = cc[IC_P2], q1 = cc[IC_Q1], q2 = cc[IC_Q2];
+      double* i = in() + e * 2 * Np + c;
+      const int na = e * C::NpP + nodes()[2 * c], nb = e * C::NpP + nodes()[2 * c + 1];
+      const double xa = fx[na], ya = fy[na];
+      if (c < C::nO) {
+        const double xb = fx[nb], yb = fy[nb];
+        const double xs = xa + xb, ys = ya + yb, xd = xa - xb, yd = ya - yb;
+        i[0] = fma(p1, xs, q1 * ys);
+        i[Np] = fma(p2, xs, q2 * ys);
+        i[nE] = fma(p1, xd, q1 * yd);
+        i[Np + nE] = fma(p2, xd, q2 * yd);
+      } else {
+        i[0] = fma(p1, xa, q1 * ya);
+        i[Np] = fma(p2, xa, q2 * ya);
+      }
+    }
+  }
+  // node r's value from the sums and differences ro[Np] of its element's rows
+  __device__ double node(const double* ro, int r) const {
+    const int inv = inverse()[r], c = inv & 127;
+    const double v = ro[c];
+    if (c >= C::nO) return v;
+    const double o = ro[C::nE + c];
+    return inv & 128 ? v - o : v + o;
+  }
+  // gradient rows of the tile from sum_diff's inputs and the x | y flux sums and
+  // differences, then both components by node
+  __device__ void grad_rows(int ne, int k0, double* ox, double* oy) const {
+    constexpr int Np = C::Np, nE = C::nE, nO = C::nO, fE = C::fE;
+    const int e = (int)threadIdx.x / Np, r = (int)threadIdx.x - e * Np;
+    const bool act = e < ne;
+    double qx = 0.0, qy = 0.0;
+    if (act) {
+      const bool sum = r < nE;
+      const double* k = K() + r;
+      const double* x = in() + e * 2 * Np;
+      const double* c = consts() + e * C::CSTR;
+      double s1 = 0.0, s2 = 0.0;
+#pragma unroll 4
+      for (int j = 0; j < nE; ++j) s1 = fma(k[j * Np], x[j], s1);
+      k += nE * Np;
+      x += nE;
+#pragma unroll 4
+      for (int j = 0; j < nO; ++j) s2 = fma(k[j * Np], x[j], s2);
+      const int ia = sum ? 0 : 1;  // D+ u is s1 in a sum row, s2 in a difference row
+      qx = fma(c[IC_P1 + ia], s1, c[IC_P2 - ia] * s2);
+      qy = fma(c[IC_Q1 + ia], s1, c[IC_Q2 - ia] * s2);
+      const double* l = L() + r;
+      const double* f = flux() + e * C::FSTR + (sum ? 0 : fE);
+#pragma unroll 4
+      for (int m = 0; m < fE; ++m) {
+        const double ll = l[m * Np];
+        qx = fma(ll, f[m], qx);
+        qy = fma(ll, f[2 * fE + m], qy);
+      }
+    }
+    __syncthreads();
+    double* ro = in() + e * 2 * Np;
+    if (act) {
+      ro[r] = qx;
+      ro[Np + r] = qy;
+    }
+    __syncthreads();
+    if (act) {
+      const size_t o = (size_t)(k0 + e) * C::NpP + r;
+      ox[o] = node(ro, r);
+      oy[o] = node(ro + Np, r);
+    }
+  }
+  // divergence row r of element e from combine's inputs and the flux sums and differences
+  __device__ double div_row(int e, int r) const {
+    constexpr int Np = C::Np, nE = C::nE, nO = C::nO, fE = C::fE;
+    const bool sum = r < nE;
+    const double* k = K() + r;
+    const double* x = in() + e * 2 * Np;
+    // sum rows take p's sums and m's differences, difference rows the others
+    const double* u = x + (sum ? 0 : Np);
+    const double* v = x + (sum ? Np : 0) + nE;
+    double s1 = 0.0, s2 = 0.0;
+#pragma unroll 4
+    for (int j = 0; j < nE; ++j) s1 = fma(k[j * Np], u[j], s1);
+    k += nE * Np;
+#pragma unroll 4
+    for (int j = 0; j < nO; ++j) s2 = fma(k[j * Np], v[j], s2);
+    const double* l = L() + r;
+    const double* f = flux() + e * C::FSTR + (sum ? 0 : fE);
+#pragma unroll 4
+    for (int m = 0; m < fE; ++m) s1 = fma(l[m * Np], f[m], s1);
+    return s1 + s2;
   }
 };
 
@@ -149,7 +268,7 @@ __global__ void __launch_bounds__(256) ipdg_grad_eo_kernel(const IpdgParams p, c
       }
     }
   }
-  t.template constants<false>(ne, false);
+  t.template constants<EO_STRONG>(ne);
   if (!__syncthreads_and(mbar_wait(t.bar() + 1, 0, p.status))) return;
   double* sU = t.field(0);
   const double beta = s_beta;
@@ -184,66 +303,9 @@ __global__ void __launch_bounds__(256) ipdg_grad_eo_kernel(const IpdgParams p, c
     fo[2 * fE] = ftwo ? ly[0] + ly[1] : ly[0];
     fo[3 * fE] = ftwo ? ly[0] - ly[1] : 0.0;
   }
-  for (int x = 255 - tid; x < ne * nE; x += 256) {
-    const int e = x / nE, c = x - e * nE;
-    double* in = t.in() + e * 2 * Np + c;
-    const double ua = sU[e * NpP + t.nodes()[2 * c]];
-    if (c < nO) {
-      const double ub = sU[e * NpP + t.nodes()[2 * c + 1]];
-      in[0] = ua + ub;
-      in[nE] = ua - ub;
-    } else {
-      in[0] = ua;
-    }
-  }
+  t.sum_diff(sU, ne);
   __syncthreads();
-  const int e = tid / Np, r = tid - e * Np;
-  const bool act = e < ne;
-  double qx = 0.0, qy = 0.0;
-  if (act) {
-    const bool sum = r < nE;
-    const double* k = t.K() + r;
-    const double* x = t.in() + e * 2 * Np;
-    const double* c = t.consts() + e * C::CSTR;
-    double s1 = 0.0, s2 = 0.0;
-#pragma unroll 4
-    for (int j = 0; j < nE; ++j) s1 = fma(k[j * Np], x[j], s1);
-    k += nE * Np;
-    x += nE;
-#pragma unroll 4
-    for (int j = 0; j < nO; ++j) s2 = fma(k[j * Np], x[j], s2);
-    const int ia = sum ? 0 : 1;  // D+ u is s1 in a sum row, s2 in a difference row
-    qx = fma(c[IC_P1 + ia], s1, c[IC_P2 - ia] * s2);
-    qy = fma(c[IC_Q1 + ia], s1, c[IC_Q2 - ia] * s2);
-    const double* l = t.L() + r;
-    const double* f = t.flux() + e * C::FSTR + (sum ? 0 : fE);
-#pragma unroll 4
-    for (int m = 0; m < fE; ++m) {
-      const double ll = l[m * Np];
-      qx = fma(ll, f[m], qx);
-      qy = fma(ll, f[2 * fE + m], qy);
-    }
-  }
-  __syncthreads();
-  double* ro = t.in() + e * 2 * Np;
-  if (act) {
-    ro[r] = qx;
-    ro[Np + r] = qy;
-  }
-  __syncthreads();
-  if (act) {
-    const int inv = t.inverse()[r], c = inv & 127;
-    qx = ro[c];
-    qy = ro[Np + c];
-    if (c < nO) {
-      const double ox = ro[nE + c], oy = ro[Np + nE + c];
-      qx = inv & 128 ? qx - ox : qx + ox;
-      qy = inv & 128 ? qy - oy : qy + oy;
-    }
-    const size_t o = (size_t)(k0 + e) * NpP + r;
-    static_cast<double*>(p.qx)[o] = qx;
-    static_cast<double*>(p.qy)[o] = qy;
-  }
+  t.grad_rows(ne, k0, static_cast<double*>(p.qx), static_cast<double*>(p.qy));
 }
 
 // ---------------------------------------------------------------- div pass
@@ -301,7 +363,7 @@ __global__ void __launch_bounds__(256) ipdg_div_eo_kernel(const IpdgParams p, co
   const size_t o = (size_t)(k0 + e) * NpP + r;
   double bv = 0.0;
   if (MODE == DIV_RESID && act) bv = static_cast<const double*>(p.b)[o];
-  t.template constants<true>(ne, SPD);
+  t.template constants<SPD ? EO_SPD : EO_STRONG, true>(ne);
   if (!__syncthreads_and(mbar_wait(t.bar() + 1, 0, p.status))) return;
   const double *sX = t.field(0), *sY = t.field(1), *sU = t.field(2);
   if (fact) {
@@ -325,46 +387,12 @@ __global__ void __launch_bounds__(256) ipdg_div_eo_kernel(const IpdgParams p, co
     fo[0] = ftwo ? fl[0] + fl[1] : fl[0];
     fo[fE] = ftwo ? fl[0] - fl[1] : 0.0;
   }
-  // p | m: the combinations of (qx, qy) that D+ and D- act on
-  for (int x = 255 - tid; x < ne * nE; x += 256) {
-    const int ie = x / nE, c = x - ie * nE;
-    const double* cc = t.consts() + ie * C::CSTR;
-    const double p1 = cc[IC_P1], p2 = cc[IC_P2], q1 = cc[IC_Q1], q2 = cc[IC_Q2];
-    double* in = t.in() + ie * 2 * Np + c;
-    const int na = ie * NpP + t.nodes()[2 * c], nb = ie * NpP + t.nodes()[2 * c + 1];
-    const double xa = sX[na], ya = sY[na];
-    if (c < nO) {
-      const double xb = sX[nb], yb = sY[nb];
-      const double xs = xa + xb, ys = ya + yb, xd = xa - xb, yd = ya - yb;
-      in[0] = fma(p1, xs, q1 * ys);
-      in[Np] = fma(p2, xs, q2 * ys);
-      in[nE] = fma(p1, xd, q1 * yd);
-      in[Np + nE] = fma(p2, xd, q2 * yd);
-    } else {
-      in[0] = fma(p1, xa, q1 * ya);
-      in[Np] = fma(p2, xa, q2 * ya);
-    }
-  }
+  t.combine(sX, sY, ne);
   __syncthreads();
   double au = 0.0;
   const bool sum = r < nE;
   if (act) {
-    const double* k = t.K() + r;
-    const double* x = t.in() + e * 2 * Np;
-    // sum rows take p's sums and m's differences, difference rows the others
-    const double* u = x + (sum ? 0 : Np);
-    const double* v = x + (sum ? Np : 0) + nE;
-    double s2 = 0.0;
-#pragma unroll 4
-    for (int j = 0; j < nE; ++j) au = fma(k[j * Np], u[j], au);
-    k += nE * Np;
-#pragma unroll 4
-    for (int j = 0; j < nO; ++j) s2 = fma(k[j * Np], v[j], s2);
-    const double* l = t.L() + r;
-    const double* f = t.flux() + e * C::FSTR + (sum ? 0 : fE);
-#pragma unroll 4
-    for (int m = 0; m < fE; ++m) au = fma(l[m * Np], f[m], au);
-    au += s2;
+    au = t.div_row(e, r);
     if (SPD && p.shift != 0.0) {  // (A - shift I) u, scaled by -J like the rest
       const int c = sum ? r : r - nE;
       const double ua = sU[e * NpP + t.nodes()[2 * c]], ub = sU[e * NpP + t.nodes()[2 * c + 1]];
@@ -392,9 +420,7 @@ __global__ void __launch_bounds__(256) ipdg_div_eo_kernel(const IpdgParams p, co
   }
   double dot = 0.0;
   if (act) {
-    const int inv = t.inverse()[r], c = inv & 127;
-    double v = ro[c];
-    if (c < nO) v = inv & 128 ? v - ro[nE + c] : v + ro[nE + c];
+    double v = t.node(ro, r);
     if (MODE == DIV_RESID) {
       v = bv - v;
       dot = v * v;

@@ -57,6 +57,31 @@ def test_laplace(N, n):
     D.check()
 
 
+@pytest.mark.parametrize("n", [1, 4, 19])
+@pytest.mark.parametrize("N", range(1, 9))
+def test_grad_div(N, n):
+    m = dg.meshes.jittered_square(n, seed=20 + N)
+    o = oracle.Oracle(m.xy, m.cells, N)
+    D = dg.Discretization(m, "laplace", N, dg.F64)
+    rng = np.random.default_rng(N)
+    u0, v0 = rng.standard_normal((2, D.K * D.Np))
+    g, h = rng.standard_normal((2, D.info.num_boundary_faces * D.Nfp))
+    u, v = D.upload(u0), D.upload(v0)
+    gx, gy = D.grad(u, g=g, sign=-1.0)
+    ref = o.grad(u0, g, -1.0)
+    d = D.div(u, v, gx=g, gy=h, sign=0.5)
+    assert rel(D.download(gx), ref[0]) < TOL and rel(D.download(gy), ref[1]) < TOL
+    assert rel(D.download(d), o.div(u0, v0, g, h, 0.5)) < TOL
+    # inputs off a 16-byte boundary take the node-by-node kernel
+    shift = lambda t: torch.cat([t.new_zeros(1), t])[1:]  # noqa: E731
+    us, vs = shift(u), shift(v)
+    assert us.data_ptr() % 16 == 8
+    gxs, gys = D.grad(us, g=g, sign=-1.0)
+    assert rel(D.download(gxs), ref[0]) < TOL and rel(D.download(gys), ref[1]) < TOL
+    assert rel(D.download(D.div(us, vs, gx=g, gy=h, sign=0.5)), D.download(d)) < TOL
+    D.check()
+
+
 def test_operators_without_the_symmetry():
     """The node-by-node kernels take over, and give the caller's operators."""
     N = 4
