@@ -71,54 +71,120 @@ __device__ __forceinline__ void block_add(double v, double* out) {
 }
 
 
-// h0 = Win x + bin; 4 nodes x 64 channels per 256 threads, groups strided over the grid
-__global__ void __launch_bounds__(256) k_fwd_in(int64_t n, int npi, const __nv_bfloat16* __restrict__ Win,
-                                                const __nv_bfloat16* __restrict__ bin, const float* __restrict__ x,
-                                                float* __restrict__ h0) {
-  __shared__ float wT[64][kW];  // [input][channel]
-  __shared__ float xs[4][64];
-  const int t = threadIdx.x, el = t >> 6, c = t & 63;
-  for (int i = t; i < kW * npi; i += 256) wT[i % npi][i / npi] = bf(Win[i]);
-  const float b = bf(bin[c]);
-  for (int64_t g0 = (int64_t)blockIdx.x * 4; g0 < n; g0 += (int64_t)gridDim.x * 4) {
+// 4 consecutive floats of a caller's array, which may start anywhere
+__device__ __forceinline__ float4 load4(const float* p, bool aligned) {
+  return aligned ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+}
+__device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
+// out (64 channels per node) = W x + b, x of npi values per node: the input
+// layer (W = Win[channel][input]) and, transposed (W = Wout^T, no bias), the
+// gradient at the last features.  A CTA takes 64 nodes; thread (node of 16, 4
+// channels) keeps 4 nodes x 4 channels, so 8 vector loads of shared memory feed
+// 64 FMAs.  Bound by writing the features: 76 -> 23 us at 262144 nodes,
+// npi = 16, against one output per thread and two barriers per 4 nodes.
+template <bool TRANS>
+__global__ void __launch_bounds__(256) k_to_features(int64_t n, int npi, const __nv_bfloat16* __restrict__ W,
+                                                     const __nv_bfloat16* __restrict__ bias,
+                                                     const float* __restrict__ x, float* __restrict__ out) {
+  __shared__ __align__(16) float w[48][kW];  // [input][channel]
+  __shared__ __align__(16) float xs[64 * 52];
+  const int t = threadIdx.x, c = 4 * (t & 15), g = t >> 4, str = npi + 4;
+  for (int i = t; i < kW * npi; i += 256) {
+    const int ch = TRANS ? i % kW : i / npi, in = TRANS ? i / kW : i % npi;
+    w[in][ch] = bf(W[i]);
+  }
+  float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (!TRANS) b = make_float4(bf(bias[c]), bf(bias[c + 1]), bf(bias[c + 2]), bf(bias[c + 3]));
+  const int q4 = npi / 4;
+  const bool al = aligned16(x);
+  for (int64_t n0 = (int64_t)blockIdx.x * 64; n0 < n; n0 += (int64_t)gridDim.x * 64) {
     __syncthreads();
-    for (int i = t; i < 4 * npi; i += 256) {
-      const int64_t e = g0 + i / npi;
-      xs[i / npi][i % npi] = e < n ? x[e * npi + i % npi] : 0.0f;
+    for (int i = t; i < 64 * q4; i += 256) {
+      const int r = i / q4, q = i - r * q4;
+      *reinterpret_cast<float4*>(xs + r * str + 4 * q) =
+          n0 + r < n ? load4(x + (n0 + r) * npi + 4 * q, al) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     __syncthreads();
-    const int64_t e = g0 + el;
-    if (e < n) {
-      float a = b;
-      for (int j = 0; j < npi; ++j) a = fmaf(wT[j][c], xs[el][j], a);
-      h0[e * kW + c] = a;
+    float4 a[4] = {b, b, b, b};
+    for (int j = 0; j < npi; j += 4) {
+      float4 wv[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) wv[k] = *reinterpret_cast<const float4*>(&w[j + k][c]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 v = *reinterpret_cast<const float4*>(xs + (g + 16 * i) * str + j);
+        const float vv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          a[i].x = fmaf(wv[k].x, vv[k], a[i].x);
+          a[i].y = fmaf(wv[k].y, vv[k], a[i].y);
+          a[i].z = fmaf(wv[k].z, vv[k], a[i].z);
+          a[i].w = fmaf(wv[k].w, vv[k], a[i].w);
+        }
+      }
     }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (n0 + g + 16 * i < n) *reinterpret_cast<float4*>(out + (n0 + g + 16 * i) * kW + c) = a[i];
   }
 }
 
-
-// y = Wout h + bout; min(256 / npi, 16) nodes x npi outputs per block
+// y = Wout h + bout: a CTA takes 64 nodes, an item 2 nodes x 4 outputs
 __global__ void __launch_bounds__(256) k_fwd_out(int64_t n, int npi, const __nv_bfloat16* __restrict__ Wout,
                                                  const __nv_bfloat16* __restrict__ bout, const float* __restrict__ h,
                                                  float* __restrict__ y) {
-  __shared__ float wT[kW][64];  // [channel][output]
-  __shared__ float hs[16][kW];
-  const int per = min(256 / npi, 16), t = threadIdx.x, el = t / npi, o = t - el * npi;
-  for (int i = t; i < npi * kW; i += 256) wT[i % kW][i / kW] = bf(Wout[i]);
-  const float b = o < npi ? bf(bout[o]) : 0.0f;
-  for (int64_t g0 = (int64_t)blockIdx.x * per; g0 < n; g0 += (int64_t)gridDim.x * per) {
+  __shared__ __align__(16) float w[kW][48];  // [channel][output]
+  __shared__ __align__(16) float hs[64][kW + 4];
+  __shared__ __align__(16) float bs[48];
+  const int t = threadIdx.x, q4 = npi / 4;
+  for (int i = t; i < npi * kW; i += 256) w[i % kW][i / kW] = bf(Wout[i]);
+  if (t < npi) bs[t] = bf(bout[t]);
+  const bool al = aligned16(y);
+  for (int64_t n0 = (int64_t)blockIdx.x * 64; n0 < n; n0 += (int64_t)gridDim.x * 64) {
     __syncthreads();
-    for (int i = t; i < per * kW; i += 256) {
-      const int64_t e = g0 + i / kW;
-      hs[i / kW][i % kW] = e < n ? h[e * kW + i % kW] : 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = (t >> 4) + 16 * i, c = 4 * (t & 15);
+      *reinterpret_cast<float4*>(&hs[r][c]) =
+          n0 + r < n ? *reinterpret_cast<const float4*>(h + (n0 + r) * kW + c) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     __syncthreads();
-    const int64_t e = g0 + el;
-    if (el < per && e < n) {
-      float a = b;
-#pragma unroll 8
-      for (int c = 0; c < kW; ++c) a = fmaf(wT[c][o], hs[el][c], a);
-      y[e * npi + o] = a;
+    for (int it = t; it < 32 * q4; it += 256) {
+      const int r = it / q4, o = 4 * (it - r * q4);
+      float4 a[2];
+      a[0] = a[1] = *reinterpret_cast<const float4*>(&bs[o]);
+#pragma unroll 4
+      for (int c = 0; c < kW; c += 4) {
+        float4 wv[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) wv[k] = *reinterpret_cast<const float4*>(&w[c + k][o]);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const float4 v = *reinterpret_cast<const float4*>(&hs[r + 32 * i][c]);
+          const float vv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            a[i].x = fmaf(wv[k].x, vv[k], a[i].x);
+            a[i].y = fmaf(wv[k].y, vv[k], a[i].y);
+            a[i].z = fmaf(wv[k].z, vv[k], a[i].z);
+            a[i].w = fmaf(wv[k].w, vv[k], a[i].w);
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        if (n0 + r + 32 * i < n) {
+          float* yo = y + (n0 + r + 32 * i) * npi + o;
+          if (al) {
+            *reinterpret_cast<float4*>(yo) = a[i];
+          } else {
+            yo[0] = a[i].x;
+            yo[1] = a[i].y;
+            yo[2] = a[i].z;
+            yo[3] = a[i].w;
+          }
+        }
     }
   }
 }
@@ -162,164 +228,192 @@ __global__ void k_mask_diff(int64_t n, int npi, int np, const float* __restrict_
   }
 }
 
-// per sample s = blockIdx.y: out[2s] += d.Sd, out[2s+1] += t.St (valid nodes)
-__global__ void k_energy_dots(int K, int npi, int np, const float* __restrict__ d, const float* __restrict__ Sd,
+// per sample s = blockIdx.y: out[2s] += d.Sd, out[2s+1] += t.St over the sample's len
+// values (padding nodes are 0 in d and t).  The FP64 conversions and products set
+// the time, not the 67 MB: 121 us with 9728 blocks' reductions at 8 samples of
+// 32768 cells, 51 us with 4 blocks per SM in all.
+__global__ void k_energy_dots(int64_t len, const float* __restrict__ d, const float* __restrict__ Sd,
                               const float* __restrict__ t, const float* __restrict__ St, double* __restrict__ out) {
   const int s = blockIdx.y;
   double a = 0.0, b = 0.0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (int64_t)K * npi;
-       i += (int64_t)gridDim.x * blockDim.x)
-    if ((int)(i % npi) < np) {
-      const int64_t g = (int64_t)s * K * npi + i;
-      a += (double)d[g] * Sd[g];
-      b += (double)t[g] * St[g];
-    }
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < len; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t g = s * len + i;
+    a += (double)d[g] * Sd[g];
+    b += (double)t[g] * St[g];
+  }
   block_add(a, out + 2 * s);
   block_add(b, out + 2 * s + 1);
 }
 
-// energy loss: dy = 2 S d / (t.St S) on valid nodes; *loss = sum_s d.Sd / t.St / S
-__global__ void k_energy_grad(int64_t n, int K, int npi, int np, int S, const float* __restrict__ Sd,
+// energy loss: dy = 2 S d / (t.St S) on valid nodes (sample s = blockIdx.y, one
+// FP64 division per CTA); *loss = sum_s d.Sd / t.St / S
+__global__ void k_energy_grad(int64_t len, int npi, int np, int S, const float* __restrict__ Sd,
                               const double* __restrict__ dots, float* __restrict__ dy, double* __restrict__ loss) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int s = (int)(i / ((int64_t)K * npi));
+  const int s = blockIdx.y;
+  __shared__ double sw;
+  if (threadIdx.x == 0) {
     const double tst = dots[2 * s + 1];
-    const double w = tst > 0.0 ? 2.0 / (tst * S) : 0.0;
-    dy[i] = (int)(i % npi) < np ? (float)(w * Sd[i]) : 0.0f;
+    sw = tst > 0.0 ? 2.0 / (tst * S) : 0.0;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  __syncthreads();
+  const double w = sw;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < len; i += (int64_t)gridDim.x * blockDim.x)
+    dy[s * len + i] = (int)((uint32_t)i % (uint32_t)npi) < np ? (float)(w * Sd[s * len + i]) : 0.0f;
+  if (blockIdx.x == 0 && s == 0 && threadIdx.x == 0) {
     double l = 0.0;
-    for (int s = 0; s < S; ++s)
-      if (dots[2 * s + 1] > 0.0) l += dots[2 * s] / dots[2 * s + 1];
+    for (int q = 0; q < S; ++q)
+      if (dots[2 * q + 1] > 0.0) l += dots[2 * q] / dots[2 * q + 1];
     *loss = l / S;
   }
 }
 
-// dh = Wout^T dy
-__global__ void __launch_bounds__(256) k_bwd_out(int64_t n, int npi, const __nv_bfloat16* __restrict__ Wout,
-                                                 const float* __restrict__ dy, float* __restrict__ dh) {
-  __shared__ float w[64][kW];  // [output][channel]
-  __shared__ float ds[4][64];
-  const int t = threadIdx.x, el = t >> 6, c = t & 63;
-  for (int i = t; i < npi * kW; i += 256) w[i / kW][i % kW] = bf(Wout[i]);
-  for (int64_t g0 = (int64_t)blockIdx.x * 4; g0 < n; g0 += (int64_t)gridDim.x * 4) {
-    __syncthreads();
-    for (int i = t; i < 4 * npi; i += 256) {
-      const int64_t e = g0 + i / npi;
-      ds[i / npi][i % npi] = e < n ? dy[e * npi + i % npi] : 0.0f;
-    }
-    __syncthreads();
-    const int64_t e = g0 + el;
-    if (e < n) {
-      float a = 0.0f;
-      for (int o = 0; o < npi; ++o) a = fmaf(w[o][c], ds[el][o], a);
-      dh[e * kW + c] = a;
-    }
-  }
-}
-
-// m = sum of h over the face neighbours
-__global__ void k_gather(int64_t n, int K, const int4* __restrict__ nbr, const float* __restrict__ h,
-                         float* __restrict__ m) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n * kW; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t e = i / kW;
-    const int c = (int)(i % kW);
-    int64_t j[3];
-    neighbours(nbr, K, e, j);
-    float v = 0.0f;
-#pragma unroll
-    for (int f = 0; f < 3; ++f)
-      if (j[f] >= 0) v += h[j[f] * kW + c];
-    m[i] = v;
-  }
-}
-
-// g = dh * (a > 0), or g = dh for the linear network
-__global__ void k_relu_bwd(int64_t n, const float* __restrict__ dh, const float* __restrict__ a,
-                           float* __restrict__ g, int linear) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    g[i] = (linear || a[i] > 0.0f) ? dh[i] : 0.0f;
-}
-
-// gW[o][i] += sum_e gout[e][o] xin[e][i], gb[o] += sum_e gout[e][o]; nout, nin <= 64.
-// A block accumulates 32-node chunks (grid-strided) in registers, then adds atomically.
+// Weight gradients of the input or output layer: gW[o][i] += sum_e gout[e][o] xin[e][i],
+// gb[o] += sum_e gout[e][o]; nout, nin <= 64, multiples of 4.  A CTA takes 32-node
+// chunks; groups of (nout / 4)(nin / 4) threads, a 4 x 4 block of gW each, share
+// the chunk's nodes, and add to gW atomically (as vectors) at the end.
 __global__ void __launch_bounds__(256) k_grad_dense(int64_t n, int nout, int nin, const float* __restrict__ gout,
                                                     const float* __restrict__ xin, float* __restrict__ gW,
                                                     float* __restrict__ gb) {
-  __shared__ float go[32][64], xi[32][64];
-  const int t = threadIdx.x;
-  const int pairs = nout * nin;
-  float acc[16];
+  __shared__ __align__(16) float buf[2][32][64];
+  float (*go)[64] = buf[0], (*xi)[64] = buf[1];
+  const int t = threadIdx.x, qo = nout / 4, qi = nin / 4, tpg = qo * qi, groups = 256 / tpg;
+  const int grp = t / tpg, u = t - grp * tpg, o = 4 * (u / qi), i0 = 4 * (u % qi);
+  const int sl = t / nout, nsl = 256 / nout, ob = t - sl * nout;  // bias: slice of the rows, output
+  float4 acc[4];
 #pragma unroll
-  for (int q = 0; q < 16; ++q) acc[q] = 0.0f;
+  for (int k = 0; k < 4; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
   float accb = 0.0f;
+  const bool al = aligned16(xin);
   for (int64_t g0 = (int64_t)blockIdx.x * 32; g0 < n; g0 += (int64_t)gridDim.x * 32) {
     __syncthreads();
-    for (int i = t; i < 32 * 64; i += 256) {
-      const int r = i >> 6, c = i & 63;
-      const int64_t e = g0 + r;
-      go[r][c] = (e < n && c < nout) ? gout[e * nout + c] : 0.0f;
-      xi[r][c] = (e < n && c < nin) ? xin[e * nin + c] : 0.0f;
+    for (int q = t; q < 32 * qo; q += 256) {
+      const int r = q / qo, c = q - r * qo;
+      *reinterpret_cast<float4*>(&go[r][4 * c]) =
+          g0 + r < n ? reinterpret_cast<const float4*>(gout)[(g0 + r) * qo + c] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    for (int q = t; q < 32 * qi; q += 256) {
+      const int r = q / qi, c = q - r * qi;
+      *reinterpret_cast<float4*>(&xi[r][4 * c]) =
+          g0 + r < n ? load4(xin + (g0 + r) * nin + 4 * c, al) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     __syncthreads();
+    if (grp < groups)
+      for (int r = grp; r < 32; r += groups) {
+        const float4 gv = *reinterpret_cast<const float4*>(&go[r][o]), xv = *reinterpret_cast<const float4*>(&xi[r][i0]);
+        const float gg[4] = {gv.x, gv.y, gv.z, gv.w};
 #pragma unroll
-    for (int q = 0; q < 16; ++q) {
-      const int pidx = t + q * 256;
-      if (pidx < pairs) {
-        const int o = pidx / nin, i = pidx - o * nin;
-        float a = acc[q];
-        for (int r = 0; r < 32; ++r) a = fmaf(go[r][o], xi[r][i], a);
-        acc[q] = a;
+        for (int k = 0; k < 4; ++k) {
+          acc[k].x = fmaf(gg[k], xv.x, acc[k].x);
+          acc[k].y = fmaf(gg[k], xv.y, acc[k].y);
+          acc[k].z = fmaf(gg[k], xv.z, acc[k].z);
+          acc[k].w = fmaf(gg[k], xv.w, acc[k].w);
+        }
       }
-    }
-    if (t < nout)
-      for (int r = 0; r < 32; ++r) accb += go[r][t];
+    if (gb && sl < nsl)
+      for (int r = sl; r < 32; r += nsl) accb += go[r][ob];
   }
+  // the groups' sums meet in shared memory: one atomic per CTA and entry
+  __syncthreads();
+  float4* red = reinterpret_cast<float4*>(buf);  // [group][4][thread]
+  if (grp < groups)
 #pragma unroll
-  for (int q = 0; q < 16; ++q) {
-    const int pidx = t + q * 256;
-    if (pidx < pairs) atomicAdd(gW + pidx, acc[q]);
+    for (int k = 0; k < 4; ++k) red[(grp * 4 + k) * tpg + u] = acc[k];
+  __syncthreads();
+  for (int q = t; q < 4 * tpg; q += 256) {
+    const int k = q / tpg, v = q - k * tpg;
+    float4 s = red[k * tpg + v];
+    for (int g = 1; g < groups; ++g) {
+      const float4 w = red[(g * 4 + k) * tpg + v];
+      s = make_float4(s.x + w.x, s.y + w.y, s.z + w.z, s.w + w.w);
+    }
+    atomicAdd(reinterpret_cast<float4*>(gW + (size_t)(4 * (v / qi) + k) * nin + 4 * (v % qi)), s);
   }
-  if (t < nout && gb) atomicAdd(gb + t, accb);
+  if (gb && sl < nsl) atomicAdd(gb + ob, accb);
 }
 
-// dh_prev = dh + Ws^T g + Wn^T (sum of g over the face neighbours)
-__global__ void __launch_bounds__(256) k_bwd_layer_in(int64_t n, int K, const int4* __restrict__ nbr,
-                                                      const __nv_bfloat16* __restrict__ Ws,
-                                                      const __nv_bfloat16* __restrict__ Wn,
-                                                      const float* __restrict__ dh, const float* __restrict__ g,
-                                                      float* __restrict__ dhp) {
-  __shared__ float ws[kW][kW], wn[kW][kW];  // [channel c][input i]
-  __shared__ float gs[4][kW], Gs[4][kW];
-  const int t = threadIdx.x, el = t >> 6, i = t & 63;
-  for (int q = t; q < kW * kW; q += 256) {
-    ws[q / kW][q % kW] = bf(Ws[q]);
-    wn[q / kW][q % kW] = bf(Wn[q]);
-  }
-  for (int64_t g0 = (int64_t)blockIdx.x * 4; g0 < n; g0 += (int64_t)gridDim.x * 4) {
+// Weight gradients of one layer: g = dh (a > 0) (linear: dh), written to g_out;
+//   gWs += g^T h, gWn += g^T (sum of h over the face neighbours), gb += sum g.
+// A CTA of 128 threads takes 32-node chunks: g, h and the neighbour sums go to
+// shared memory (rows of 256 contiguous bytes), then a thread accumulates 8
+// outputs x 4 inputs of both matrices, 4 vector loads of shared memory per 64
+// FMAs.  One pass instead of five (mask, gather, two products, each re-reading
+// its operands; the products at one shared load per FMA): at 262144 nodes
+// 35 + 61 + 2 x 252 us -> 136 us.
+__global__ void __launch_bounds__(128) k_grad_layer(int64_t n, int K, const int4* __restrict__ nbr,
+                                                    const float* __restrict__ dh, const float* __restrict__ a,
+                                                    const float* __restrict__ h, float* __restrict__ g_out,
+                                                    float* __restrict__ gWs, float* __restrict__ gWn,
+                                                    float* __restrict__ gb, int linear) {
+  __shared__ __align__(16) float sg[32][kW], sx[32][2 * kW];
+  const int t = threadIdx.x, q = t & 15, r0 = t >> 4;  // loads: 4 channels, row of 8
+  const int o = 8 * (t >> 4), c = 4 * (t & 15);        // products: 8 outputs, 4 inputs of h and of the sums
+  float4 acc[8][2];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) acc[k][0] = acc[k][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 accb = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int64_t n0 = (int64_t)blockIdx.x * 32; n0 < n; n0 += (int64_t)gridDim.x * 32) {
     __syncthreads();
-    {
-      const int64_t e = g0 + el;
-      float gv = 0.0f, Gv = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = r0 + 8 * i;
+      const int64_t e = n0 + r;
+      float4 gv = z4, hv = z4, m[3] = {z4, z4, z4};
       if (e < n) {
-        gv = g[e * kW + i];
+        const size_t p = (size_t)e * kW + 4 * q;
+        gv = *reinterpret_cast<const float4*>(dh + p);
+        hv = __ldg(reinterpret_cast<const float4*>(h + p));
         int64_t j[3];
         neighbours(nbr, K, e, j);
 #pragma unroll
         for (int f = 0; f < 3; ++f)
-          if (j[f] >= 0) Gv += g[j[f] * kW + i];
+          if (j[f] >= 0) m[f] = __ldg(reinterpret_cast<const float4*>(h + j[f] * kW + 4 * q));
+        if (!linear) {
+          const float4 av = *reinterpret_cast<const float4*>(a + p);
+          gv = make_float4(av.x > 0.f ? gv.x : 0.f, av.y > 0.f ? gv.y : 0.f, av.z > 0.f ? gv.z : 0.f,
+                           av.w > 0.f ? gv.w : 0.f);
+        }
+        *reinterpret_cast<float4*>(g_out + p) = gv;
+        accb = make_float4(accb.x + gv.x, accb.y + gv.y, accb.z + gv.z, accb.w + gv.w);
       }
-      gs[el][i] = gv;
-      Gs[el][i] = Gv;
+      *reinterpret_cast<float4*>(&sg[r][4 * q]) = gv;
+      *reinterpret_cast<float4*>(&sx[r][4 * q]) = hv;
+      *reinterpret_cast<float4*>(&sx[r][kW + 4 * q]) =
+          make_float4((m[0].x + m[1].x) + m[2].x, (m[0].y + m[1].y) + m[2].y, (m[0].z + m[1].z) + m[2].z,
+                      (m[0].w + m[1].w) + m[2].w);
     }
     __syncthreads();
-    const int64_t e = g0 + el;
-    if (e < n) {
-      float a = dh[e * kW + i];
-#pragma unroll 8
-      for (int c = 0; c < kW; ++c) a = fmaf(ws[c][i], gs[el][c], fmaf(wn[c][i], Gs[el][c], a));
-      dhp[e * kW + i] = a;
+#pragma unroll 4
+    for (int r = 0; r < 32; ++r) {
+      const float4 g0 = *reinterpret_cast<const float4*>(&sg[r][o]), g1 = *reinterpret_cast<const float4*>(&sg[r][o + 4]);
+      const float4 x0 = *reinterpret_cast<const float4*>(&sx[r][c]), x1 = *reinterpret_cast<const float4*>(&sx[r][kW + c]);
+      const float gg[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        acc[k][0].x = fmaf(gg[k], x0.x, acc[k][0].x);
+        acc[k][0].y = fmaf(gg[k], x0.y, acc[k][0].y);
+        acc[k][0].z = fmaf(gg[k], x0.z, acc[k][0].z);
+        acc[k][0].w = fmaf(gg[k], x0.w, acc[k][0].w);
+        acc[k][1].x = fmaf(gg[k], x1.x, acc[k][1].x);
+        acc[k][1].y = fmaf(gg[k], x1.y, acc[k][1].y);
+        acc[k][1].z = fmaf(gg[k], x1.z, acc[k][1].z);
+        acc[k][1].w = fmaf(gg[k], x1.w, acc[k][1].w);
+      }
     }
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    atomicAdd(reinterpret_cast<float4*>(gWs + (o + k) * kW + c), acc[k][0]);
+    atomicAdd(reinterpret_cast<float4*>(gWn + (o + k) * kW + c), acc[k][1]);
+  }
+  __syncthreads();
+  *reinterpret_cast<float4*>(&sg[r0][4 * q]) = accb;
+  __syncthreads();
+  if (t < kW) {
+    float v = 0.0f;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) v += sg[r][t];
+    atomicAdd(gb + t, v);
   }
 }
 
@@ -453,7 +547,7 @@ struct dgc_mpnn_s {
   int cap = 0;
   std::vector<float*> hs;        // h_0 .. h_L  [S K W]
   std::vector<float*> as;        // a_1 .. a_L  [S K W]
-  float *y = nullptr, *dy = nullptr, *dh0 = nullptr, *dh1 = nullptr, *g = nullptr, *m = nullptr;
+  float *y = nullptr, *dy = nullptr, *dh0 = nullptr, *dh1 = nullptr, *g = nullptr;
   float *sd = nullptr, *tm = nullptr, *st = nullptr;  // energy loss: S d, masked t, S t
   int loss_kind = DGC_MPNN_LOSS_ENERGY;
   int linear = 0;                // DGC_MPNN_ACT_LINEAR: no ReLU, biases held at zero
@@ -527,7 +621,7 @@ int ensure_train(dgc_mpnn m, int S) {
   auto fr = [](float*& p) { cudaFree(p); p = nullptr; };
   for (auto& p : m->hs) fr(p);
   for (auto& p : m->as) fr(p);
-  fr(m->y); fr(m->dy); fr(m->dh0); fr(m->dh1); fr(m->g); fr(m->m);
+  fr(m->y); fr(m->dy); fr(m->dh0); fr(m->dh1); fr(m->g);
   fr(m->sd); fr(m->tm); fr(m->st);
   const size_t nW = (size_t)S * m->h->K * dgk::kW, nY = (size_t)S * field_len(m);
   m->hs.assign(m->lay.L + 1, nullptr);
@@ -539,7 +633,6 @@ int ensure_train(dgc_mpnn m, int S) {
   CKM(zalloc(&m->dh0, nW));
   CKM(zalloc(&m->dh1, nW));
   CKM(zalloc(&m->g, nW));
-  CKM(zalloc(&m->m, nW));
   CKM(zalloc(&m->sd, nY));
   CKM(zalloc(&m->tm, nY));
   CKM(zalloc(&m->st, nY));
@@ -570,27 +663,28 @@ int ensure_fcg(dgc_mpnn m, int window) {
   return ensure_scal(m, dgk::kMaxDots);
 }
 
+// tensor-core layer (mpnn_tc.cuh): persistent CTAs over 128-node tiles, 2 per SM
+int layer_grid(const dgc_mpnn_s* m, int64_t n) {
+  return (int)std::min<int64_t>((n + dgk::MpnnTc::kRows - 1) / dgk::MpnnTc::kRows, (int64_t)m->sm_count * 2);
+}
+
 // forward over n graph nodes; h ping-pong through (ha, hb) or the stored layers
 int forward(dgc_mpnn m, int64_t n, const float* x, float* y, float* ha, float* hb, bool store, cudaStream_t s) {
   const auto& L = m->lay;
   const int4* nbr = reinterpret_cast<const int4*>(m->h->d_nbr);
   const int K = m->h->K;
   float* cur = store ? m->hs[0] : ha;
-  dgk::k_fwd_in<<<grid_for(m, n, 4), 256, 0, s>>>(n, L.npi, m->w16 + L.oWin, m->w16 + L.obin, x, cur);
+  dgk::k_to_features<false><<<grid_for(m, n, 64), 256, 0, s>>>(n, L.npi, m->w16 + L.oWin, m->w16 + L.obin, x, cur);
   CKM(cudaGetLastError());
   for (int l = 0; l < L.L; ++l) {
     float* nxt = store ? m->hs[l + 1] : (cur == ha ? hb : ha);
-    // tensor-core layer (mpnn_tc.cuh): persistent CTAs over 128-node tiles, 2 per SM
-    const int tiles = (int)std::min<int64_t>((n + dgk::MpnnTc::kRows - 1) / dgk::MpnnTc::kRows,
-                                             (int64_t)m->sm_count * 2);
-    dgk::k_fwd_layer_tc<<<tiles, dgk::MpnnTc::kThreads, dgk::MpnnTc::kSmem, s>>>(
-        n, K, nbr, m->w16 + L.oWs(l), m->w16 + L.oWn(l), m->w16 + L.ob(l), cur, store ? m->as[l] : nullptr, nxt,
-        m->linear, m->h->d_status);
+    dgk::k_layer_tc<false><<<layer_grid(m, n), dgk::MpnnTc::kThreads, dgk::MpnnTc::kSmem, s>>>(
+        n, K, nbr, m->w16 + L.oWs(l), m->w16 + L.oWn(l), m->w16 + L.ob(l), cur, nullptr,
+        store ? m->as[l] : nullptr, nxt, m->linear, m->h->d_status);
     CKM(cudaGetLastError());
     cur = nxt;
   }
-  const int per = std::min(256 / L.npi, 16);
-  dgk::k_fwd_out<<<grid_for(m, n, per), 256, 0, s>>>(n, L.npi, m->w16 + L.oWout, m->w16 + L.obout, cur, y);
+  dgk::k_fwd_out<<<grid_for(m, n, 64), 256, 0, s>>>(n, L.npi, m->w16 + L.oWout, m->w16 + L.obout, cur, y);
   CKM(cudaGetLastError());
   m->h->launches += L.L + 2;
   return DGC_OK;
@@ -702,7 +796,9 @@ extern "C" int dgc_mpnn_create(dgc_handle h, int layers, uint64_t seed, dgc_mpnn
   if (e == cudaSuccess) e = cudaMemset(m->av, 0, P * 4);
   if (e != cudaSuccess) return fail(mcuda(e, "mpnn set-up"));
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(dgk::k_fwd_layer_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, dgk::MpnnTc::kSmem);
+    e = cudaFuncSetAttribute(dgk::k_layer_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, dgk::MpnnTc::kSmem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(dgk::k_layer_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dgk::MpnnTc::kSmem);
   if (e != cudaSuccess) return fail(mcuda(e, "mpnn set-up"));
   dgk::k_to_bf16<<<grid_for(m, P, 256), 256>>>(P, m->w, m->w16);
   if ((e = cudaGetLastError()) != cudaSuccess) return fail(mcuda(e, "mpnn set-up"));
@@ -712,7 +808,7 @@ extern "C" int dgc_mpnn_create(dgc_handle h, int layers, uint64_t seed, dgc_mpnn
 
 extern "C" int dgc_mpnn_destroy(dgc_mpnn m) {
   if (!m) return DGC_OK;
-  for (float* p : {m->w, m->grad, m->am, m->av, m->y, m->dy, m->dh0, m->dh1, m->g, m->m, m->sd, m->tm, m->st,
+  for (float* p : {m->w, m->grad, m->am, m->av, m->y, m->dy, m->dh0, m->dh1, m->g, m->sd, m->tm, m->st,
                    m->px, m->ph0, m->ph1,
                    m->py, m->pt})
     cudaFree(p);
@@ -828,35 +924,32 @@ extern "C" int dgc_mpnn_train_step(dgc_mpnn m, const float* x, const float* t, i
       if (int rc = dgc::ipdg_spd_apply_f32(m->h, m->tm + j * f, m->st + j * f, s)) return rc;
     }
     double* dots = m->scal + 1 + S;
-    dgk::k_energy_dots<<<dim3(grid_for(m, f, 256), S), 256, 0, s>>>(K, npi, np, m->dy, m->sd, m->tm, m->st, dots);
-    dgk::k_energy_grad<<<grid_for(m, n * npi, 256), 256, 0, s>>>(n * npi, K, npi, np, S, m->sd, dots, m->dy,
-                                                                 m->scal);
+    const int per = (int)std::max<int64_t>(1, std::min<int64_t>((f + 255) / 256, (4 * m->sm_count + S - 1) / S));
+    dgk::k_energy_dots<<<dim3(per, S), 256, 0, s>>>(f, m->dy, m->sd, m->tm, m->st, dots);
+    dgk::k_energy_grad<<<dim3(2 * per, S), 256, 0, s>>>(f, npi, np, S, m->sd, dots, m->dy, m->scal);
     CKM(cudaGetLastError());
     m->h->launches += 3;
   }
   // backward
   CKM(cudaMemsetAsync(m->grad, 0, L.total * 4, s));
-  dgk::k_grad_dense<<<grid_for(m, n, 32), 256, 0, s>>>(n, npi, dgk::kW, m->dy, m->hs[L.L], m->grad + L.oWout,
-                                                       m->grad + L.obout);
-  dgk::k_bwd_out<<<grid_for(m, n, 4), 256, 0, s>>>(n, npi, m->w16 + L.oWout, m->dy, m->dh0);
+  // reductions over the nodes end in one atomic per CTA and gradient entry: 4 CTAs per SM
+  const int gg = (int)std::max<int64_t>(1, std::min<int64_t>((n + 31) / 32, (int64_t)m->sm_count * 4));
+  dgk::k_grad_dense<<<gg, 256, 0, s>>>(n, npi, dgk::kW, m->dy, m->hs[L.L], m->grad + L.oWout, m->grad + L.obout);
+  dgk::k_to_features<true><<<grid_for(m, n, 64), 256, 0, s>>>(n, npi, m->w16 + L.oWout, nullptr, m->dy, m->dh0);
   CKM(cudaGetLastError());
   float* dh = m->dh0;
   float* dhp = m->dh1;
   for (int l = L.L - 1; l >= 0; --l) {
-    dgk::k_relu_bwd<<<grid_for(m, n * dgk::kW, 256), 256, 0, s>>>(n * dgk::kW, dh, m->as[l], m->g, m->linear);
-    dgk::k_grad_dense<<<grid_for(m, n, 32), 256, 0, s>>>(n, dgk::kW, dgk::kW, m->g, m->hs[l], m->grad + L.oWs(l),
-                                                         m->grad + L.ob(l));
-    dgk::k_gather<<<grid_for(m, n * dgk::kW, 256), 256, 0, s>>>(n, K, nbr, m->hs[l], m->m);
-    dgk::k_grad_dense<<<grid_for(m, n, 32), 256, 0, s>>>(n, dgk::kW, dgk::kW, m->g, m->m, m->grad + L.oWn(l),
-                                                         nullptr);
-    dgk::k_bwd_layer_in<<<grid_for(m, n, 4), 256, 0, s>>>(n, K, nbr, m->w16 + L.oWs(l), m->w16 + L.oWn(l), dh,
-                                                          m->g, dhp);
+    dgk::k_grad_layer<<<gg, 128, 0, s>>>(n, K, nbr, dh, m->as[l], m->hs[l], m->g, m->grad + L.oWs(l),
+                                         m->grad + L.oWn(l), m->grad + L.ob(l), m->linear);
+    dgk::k_layer_tc<true><<<layer_grid(m, n), dgk::MpnnTc::kThreads, dgk::MpnnTc::kSmem, s>>>(
+        n, K, nbr, m->w16 + L.oWs(l), m->w16 + L.oWn(l), nullptr, m->g, dh, nullptr, dhp, m->linear, m->h->d_status);
     CKM(cudaGetLastError());
     std::swap(dh, dhp);
   }
-  dgk::k_grad_dense<<<grid_for(m, n, 32), 256, 0, s>>>(n, dgk::kW, npi, dh, x, m->grad + L.oWin, m->grad + L.obin);
+  dgk::k_grad_dense<<<gg, 256, 0, s>>>(n, dgk::kW, npi, dh, x, m->grad + L.oWin, m->grad + L.obin);
   CKM(cudaGetLastError());
-  m->h->launches += 3 + 5 * L.L;  // output grads, 5 per layer, input grads
+  m->h->launches += 3 + 2 * L.L;  // output grads, 2 per layer, input grads
   if (m->linear) {  // the biases stay at zero: the network remains a linear map
     if (int rc = zero_biases(m, m->grad, s)) return rc;
   }

@@ -7,27 +7,31 @@
 // i.e. for a tile of 128 nodes the product D[128 x 64] = X[128 x 128] W^T with
 // X = [h | m] (FP32) and W = [Ws | Wn] (64 x 128, BF16 copies of the FP32
 // master weights).  W is exact in BF16; X is not, so X is split into three
-// BF16 parts X = X0 + X1 + X2 (each the BF16 rounding of what the previous
+// BF16 parts X = X0 + X1 + X2 (each the leading bits of what the previous
 // parts leave; 3 x 8 significand bits cover FP32's 24) and the tile is three
 // accumulating products per K step.  The result matches the FP32 SIMT form of
 // the same layer to FP32 accumulation round-off.
+//
+// The backward pass through the layer's input has the same form,
+//   dh_e <- dh_e + Ws^T g_e + Wn^T (sum of g over the face neighbours),
+// with X = [g | sum g] and the transposed weights.
 //
 // CTA: 256 threads, one 128-node tile at a time (persistent over tiles).
 //   * W is staged once per CTA in shared memory (K-major, no swizzle, core
 //     matrices of 8 rows x 16 bytes: element (row, k) at byte
 //     (row / 8) * 2048 + (k / 8) * 128 + (row % 8) * 16 + (k % 8) * 2);
-//   * two threads per tile row gather h_e and the neighbour rows (float4
-//     loads, two 8-channel chunks in flight at a time), sum, split and store
-//     the three X parts in the same layout;
-//   * one thread issues 8 K steps x 3 MMAs (M = 128, N = 64, K = 16) into 64
-//     TMEM columns and commits to an mbarrier (bounded wait);
-//   * the epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31 (its rows),
-//     columns 32 (w / 4) .. + 31, adds the bias, writes a (optional) and h'.
-// Shared memory 112 KB + barriers: 2 CTAs per SM; TMEM 64 columns per CTA.
-// (Forming the neighbour sums in a separate gather kernel first, so that this
-// kernel reads two contiguous rows per node, was measured: 22.5 us for this
-// kernel plus the gather, 6 % slower per network application than the fused
-// gather here.)
+//   * a warp gathers 16 rows: 8 rows x 64 contiguous bytes per load instruction
+//     (with a thread per row every load touched 32 lines: 187 us per layer at
+//     262144 nodes, 73 us with this mapping and the epilogue below), 16 loads in
+//     flight per thread;
+//     the split is by truncation (exact: 8 + 8 + 8 bits, no conversions);
+//   * one thread issues 3 parts x 8 K steps of MMAs (M = 128, N = 64, K = 16) into
+//     64 TMEM columns and commits to an mbarrier (bounded wait);
+//   * the epilogue moves D through the (now free) operand tile so that bias,
+//     activation and the global accesses run on whole 256-byte rows.  The
+//     backward form replaces an FP32 SIMT kernel (400 us at 262144 nodes, 86 us).
+// Bound by DRAM and the gather's L2 traffic.  Shared memory 112 KB + barriers:
+// 2 CTAs per SM, one gathering while the other multiplies; TMEM 64 columns each.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -50,16 +54,17 @@ struct MpnnTc {
   static constexpr uint32_t oA = oB + kBBytes;
   static constexpr uint32_t kSmem = oA + 3 * kABytes;
   static constexpr uint32_t kTmemCols = 64;
+  static constexpr int kDStr = kN + 4;              // floats between rows of the staged D
   // instruction descriptor: D f32 (bits 4-5 = 1), A and B bf16 (bits 7-9, 10-12 = 1),
   // both K-major, N >> 3 at bit 17, M >> 4 at bit 24
   static constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kN >> 3) << 17) |
                                      ((uint32_t)(kRows >> 4) << 24);
-  static_assert(kSmem % 16 == 0 && oA % 128 == 0, "operand alignment");
+  static_assert(kSmem % 16 == 0 && oA % 128 == 0 && kRows * kDStr * 4 <= 3 * kABytes, "operand alignment");
 };
 
 // face neighbours of graph node e (sample s = e / K): up to 3 node indices, -1 on the boundary
 __device__ __forceinline__ void neighbours(const int4* __restrict__ nbr, int K, int64_t e, int64_t (&j)[3]) {
-  const int64_t s = e / K;
+  const int64_t s = e <= 0x7fffffff ? (int64_t)((uint32_t)e / (uint32_t)K) : e / K;
   const int4 n4 = __ldg(nbr + (e - s * K));
   const int c[3] = {n4.x, n4.y, n4.z};
 #pragma unroll
@@ -79,36 +84,42 @@ __device__ __forceinline__ void tc_mma_bf16(uint32_t d_tmem, uint64_t a_desc, ui
       : "memory");
 }
 
-// eight FP32 values -> three 16-byte rows of BF16 parts (x = p0 + p1 + p2)
-__device__ __forceinline__ void split3_store(const float (&v)[8], unsigned char* a0, unsigned char* a1,
-                                             unsigned char* a2) {
-  __align__(16) __nv_bfloat16 p[3][8];
+// four FP32 values -> three 8-byte rows of BF16 parts, x = p0 + p1 + p2 exactly:
+// each part is the leading 8 significand bits of what the previous ones leave
+// (infinities and NaN come out as NaN)
+__device__ __forceinline__ void split3_store(const float4& x, unsigned char* a0) {
+  const float v[4] = {x.x, x.y, x.z, x.w};
+  uint32_t w[3][4];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const __nv_bfloat16 b0 = __float2bfloat16_rn(v[i]);
-    const float r1 = v[i] - __bfloat162float(b0);
-    const __nv_bfloat16 b1 = __float2bfloat16_rn(r1);
-    const float r2 = r1 - __bfloat162float(b1);
-    p[0][i] = b0;
-    p[1][i] = b1;
-    p[2][i] = __float2bfloat16_rn(r2);
+  for (int i = 0; i < 4; ++i) {
+    float r = v[i];
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+      w[p][i] = __float_as_uint(r) & 0xffff0000u;
+      if (p < 2) r -= __uint_as_float(w[p][i]);
+    }
   }
-  *reinterpret_cast<uint4*>(a0) = *reinterpret_cast<const uint4*>(p[0]);
-  *reinterpret_cast<uint4*>(a1) = *reinterpret_cast<const uint4*>(p[1]);
-  *reinterpret_cast<uint4*>(a2) = *reinterpret_cast<const uint4*>(p[2]);
+#pragma unroll
+  for (int p = 0; p < 3; ++p)
+    *reinterpret_cast<uint2*>(a0 + p * MpnnTc::kABytes) =
+        make_uint2(__byte_perm(w[p][0], w[p][1], 0x7632), __byte_perm(w[p][2], w[p][3], 0x7632));
 }
 
+// BWD false: a_out (may be NULL) = W X + b, out = x + relu(a) (linear: x + a), x = the tile's own rows.
+// BWD true:  out = add + W^T X.
+template <bool BWD>
 __global__ void __launch_bounds__(MpnnTc::kThreads, 2)
-    k_fwd_layer_tc(int64_t n, int K, const int4* __restrict__ nbr, const __nv_bfloat16* __restrict__ Ws,
-                   const __nv_bfloat16* __restrict__ Wn, const __nv_bfloat16* __restrict__ bl,
-                   const float* __restrict__ h, float* __restrict__ a_out, float* __restrict__ hn,
-                   int linear, int* __restrict__ status) {
+    k_layer_tc(int64_t n, int K, const int4* __restrict__ nbr, const __nv_bfloat16* __restrict__ Ws,
+               const __nv_bfloat16* __restrict__ Wn, const __nv_bfloat16* __restrict__ bl,
+               const float* __restrict__ x, const float* __restrict__ add, float* __restrict__ a_out,
+               float* __restrict__ out, int linear, int* __restrict__ status) {
   using C = MpnnTc;
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + C::oBar);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::oBar + 8);
   unsigned char* sB = smem + C::oB;
   unsigned char* sA = smem + C::oA;
+  float* sD = reinterpret_cast<float*>(sA);  // [row][kDStr], after the products
   float* sBias = reinterpret_cast<float*>(smem + C::oBias);
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
 
@@ -117,73 +128,60 @@ __global__ void __launch_bounds__(MpnnTc::kThreads, 2)
     fence_barrier_init();
   }
   if (warp == 0) tmem_alloc_n(tmem_slot, C::kTmemCols);
-  // W: row c = output channel, k < 64 from Ws[c][k], k >= 64 from Wn[c][k - 64];
-  // 16-byte chunks of 8 consecutive k
-  for (int q = t; q < C::kN * (C::kK / 8); q += C::kThreads) {
-    const int c = q / (C::kK / 8), k0 = (q % (C::kK / 8)) * 8;
-    const __nv_bfloat16* src = (k0 < C::kN ? Ws + c * C::kN + k0 : Wn + c * C::kN + (k0 - C::kN));
-    *reinterpret_cast<uint4*>(sB + tc_off(c, k0)) = *reinterpret_cast<const uint4*>(src);
+  if (BWD) {
+    // row i = input channel, column c (Ws) or 64 + c (Wn) = output channel
+    for (int q = t; q < 2 * C::kN * C::kN; q += C::kThreads) {
+      const int k = q / C::kN, i = q % C::kN;
+      *reinterpret_cast<__nv_bfloat16*>(sB + tc_off(i, k)) = k < C::kN ? Ws[k * C::kN + i] : Wn[(k - C::kN) * C::kN + i];
+    }
+  } else {
+    // row c = output channel, k < 64 from Ws[c][k], k >= 64 from Wn[c][k - 64];
+    // 16-byte chunks of 8 consecutive k
+    for (int q = t; q < C::kN * (C::kK / 8); q += C::kThreads) {
+      const int c = q / (C::kK / 8), k0 = (q % (C::kK / 8)) * 8;
+      const __nv_bfloat16* src = (k0 < C::kN ? Ws + c * C::kN + k0 : Wn + c * C::kN + (k0 - C::kN));
+      *reinterpret_cast<uint4*>(sB + tc_off(c, k0)) = *reinterpret_cast<const uint4*>(src);
+    }
+    if (t < C::kN) sBias[t] = __bfloat162float(bl[t]);
   }
-  if (t < C::kN) sBias[t] = __bfloat162float(bl[t]);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t sA_u = smem_u32(sA), sB_u = smem_u32(sB);
-  // thread t fills row t % 128, channel chunks (t / 128) * 4 .. + 3 of h and of m
-  const int row = t & 127, half = t >> 7;
-  // epilogue: rows of the warp's lane quadrant, its half of the channels
-  const int erow = (warp & 3) * 32 + lane, ecol = (warp >> 2) * 32;
+  const int lrow = lane >> 2, lq = lane & 3;  // gather: row within 8, 4-channel quad within 4
+  const int erow = (warp & 3) * 32 + lane, ecol = (warp >> 2) * 32;  // TMEM lanes and columns of the epilogue
   uint32_t phase = 0;
   bool ok = true;
   for (int64_t n0 = (int64_t)blockIdx.x * C::kRows; n0 < n && ok; n0 += (int64_t)gridDim.x * C::kRows) {
-    // ---- X = [h | m] of the tile, split into three BF16 parts
-    {
-      const int64_t e = n0 + row;
-      int64_t j[3] = {-1, -1, -1};
-      if (e < n) neighbours(nbr, K, e, j);
-      // two chunks of 8 channels at a time, every load of both issued before use
+    // ---- X = [x | sum of x over the neighbours], split into three BF16 parts
 #pragma unroll 1
-      for (int cp = 0; cp < 2; ++cp) {
-        float4 hl[2][2], ml[2][3][2];
+    for (int hh = 0; hh < 2; ++hh) {
+      const int row = warp * 16 + hh * 8 + lrow;
+      const int64_t e = n0 + row;
+      int64_t j[4] = {-1, -1, -1, -1};
+      if (e < n) {
+        int64_t nb[3];
+        neighbours(nbr, K, e, nb);
+        j[0] = e;
+        j[1] = nb[0];
+        j[2] = nb[1];
+        j[3] = nb[2];
+      }
+      float4 v[4][4];
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int c0 = (half * 4 + cp * 2 + u) * 8;  // channels c0 .. c0 + 7
-          const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-          hl[u][0] = hl[u][1] = z4;
-          if (e < n) {
-            const float4* hp = reinterpret_cast<const float4*>(h + e * C::kN + c0);
-            hl[u][0] = hp[0];
-            hl[u][1] = hp[1];
-          }
+      for (int f = 0; f < 4; ++f) {
+        const float4* src = reinterpret_cast<const float4*>(x + j[f] * C::kN) + lq;
 #pragma unroll
-          for (int f = 0; f < 3; ++f) {
-            ml[u][f][0] = ml[u][f][1] = z4;
-            if (j[f] >= 0) {
-              const float4* mp = reinterpret_cast<const float4*>(h + j[f] * C::kN + c0);
-              ml[u][f][0] = mp[0];
-              ml[u][f][1] = mp[1];
-            }
-          }
-        }
+        for (int u = 0; u < 4; ++u) v[f][u] = j[f] >= 0 ? __ldg(src + 4 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int c0 = (half * 4 + cp * 2 + u) * 8;
-          const float hv[8] = {hl[u][0].x, hl[u][0].y, hl[u][0].z, hl[u][0].w,
-                               hl[u][1].x, hl[u][1].y, hl[u][1].z, hl[u][1].w};
-          float mv[8];
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            mv[4 * q] = (ml[u][0][q].x + ml[u][1][q].x) + ml[u][2][q].x;
-            mv[4 * q + 1] = (ml[u][0][q].y + ml[u][1][q].y) + ml[u][2][q].y;
-            mv[4 * q + 2] = (ml[u][0][q].z + ml[u][1][q].z) + ml[u][2][q].z;
-            mv[4 * q + 3] = (ml[u][0][q].w + ml[u][1][q].w) + ml[u][2][q].w;
-          }
-          split3_store(hv, sA + tc_off(row, c0), sA + C::kABytes + tc_off(row, c0),
-                       sA + 2 * C::kABytes + tc_off(row, c0));
-          split3_store(mv, sA + tc_off(row, C::kN + c0), sA + C::kABytes + tc_off(row, C::kN + c0),
-                       sA + 2 * C::kABytes + tc_off(row, C::kN + c0));
-        }
+      for (int u = 0; u < 4; ++u) {
+        const int k = 4 * (lq + 4 * u);
+        split3_store(v[0][u], sA + tc_off(row, k));
+        const float4 m = make_float4((v[1][u].x + v[2][u].x) + v[3][u].x, (v[1][u].y + v[2][u].y) + v[3][u].y,
+                                     (v[1][u].z + v[2][u].z) + v[3][u].z, (v[1][u].w + v[2][u].w) + v[3][u].w);
+        split3_store(m, sA + tc_off(row, C::kN + k));
       }
     }
     // generic-proxy stores of X -> visible to the tensor core's async proxy
@@ -192,15 +190,17 @@ __global__ void __launch_bounds__(MpnnTc::kThreads, 2)
     __syncthreads();
     tc_fence_after();
     if (t == 0) {
+      // the small parts first, so that only the leading part's 8 steps round at full
+      // magnitude (gradient error against 64 bits at K = 32768, 8 samples: 2.6e-6
+      // part by part within each step, 0.7-1.1e-6 so; an FP32 SIMT layer 1.2-2.1e-6)
 #pragma unroll
-      for (int s = 0; s < C::kK / 16; ++s) {
-        const uint64_t db = smem_desc(sB_u + s * 256, 128, C::kSbo);
+      for (int p = 2; p >= 0; --p)
 #pragma unroll
-        for (int p = 0; p < 3; ++p) {
+        for (int s = 0; s < C::kK / 16; ++s) {
+          const uint64_t db = smem_desc(sB_u + s * 256, 128, C::kSbo);
           const uint64_t da = smem_desc(sA_u + p * C::kABytes + s * 256, 128, C::kSbo);
-          tc_mma_bf16(tmem, da, db, C::kIdesc, (s > 0 || p > 0) ? 1u : 0u);
+          tc_mma_bf16(tmem, da, db, C::kIdesc, (s > 0 || p < 2) ? 1u : 0u);
         }
-      }
       tc_commit(bar);
     }
     ok = __syncthreads_and(mbar_wait(bar, phase, status));
@@ -212,30 +212,41 @@ __global__ void __launch_bounds__(MpnnTc::kThreads, 2)
     }
     phase ^= 1;
     tc_fence_after();
-    // ---- epilogue
+    // ---- epilogue: D to shared memory (the operand tile has been consumed),
+    //      then by whole rows
     {
-      float v[32];
-      tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + ecol, v);
-      const int64_t e = n0 + erow;
-      if (e < n) {
+      float d[32];
+      tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + ecol, d);
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const float4 bq = *reinterpret_cast<const float4*>(sBias + ecol + 4 * q);
-          const float4 a = make_float4(v[4 * q] + bq.x, v[4 * q + 1] + bq.y, v[4 * q + 2] + bq.z,
-                                       v[4 * q + 3] + bq.w);
-          if (a_out) *reinterpret_cast<float4*>(a_out + e * C::kN + ecol + 4 * q) = a;
-          const float4 hh = *reinterpret_cast<const float4*>(h + e * C::kN + ecol + 4 * q);
-          *reinterpret_cast<float4*>(hn + e * C::kN + ecol + 4 * q) =
-              linear ? make_float4(hh.x + a.x, hh.y + a.y, hh.z + a.z, hh.w + a.w)
-                     : make_float4(hh.x + fmaxf(a.x, 0.f), hh.y + fmaxf(a.y, 0.f), hh.z + fmaxf(a.z, 0.f),
-                                   hh.w + fmaxf(a.w, 0.f));
-        }
-      }
+      for (int q = 0; q < 8; ++q)
+        *reinterpret_cast<float4*>(sD + erow * C::kDStr + ecol + 4 * q) =
+            make_float4(d[4 * q], d[4 * q + 1], d[4 * q + 2], d[4 * q + 3]);
     }
-    // TMEM read and the tile's shared rows consumed before the next tile overwrites them
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+#pragma unroll
+    for (int i = 0; i < C::kRows * 16 / C::kThreads; ++i) {
+      const int row = (t >> 4) + 16 * i, c = 4 * (t & 15);
+      const int64_t e = n0 + row;
+      if (e >= n) break;
+      const size_t o = (size_t)e * C::kN + c;
+      const float4 d = *reinterpret_cast<const float4*>(sD + row * C::kDStr + c);
+      if (BWD) {
+        const float4 b = *reinterpret_cast<const float4*>(add + o);
+        *reinterpret_cast<float4*>(out + o) = make_float4(b.x + d.x, b.y + d.y, b.z + d.z, b.w + d.w);
+      } else {
+        const float4 bq = *reinterpret_cast<const float4*>(sBias + c);
+        const float4 a = make_float4(d.x + bq.x, d.y + bq.y, d.z + bq.z, d.w + bq.w);
+        if (a_out) *reinterpret_cast<float4*>(a_out + o) = a;
+        const float4 hh = __ldg(reinterpret_cast<const float4*>(x + o));
+        *reinterpret_cast<float4*>(out + o) =
+            linear ? make_float4(hh.x + a.x, hh.y + a.y, hh.z + a.z, hh.w + a.w)
+                   : make_float4(hh.x + fmaxf(a.x, 0.f), hh.y + fmaxf(a.y, 0.f), hh.z + fmaxf(a.z, 0.f),
+                                 hh.w + fmaxf(a.w, 0.f));
+      }
+    }
+    __syncthreads();  // the tile's shared rows consumed before the next tile overwrites them
   }
   tc_fence_before();
   __syncthreads();
