@@ -17,7 +17,7 @@
 //     operations per face node instead of 15.
 // About 3.3k FP64 instructions per element instead of 7.4k.
 //
-// A CTA takes one tile of `te` elements (at most 256 / Np, see eo_tile).  One
+// A CTA takes one tile of at most 256 / Np elements (see eo_pick_tiles).  One
 // CTA per tile lets the hardware hand out tiles as SMs become free; persistent
 // CTAs, with their fixed share of tiles, took 206.9 instead of 203.5 us per stage
 // at K = 32768, N = 6 and 28.4 instead of 27.0 us at K = 8192, N = 4 (Maxwell TE).
@@ -79,18 +79,18 @@ enum EoConst : int {
   EC_Y = 10,             // Maxwell, faces 0..2: -sg H ny
 };
 
-// elements per tile of the stage kernel, from its FP64 instructions per row,
+// tiles of the stage kernel, from its FP64 instructions per row,
 // flux, input and constant item
 template <typename R, int N, int P>
-inline int eo_tile(int K, int sm_count) {
+inline int eo_tiles(int K, int sm_count) {
   using C = EoConfig<R, N, P>;
   constexpr bool adv = P == PHYS_ADV;
-  return eo_pick_tile(C::D, K, sm_count, C::TE,
-                      adv ? EoCost{C::Np + C::fE + 7, 5, 2, 6} : EoCost{2 * C::Np + 3 * C::fE + 14, 24, 14, 10});
+  return eo_pick_tiles(C::D, K, sm_count, C::TE,
+                       adv ? EoCost{C::Np + C::fE + 7, 5, 2, 6} : EoCost{2 * C::Np + 3 * C::fE + 14, 24, 14, 10});
 }
 
 template <typename R, int N, int P>
-__global__ void __launch_bounds__(256) dg_rhs_eo_kernel(const RhsParams p, const int te) {
+__global__ void __launch_bounds__(256) dg_rhs_eo_kernel(const RhsParams p) {
   using C = EoConfig<R, N, P>;
   constexpr int Np = C::Np, NpP = C::NpP, Nfp = C::Nfp, NF = C::Nf, ESTR = C::ESTR;
   constexpr int nE = C::nE, nO = C::nO, fE = C::fE, fO = C::fO;
@@ -120,7 +120,8 @@ __global__ void __launch_bounds__(256) dg_rhs_eo_kernel(const RhsParams p, const
   R* q0 = static_cast<R*>(p.q0);
   const R cca = (R)p.ca, ccb = (R)p.cb;
   const R scale = p.mode == MODE_LSERK ? (R)p.dt : (R)1;
-  const int k0 = blockIdx.x * te, ne = min(te, p.K - k0);
+  const TileCut tiles(p.K, gridDim.x);
+  const int k0 = tiles.start(blockIdx.x), ne = tiles.size(blockIdx.x);
   if (tid == 0) {
     s_nbnd = 0;
     mbar_init(&bar[0], 1);

@@ -55,15 +55,17 @@ struct EoCost {
   int row, flux, in, cst;
 };
 
-// Elements per tile (one CTA of 256 threads each): the size with the least FP64
-// work on the busiest SM, in warp instructions.  A tile costs its phases' warps
-// times their instructions (a partly filled warp costs a full one) plus a fixed
-// share for its barriers and copies; an SM gets ceil(tiles / SMs) of them.  The
-// model follows the measured times within 5 % over tile sizes: stage kernel,
+// Number of tiles (one CTA of 256 threads each, at most te_max elements, cut
+// evenly, TileCut): the tile size with the least
+// FP64 work on the busiest SM, in warp instructions.  A tile costs its phases'
+// warps times their instructions (a partly filled warp costs a full one) plus a
+// fixed share for its barriers and copies; an SM gets ceil(tiles / SMs) of them.
+// The model follows the measured times within 5 % over tile sizes: stage kernel,
 // Maxwell TE, K = 2048, N = 6: 17.3 us at the 7 or 8 elements it picks against
 // 20.1 at the largest tile (9), 18.3 at 5 and 22.5 at 4; K = 8192, N = 4: 27.0 us
-// at 14 against 31.3 at 17 and 31.3 at 8.
-inline int eo_pick_tile(const EoDims& d, int K, int sm_count, int te_max, const EoCost& w) {
+// at 14 against 31.3 at 17 and 31.3 at 8.  Where one tile per SM is enough, every
+// SM gets one (an SM left out draws several CTAs of an overlapped next launch).
+inline int eo_pick_tiles(const EoDims& d, int K, int sm_count, int te_max, const EoCost& w) {
   auto warps = [](int lanes) { return (lanes + 31) / 32; };
   int best = 1;
   long long cost = -1;
@@ -73,11 +75,19 @@ inline int eo_pick_tile(const EoDims& d, int K, int sm_count, int te_max, const 
     const long long c = (long long)(((K + te - 1) / te + sm_count - 1) / sm_count) * tile;
     if (cost < 0 || c < cost) {
       cost = c;
-      best = te;
+      best = (K + te - 1) / te;
     }
   }
-  return best;
+  return best < sm_count ? (K < sm_count ? K : sm_count) : best;
 }
+
+// K elements cut into n tiles of K / n elements, the first K % n tiles one more
+struct TileCut {
+  int len, rem;
+  DGC_HD TileCut(int K, int n) : len((int)((unsigned)K / (unsigned)n)), rem(K - len * n) {}
+  DGC_HD int start(int i) const { return i * len + (i < rem ? i : rem); }
+  DGC_HD int size(int i) const { return len + (i < rem ? 1 : 0); }
+};
 
 }  // namespace dgk
 

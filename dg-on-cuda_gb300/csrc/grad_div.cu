@@ -145,13 +145,14 @@ struct GradDivBc {
 
 // gradient of p.u into p.qx, p.qy
 template <int N>
-__global__ void __launch_bounds__(256) k_grad_eo(const IpdgParams p, const GradDivBc bc, const int te) {
+__global__ void __launch_bounds__(256) k_grad_eo(const IpdgParams p, const GradDivBc bc) {
   using C = IpdgEo<N>;
   constexpr int Np = C::Np, NpP = C::NpP, Nfp = C::Nfp, nE = C::nE, nO = C::nO, fE = C::fE, fO = C::fO;
   extern __shared__ __align__(128) unsigned char smem[];
   const IpdgEoTile<N> t{smem};
   const int tid = threadIdx.x;
-  const int k0 = blockIdx.x * te, ne = min(te, p.K - k0);
+  const TileCut tiles(p.K, gridDim.x);
+  const int k0 = tiles.start(blockIdx.x), ne = tiles.size(blockIdx.x);
   if (!t.setup(p, k0, ne, C::kOpsG, false)) return;
   const double* u = static_cast<const double*>(p.u);
   grid_dep_wait();
@@ -206,13 +207,14 @@ __global__ void __launch_bounds__(256) k_grad_eo(const IpdgParams p, const GradD
 
 // divergence of (p.qx, p.qy) into p.out
 template <int N>
-__global__ void __launch_bounds__(256) k_div_eo(const IpdgParams p, const GradDivBc bc, const int te) {
+__global__ void __launch_bounds__(256) k_div_eo(const IpdgParams p, const GradDivBc bc) {
   using C = IpdgEo<N>;
   constexpr int Np = C::Np, NpP = C::NpP, Nfp = C::Nfp, nE = C::nE, nO = C::nO, fE = C::fE, fO = C::fO;
   extern __shared__ __align__(128) unsigned char smem[];
   const IpdgEoTile<N> t{smem};
   const int tid = threadIdx.x;
-  const int k0 = blockIdx.x * te, ne = min(te, p.K - k0);
+  const TileCut tiles(p.K, gridDim.x);
+  const int k0 = tiles.start(blockIdx.x), ne = tiles.size(blockIdx.x);
   if (!t.setup(p, k0, ne, C::kOpsG, false)) return;
   const double* u0 = static_cast<const double*>(p.qx);
   const double* u1 = static_cast<const double*>(p.qy);
@@ -289,9 +291,9 @@ cudaError_t launch_eo(const IpdgParams& p, const GradDivBc& bc, int sm, cudaStre
   if (st != cudaSuccess) return st;
   // the passes' cost, without the mass rows
   const EoCost w = DIV ? EoCost{C::kCostDiv.row - C::nE, C::kCostDiv.flux, C::kCostDiv.in, C::kCostDiv.cst} : C::kCostGrad;
-  const int te = eo_pick_tile(C::D, p.K, sm, C::TE, w), ntiles = (p.K + te - 1) / te;
-  if (ntiles <= sm) return launch_stage(kern, ntiles, 256, C::kSmemGrad, s, p, bc, te);
-  kern<<<ntiles, 256, C::kSmemGrad, s>>>(p, bc, te);
+  const int ntiles = eo_pick_tiles(C::D, p.K, sm, C::TE, w);
+  if (ntiles <= sm) return launch_stage(kern, ntiles, 256, C::kSmemGrad, s, p, bc);
+  kern<<<ntiles, 256, C::kSmemGrad, s>>>(p, bc);
   return cudaGetLastError();
 }
 

@@ -66,24 +66,29 @@ cudaError_t ipdg_launch_n(int kind, const IpdgParams& p, int sm, cudaStream_t s)
 template <int N>
 cudaError_t ipdg_eo_launch_n(int kind, const IpdgParams& p, int sm, cudaStream_t s) {
   using C = IpdgEo<N>;
-  using Fn = void (*)(const IpdgParams, int);
+  using Fn = void (*)(const IpdgParams);
   static const Fn fns[6] = {ipdg_grad_eo_kernel<N, GRAD_PLAIN>, ipdg_grad_eo_kernel<N, GRAD_PCG>,
                             ipdg_div_eo_kernel<N, DIV_LAPLACE>, ipdg_div_eo_kernel<N, DIV_SPD>,
                             ipdg_div_eo_kernel<N, DIV_SPD_DOT>, ipdg_div_eo_kernel<N, DIV_RESID>};
   static std::once_flag once;
   static cudaError_t st = cudaSuccess;
   std::call_once(once, [] {
-    for (int k = 0; k < 6 && st == cudaSuccess; ++k)
+    for (int k = 0; k < 6 && st == cudaSuccess; ++k) {
       st = cudaFuncSetAttribute(fns[k], cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 k <= IK_GRAD_PCG ? C::kSmemGrad : C::kSmemDiv);
+      // the same carveout for both passes: with the driver's choice for each, every
+      // overlapped launch of the one after the other drained the SMs (CG iteration
+      // at K = 2048, N = 4: 48 us instead of 20)
+      if (st == cudaSuccess)
+        st = cudaFuncSetAttribute(fns[k], cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    }
   });
   if (st != cudaSuccess) return st;
   const bool grad = kind <= IK_GRAD_PCG;
-  const int te = eo_pick_tile(C::D, p.K, sm, C::TE, grad ? C::kCostGrad : C::kCostDiv);
-  const int ntiles = (p.K + te - 1) / te;
+  const int ntiles = eo_pick_tiles(C::D, p.K, sm, C::TE, grad ? C::kCostGrad : C::kCostDiv);
   const size_t smem = grad ? C::kSmemGrad : C::kSmemDiv;
-  if (ntiles <= sm) return launch_stage(fns[kind], ntiles, 256, smem, s, p, te);
-  fns[kind]<<<ntiles, 256, smem, s>>>(p, te);
+  if (ntiles <= sm) return launch_stage(fns[kind], ntiles, 256, smem, s, p);
+  fns[kind]<<<ntiles, 256, smem, s>>>(p);
   return cudaGetLastError();
 }
 
@@ -105,7 +110,7 @@ cudaError_t ipdg_eo_launch(int N, int kind, const IpdgParams& p, int sm, cudaStr
 enum IpdgBlkKernel : int { IB_GRAD = 0, IB_DIV = 1, IB_UPDATE = 2 };
 
 template <int N>
-cudaError_t ipdg_blk_launch_n(int kind, const IpdgParams& p, int sm, cudaStream_t s) {
+cudaError_t ipdg_blk_launch_n(int kind, const IpdgParams& p, int sm, cudaStream_t s, bool graph) {
   using B = IpdgBlk<N>;
   static std::once_flag once[3];
   static int bps[3];
@@ -124,12 +129,17 @@ cudaError_t ipdg_blk_launch_n(int kind, const IpdgParams& p, int sm, cudaStream_
       st[kind] = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps[kind], fn, 256, smem);
   });
   if (st[kind] != cudaSuccess) return st[kind];
-  const int ntiles = (p.K + B::TE - 1) / B::TE;
-  int grid = sm * (bps[kind] > 0 ? bps[kind] : 1);
-  if (grid > ntiles) grid = ntiles;
-  // programmatic dependent launch: the kernels wait (grid_dep_wait) before
-  // their first access to the CG scalars and vectors
-  void* args[] = {const_cast<IpdgParams*>(&p)};
+  IpdgParams q = p;
+  q.ntiles = blk_tiles_for(p.K, sm, B::TE);
+  const int grid = std::min(q.ntiles, sm * (bps[kind] > 0 ? bps[kind] : 1));
+  // programmatic dependent launch (the kernels wait, grid_dep_wait, before their
+  // first access to the CG scalars and vectors), but from a graph only where every
+  // CTA has one tile: iteration at K = 32768, N = 4 35.1 us against 36.7 launched
+  // plainly.  CTAs of several tiles hold their SMs until the end, an early next
+  // launch takes room from them (K = 131072: 92.7 us overlapped, 89.4 plainly), and
+  // a graph's launches have little latency to hide; a stream's have more (the
+  // two-level solve at K = 131072: 273 ms overlapped, 281 plainly).
+  void* args[] = {&q};
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(256);
@@ -139,20 +149,21 @@ cudaError_t ipdg_blk_launch_n(int kind, const IpdgParams& p, int sm, cudaStream_
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = stage_overlap_enabled() ? 1 : 0;
+  cfg.numAttrs = stage_overlap_enabled() && (!graph || grid == q.ntiles) ? 1 : 0;
   return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
-cudaError_t ipdg_blk_launch(int N, int kind, const IpdgParams& p, int sm, cudaStream_t s) {
+// graph: the launch is replayed from a graph (the CG iterations)
+cudaError_t ipdg_blk_launch(int N, int kind, const IpdgParams& p, int sm, cudaStream_t s, bool graph) {
   switch (N) {
-    case 1: return ipdg_blk_launch_n<1>(kind, p, sm, s);
-    case 2: return ipdg_blk_launch_n<2>(kind, p, sm, s);
-    case 3: return ipdg_blk_launch_n<3>(kind, p, sm, s);
-    case 4: return ipdg_blk_launch_n<4>(kind, p, sm, s);
-    case 5: return ipdg_blk_launch_n<5>(kind, p, sm, s);
-    case 6: return ipdg_blk_launch_n<6>(kind, p, sm, s);
-    case 7: return ipdg_blk_launch_n<7>(kind, p, sm, s);
-    case 8: return ipdg_blk_launch_n<8>(kind, p, sm, s);
+    case 1: return ipdg_blk_launch_n<1>(kind, p, sm, s, graph);
+    case 2: return ipdg_blk_launch_n<2>(kind, p, sm, s, graph);
+    case 3: return ipdg_blk_launch_n<3>(kind, p, sm, s, graph);
+    case 4: return ipdg_blk_launch_n<4>(kind, p, sm, s, graph);
+    case 5: return ipdg_blk_launch_n<5>(kind, p, sm, s, graph);
+    case 6: return ipdg_blk_launch_n<6>(kind, p, sm, s, graph);
+    case 7: return ipdg_blk_launch_n<7>(kind, p, sm, s, graph);
+    case 8: return ipdg_blk_launch_n<8>(kind, p, sm, s, graph);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -325,14 +336,6 @@ __global__ void k_cg_start(CgScalars* cg, double tol2, int maxit) {
   cg->tol2 = tol2;
   cg->maxit = maxit;
   if (cg->rr[0] == 0.0) cg->done = 1;
-}
-// convergence bookkeeping, one thread: done when rr <= tol2 * bb or iters >= maxit
-// a plain launch: it ends the overlap chain of one iteration's launches
-__global__ void k_cg_check(CgScalars* cg, int slot) {
-  if (cg->done) return;
-  cg->iters += 1;
-  if (cg->rr[slot] <= cg->tol2 * cg->bb) cg->done = 1;
-  else if (cg->iters >= cg->maxit) cg->done = 2;
 }
 
 }  // namespace dgk
@@ -750,7 +753,7 @@ int apply(dgc_handle_s* h, int div_kind, const R* u, R* out, const R* b, double*
   return launch<R>(h, div_kind, p, s);
 }
 
-// one CG iteration (three launches) for slot i mod 3
+// one CG iteration (three launches; the next one's grad pass decides convergence) for slot i mod 3
 template <typename R>
 int cg_iteration(dgc_handle_s* h, int cgi, int slot, int first, cudaStream_t s) {
   dgk::IpdgParams p = base<R>(h);
@@ -765,7 +768,7 @@ int cg_iteration(dgc_handle_s* h, int cgi, int slot, int first, cudaStream_t s) 
   // FP32: the register-blocked kernels (ipdg_blk.cuh); FP64: the one-node-per-thread ones
   auto run = [&](int kind_r, int kind_blk) -> int {
     if (sizeof(R) == 4) {
-      const cudaError_t e = dgk::ipdg_blk_launch(h->N, kind_blk, p, h->sm_count, s);
+      const cudaError_t e = dgk::ipdg_blk_launch(h->N, kind_blk, p, h->sm_count, s, true);
       if (e != cudaSuccess) return cuda_err(e, "ipdg blocked kernel launch");
       ++h->launches;
       return DGC_OK;
@@ -781,9 +784,6 @@ int cg_iteration(dgc_handle_s* h, int cgi, int slot, int first, cudaStream_t s) 
   p.z = wv<R>(h, W_Z);
   p.Ap = wv<R>(h, W_AP);
   if (int rc = run(dgk::IK_UPDATE, dgk::IB_UPDATE)) return rc;
-  dgk::k_cg_check<<<1, 1, 0, s>>>(h->ipdg->cg + cgi, (slot + 1) % 3);
-  CKI(cudaGetLastError());
-  ++h->launches;
   return DGC_OK;
 }
 
@@ -838,7 +838,7 @@ int pcg_core(dgc_handle_s* h, double rtol, int maxit, bool use_graph, int* iters
     for (int c = 0; c < chunks_per_check; ++c) {
       if (use_graph) {
         CKI(cudaGraphLaunch(st->chunk[cgi], s));
-        h->launches += 12;
+        h->launches += 9;
       } else {
         for (int i = 1; i <= 3; ++i)
           if (int rc = cg_iteration<R>(h, cgi, i % 3, 0, s)) return rc;
@@ -847,6 +847,7 @@ int pcg_core(dgc_handle_s* h, double rtol, int maxit, bool use_graph, int* iters
     }
     CKI(cudaMemcpyAsync(st->h_cg + cgi, st->cg + cgi, sizeof(dgk::CgScalars), cudaMemcpyDeviceToHost, s));
     CKI(cudaStreamSynchronize(s));
+    st->h_cg[cgi].done = dgk::cg_decide(st->h_cg[cgi], done_it % 3);  // the last update's sums
     if (st->h_cg[cgi].done) break;
     if (done_it > maxit + 12) break;
   }
@@ -884,11 +885,11 @@ int ipdg_spd_apply_f32(dgc_handle_s* h, const float* u, float* out, cudaStream_t
   p.p = wv<float>(h, W_T);
   p.qx = wv<float>(h, W_QX);
   p.qy = wv<float>(h, W_QY);
-  cudaError_t e = dgk::ipdg_blk_launch(h->N, dgk::IB_GRAD, p, h->sm_count, s);
+  cudaError_t e = dgk::ipdg_blk_launch(h->N, dgk::IB_GRAD, p, h->sm_count, s, false);
   if (e != cudaSuccess) return cuda_err(e, "ipdg blocked kernel launch");
   p.du_src = wv<float>(h, W_T);
   p.out = out;
-  e = dgk::ipdg_blk_launch(h->N, dgk::IB_DIV, p, h->sm_count, s);
+  e = dgk::ipdg_blk_launch(h->N, dgk::IB_DIV, p, h->sm_count, s, false);
   if (e != cudaSuccess) return cuda_err(e, "ipdg blocked kernel launch");
   h->launches += 2;
   return DGC_OK;

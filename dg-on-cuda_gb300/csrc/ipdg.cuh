@@ -20,6 +20,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "eo.hpp"
 
 namespace dgk {
 
@@ -38,6 +39,16 @@ struct CgScalars {
   int maxit;        // iteration budget of this solve
   int pad;
 };
+
+// Whether the solve ends before the iteration whose residual sums are in `slot`:
+// the grad pass of every iteration but the first asks on all CTAs and block 0
+// records the answer for the passes that follow it (no launch of its own for it;
+// the host asks the same of the last iteration's sums).
+__host__ __device__ inline int cg_decide(const CgScalars& cg, int slot) {
+  if (cg.done) return cg.done;
+  if (cg.rr[slot] <= cg.tol2 * cg.bb) return 1;
+  return cg.iters >= cg.maxit ? 2 : 0;
+}
 
 struct IpdgParams {
   int K;
@@ -73,6 +84,7 @@ struct IpdgParams {
   double shift;         // SPD modes: S = -J M (A - shift I) (Helmholtz-type operators; 0 = laplace)
   CgScalars* cg;
   double* dot_out;      // DIV_SPD_DOT / DIV_RESID: accumulated dot product
+  int ntiles;           // register-blocked kernels: tiles, cut evenly (TileCut)
   int slot;             // iteration slot (i mod 3)
   int first;            // first iteration: beta = 0
   int* status;
@@ -115,6 +127,32 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
   if (threadIdx.x == 0)
     for (int i = 0; i < (int)(blockDim.x >> 5); ++i) s += red[i];
   return s;  // valid in thread 0
+}
+
+// Two block sums at once, each by warp shuffles and then by the first warp over
+// the warps' partials: 8 dependent FP64 additions (their latency is what a small
+// grid waits for) where block_sum's serial end takes 5 + 8 per value.  red: 16
+// doubles; valid in thread 0; 256 threads.
+__device__ __forceinline__ void block_sum2(double& a, double& b, double* red) {
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b += __shfl_xor_sync(0xffffffffu, b, o);
+  }
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  __syncthreads();
+  if (l == 0) {
+    red[w] = a;
+    red[8 + w] = b;
+  }
+  __syncthreads();
+  if (w == 0) {
+    a = l < 8 ? red[l] : 0.0;
+    b = l < 8 ? red[8 + l] : 0.0;
+    for (int o = 4; o > 0; o >>= 1) {
+      a += __shfl_xor_sync(0xffffffffu, a, o);
+      b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+  }
 }
 
 template <typename R, int N>
@@ -204,7 +242,13 @@ __global__ void __launch_bounds__(256) ipdg_grad_kernel(const IpdgParams p) {
   using C = IpdgConfig<R, N>;
   constexpr int Np = T::Np, NpP = T::NpP, Nfp = T::Nfp, NFACE = T::NFACE, TE = T::TE;
   extern __shared__ __align__(128) unsigned char smem[];
-  if (MODE == GRAD_PCG && p.cg->done) return;
+  if (MODE == GRAD_PCG) {
+    const int d = p.first ? p.cg->done : cg_decide(*p.cg, p.slot);
+    if (d) {
+      if (blockIdx.x == 0 && threadIdx.x == 0) p.cg->done = d;
+      return;
+    }
+  }
   T t{smem};
   // beta = rz_new / rz_old: one FP64 division per CTA, broadcast through shared
   // memory (t.init's barrier publishes it)
@@ -443,23 +487,31 @@ __global__ void __launch_bounds__(256) pcg_update_kernel(const IpdgParams p) {
       sr[e * NpP + i] = rv;
       rr += (double)rv * (double)rv;
     }
+    // the first columns of the block are loaded before the barrier
+    constexpr int kPre = Np < 16 ? Np : 16;
+    R bpre[kPre];
+    const R* be = binv + (size_t)(k0 + e) * BSTR + i;
+    if (act)
+#pragma unroll
+      for (int j = 0; j < kPre; ++j) bpre[j] = __ldg(be + j * Np);
     __syncthreads();
     if (act) {
-      const R* be = binv + (size_t)(k0 + e) * BSTR;
       const R* re = sr + e * NpP;
       R zv = 0;
+#pragma unroll
+      for (int j = 0; j < kPre; ++j) zv = fma(bpre[j], re[j], zv);
 #pragma unroll 5
-      for (int j = 0; j < Np; ++j) zv = fma(__ldg(be + j * Np + i), re[j], zv);
+      for (int j = kPre; j < Np; ++j) zv = fma(__ldg(be + j * Np), re[j], zv);
       z[(size_t)(k0 + e) * NpP + i] = zv;
       rz += (double)rv * (double)zv;
     }
     __syncthreads();
   }
-  const double a = block_sum(rz, red);
-  const double b = block_sum(rr, red);
+  block_sum2(rz, rr, red);
   if (threadIdx.x == 0) {
-    atomicAdd(&cg->rz[s1], a);
-    atomicAdd(&cg->rr[s1], b);
+    atomicAdd(&cg->rz[s1], rz);
+    atomicAdd(&cg->rr[s1], rr);
+    if (blockIdx.x == 0) cg->iters += 1;
   }
 }
 

@@ -18,6 +18,16 @@
 
 namespace dgk {
 
+// Tiles of the register-blocked kernels, cut evenly (TileCut): as many as full
+// tiles make, at least one per SM.  On meshes with fewer full tiles than SMs an
+// iteration is latency (K = 3200, N = 3: 19.8 -> 15.0 us with one tile per SM and
+// the convergence test in the grad pass instead of a launch); rounding larger counts up to whole waves
+// took K = 131072, N = 4 from 95 to 98 us per iteration.
+inline int blk_tiles_for(int K, int sm_count, int te_max) {
+  const int full = (K + te_max - 1) / te_max;
+  return full >= sm_count ? full : (K < sm_count ? K : sm_count);
+}
+
 template <int N>
 struct IpdgBlk {
   using O = Order<N>;
@@ -107,9 +117,11 @@ __global__ void __launch_bounds__(256, 4) ipdg_grad_blk_kernel(const IpdgParams 
     return reinterpret_cast<int4*>(smem + B::oBufG + b * B::kBufG + 2 * B::kF + B::kG);
   };
   __shared__ float s_beta;
+  __shared__ int s_done;
   const int tid = threadIdx.x;
   const int slot = tid / NG, grp = tid - slot * NG;
-  const int ntiles = (p.K + TE - 1) / TE;
+  const int ntiles = p.ntiles;
+  const TileCut tiles(p.K, ntiles);
   const float* zin = static_cast<const float*>(p.u);
   const float* pold = static_cast<const float*>(p.p_old);
   float* pv = static_cast<float*>(p.p);
@@ -117,7 +129,7 @@ __global__ void __launch_bounds__(256, 4) ipdg_grad_blk_kernel(const IpdgParams 
   float* qyo = static_cast<float*>(p.qy);
 
   auto issue = [&](int tile, int b) {
-    const int k0 = tile * TE, ne = min(TE, p.K - k0);
+    const int k0 = tiles.start(tile), ne = tiles.size(tile);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     const uint32_t bf = ne * NpP * 4, bg = ne * 64, bn = ne * 16;
     mbar_arrive_expect_tx(&bar[b], 2 * bf + bg + bn);
@@ -142,24 +154,29 @@ __global__ void __launch_bounds__(256, 4) ipdg_grad_blk_kernel(const IpdgParams 
   // the CG scalars and vectors are earlier launches' output; the operators
   // are set-up data (their copy is in flight already)
   grid_dep_wait();
-  const bool done = p.cg->done != 0;
-  if (tid == 0 && !done) {
-    s_beta = 0.0f;
-    if (!p.first) {
-      const int s = p.slot, sp = (s + 2) % 3;
-      s_beta = (float)(p.cg->rz[s] / p.cg->rz[sp]);
+  if (tid == 0) {
+    const int d = p.first ? p.cg->done : cg_decide(*p.cg, p.slot);
+    s_done = d;
+    if (!d) {
+      if ((int)blockIdx.x < ntiles) issue(blockIdx.x, 0);  // in flight during the division
+      s_beta = 0.0f;
+      if (!p.first) {
+        const int s = p.slot, sp = (s + 2) % 3;
+        s_beta = (float)(p.cg->rz[s] / p.cg->rz[sp]);
+      }
+      if (blockIdx.x == 0) p.cg->pAp = 0.0;
+    } else if (blockIdx.x == 0) {
+      p.cg->done = d;
     }
-    if (blockIdx.x == 0) p.cg->pAp = 0.0;
-    if ((int)blockIdx.x < ntiles) issue(blockIdx.x, 0);
   }
   if (!__syncthreads_and(mbar_wait(&bar[2], 0, p.status))) return;
-  if (done) return;  // converged: nothing in flight once the operators have landed
+  if (s_done) return;  // converged: nothing in flight once the operators have landed
   const float beta = s_beta;
   uint32_t ph[2] = {0, 0};
   int it = 0;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
     const int b = it & 1;
-    const int k0 = tile * TE, ne = min(TE, p.K - k0);
+    const int k0 = tiles.start(tile), ne = tiles.size(tile);
     const int nxt = tile + gridDim.x;
     if (tid == 0 && nxt < ntiles) issue(nxt, b ^ 1);
     if (!__syncthreads_and(mbar_wait(&bar[b], ph[b], p.status))) return;
@@ -306,14 +323,15 @@ __global__ void __launch_bounds__(256, 4) ipdg_div_blk_kernel(const IpdgParams p
   };
   const int tid = threadIdx.x;
   const int slot = tid / NG, grp = tid - slot * NG;
-  const int ntiles = (p.K + TE - 1) / TE;
+  const int ntiles = p.ntiles;
+  const TileCut tiles(p.K, ntiles);
   const float* qx = static_cast<const float*>(p.qx);
   const float* qy = static_cast<const float*>(p.qy);
   const float* uj = static_cast<const float*>(p.du_src);
   float* out = static_cast<float*>(p.out);
 
   auto issue = [&](int tile, int b) {
-    const int k0 = tile * TE, ne = min(TE, p.K - k0);
+    const int k0 = tiles.start(tile), ne = tiles.size(tile);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     const uint32_t bf = ne * NpP * 4, bg = ne * 64, bn = ne * 16, bt = ne * 16;
     mbar_arrive_expect_tx(&bar[b], 3 * bf + bg + bn + bt);
@@ -356,7 +374,7 @@ __global__ void __launch_bounds__(256, 4) ipdg_div_blk_kernel(const IpdgParams p
   int it = 0;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
     const int b = it & 1;
-    const int k0 = tile * TE, ne = min(TE, p.K - k0);
+    const int k0 = tiles.start(tile), ne = tiles.size(tile);
     const int nxt = tile + gridDim.x;
     if (tid == 0 && nxt < ntiles) issue(nxt, b ^ 1);
     if (!__syncthreads_and(mbar_wait(&bar[b], ph[b], p.status))) return;
@@ -513,7 +531,8 @@ __global__ void __launch_bounds__(256, 2) pcg_update_blk_kernel(const IpdgParams
   const int tid = threadIdx.x;
   const int slot = tid / NG, grp = tid - slot * NG;
   const int s = p.slot, s1 = (s + 1) % 3;
-  const int ntiles = (p.K + TE - 1) / TE;
+  const int ntiles = p.ntiles;
+  const TileCut tiles(p.K, ntiles);
   float* x = static_cast<float*>(p.x);
   float* r = static_cast<float*>(p.r);
   float* z = static_cast<float*>(p.z);
@@ -521,7 +540,7 @@ __global__ void __launch_bounds__(256, 2) pcg_update_blk_kernel(const IpdgParams
   const float* Ap = static_cast<const float*>(p.Ap);
   const float* bpk = static_cast<const float*>(p.binv_pk);
   auto issue = [&](int tile, int b) {
-    const int k0 = tile * TE, ne = min(TE, p.K - k0);
+    const int k0 = tiles.start(tile), ne = tiles.size(tile);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     const uint32_t bf = ne * NpP * 4;
     mbar_arrive_expect_tx(&bar[b], 4 * bf + ne * PK * 4);
@@ -546,9 +565,11 @@ __global__ void __launch_bounds__(256, 2) pcg_update_blk_kernel(const IpdgParams
   // the CG scalars and vectors are earlier launches' output
   grid_dep_wait();
   if (cg->done) return;  // nothing issued yet
-  if (tid == 0) s_alpha = (float)(cg->rz[s] / cg->pAp);  // one FP64 division per CTA
+  if (tid == 0) {
+    if ((int)blockIdx.x < ntiles) issue(blockIdx.x, 0);  // in flight during the division
+    s_alpha = (float)(cg->rz[s] / cg->pAp);              // one FP64 division per CTA
+  }
   __syncthreads();
-  if (tid == 0 && (int)blockIdx.x < ntiles) issue(blockIdx.x, 0);
   const float alpha = s_alpha;
   const uint2* tab2 = reinterpret_cast<const uint2*>(tab);
   double rz = 0.0, rr = 0.0;
@@ -557,7 +578,7 @@ __global__ void __launch_bounds__(256, 2) pcg_update_blk_kernel(const IpdgParams
   const int i0 = grp * 4;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
     const int b = it & 1;
-    const int k0 = tile * TE, ne = min(TE, p.K - k0);
+    const int k0 = tiles.start(tile), ne = tiles.size(tile);
     const int nxt = tile + gridDim.x;
     // buffer b ^ 1 was last read before the barrier that ended the previous tile
     if (tid == 0 && nxt < ntiles) issue(nxt, b ^ 1);
@@ -607,11 +628,11 @@ __global__ void __launch_bounds__(256, 2) pcg_update_blk_kernel(const IpdgParams
     }
     __syncthreads();
   }
-  const double a = block_sum(rz, red);
-  const double bsum = block_sum(rr, red + 8);
+  block_sum2(rz, rr, red);
   if (tid == 0) {
-    atomicAdd(&cg->rz[s1], a);
-    atomicAdd(&cg->rr[s1], bsum);
+    atomicAdd(&cg->rz[s1], rz);
+    atomicAdd(&cg->rr[s1], rr);
+    if (blockIdx.x == 0) cg->iters += 1;
   }
 }
 

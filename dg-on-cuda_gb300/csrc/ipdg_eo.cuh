@@ -11,7 +11,7 @@
 //     and M half of theirs;
 //   * -1/J (the SPD form: J (1/J) = 1), faceJ, normals and penalties are
 //     multiplied into per-element constants.
-// One tile of `te` elements per CTA (eo_pick_tile); set-up data are fetched
+// One tile per CTA (eo_pick_tiles); set-up data are fetched
 // before the wait for the previous launch, exterior traces while the tile's own
 // fields arrive.
 #pragma once
@@ -39,7 +39,7 @@ struct IpdgEo {
   static constexpr uint32_t kSmemGrad = oOps + kOpsG, kSmemDiv = oOps + kOpsD;
   static_assert(TE * fE <= 256, "one face-node pair per thread");
   static_assert(oGeom % 16 == 0 && oFld % 16 == 0 && kF % 16 == 0 && oRed % 16 == 0 && kOpsG % 16 == 0, "alignment");
-  // FP64 instructions per item (eo_pick_tile)
+  // FP64 instructions per item (eo_pick_tiles)
   static constexpr EoCost kCostGrad{Np + 2 * fE + 6, 12, 2, 8}, kCostDiv{Np + fE + nE + 5, 14, 8, 8};
 };
 
@@ -225,7 +225,7 @@ struct IpdgEoTile {
 
 // ---------------------------------------------------------------- grad pass
 template <int N, int MODE>
-__global__ void __launch_bounds__(256) ipdg_grad_eo_kernel(const IpdgParams p, const int te) {
+__global__ void __launch_bounds__(256) ipdg_grad_eo_kernel(const IpdgParams p) {
   using C = IpdgEo<N>;
   constexpr int Np = C::Np, NpP = C::NpP, Nfp = C::Nfp, nE = C::nE, nO = C::nO, fE = C::fE, fO = C::fO;
   constexpr bool PCG = MODE == GRAD_PCG;
@@ -233,13 +233,20 @@ __global__ void __launch_bounds__(256) ipdg_grad_eo_kernel(const IpdgParams p, c
   __shared__ double s_beta;
   const IpdgEoTile<N> t{smem};
   const int tid = threadIdx.x;
-  const int k0 = blockIdx.x * te, ne = min(te, p.K - k0);
+  const TileCut tiles(p.K, gridDim.x);
+  const int k0 = tiles.start(blockIdx.x), ne = tiles.size(blockIdx.x);
   if (!t.setup(p, k0, ne, C::kOpsG, false)) return;
   const double* u_in = static_cast<const double*>(p.u);
   const double* pold = static_cast<const double*>(p.p_old);
   grid_dep_wait();
   grid_dep_launch();
-  if (PCG && p.cg->done) return;
+  if (PCG) {
+    const int d = p.first ? p.cg->done : cg_decide(*p.cg, p.slot);
+    if (d) {
+      if (blockIdx.x == 0 && tid == 0) p.cg->done = d;
+      return;
+    }
+  }
   if (tid == 0) {
     mbar_arrive_expect_tx(t.bar() + 1, (PCG ? 2 : 1) * ne * NpP * 8);
     bulk_g2s(t.field(0), u_in + (size_t)k0 * NpP, ne * NpP * 8, t.bar() + 1);
@@ -310,14 +317,15 @@ __global__ void __launch_bounds__(256) ipdg_grad_eo_kernel(const IpdgParams p, c
 
 // ---------------------------------------------------------------- div pass
 template <int N, int MODE>
-__global__ void __launch_bounds__(256) ipdg_div_eo_kernel(const IpdgParams p, const int te) {
+__global__ void __launch_bounds__(256) ipdg_div_eo_kernel(const IpdgParams p) {
   using C = IpdgEo<N>;
   constexpr int Np = C::Np, NpP = C::NpP, Nfp = C::Nfp, nE = C::nE, nO = C::nO, fE = C::fE, fO = C::fO;
   constexpr bool SPD = MODE != DIV_LAPLACE;
   extern __shared__ __align__(128) unsigned char smem[];
   const IpdgEoTile<N> t{smem};
   const int tid = threadIdx.x;
-  const int k0 = blockIdx.x * te, ne = min(te, p.K - k0);
+  const TileCut tiles(p.K, gridDim.x);
+  const int k0 = tiles.start(blockIdx.x), ne = tiles.size(blockIdx.x);
   if (!t.setup(p, k0, ne, SPD ? C::kOpsD : C::kOpsG, true)) return;
   const double* qx = static_cast<const double*>(p.qx);
   const double* qy = static_cast<const double*>(p.qy);

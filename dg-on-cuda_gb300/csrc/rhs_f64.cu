@@ -16,6 +16,10 @@ static cudaError_t rhs_f64(const RhsParams& p, int sm, cudaStream_t s, LaunchInf
   static int bps = 0;
   std::call_once(once, [] {
     st = cudaFuncSetAttribute(dg_rhs_eo_kernel<double, N, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
+    // one shared-memory carveout for all kernels that launch overlapped: a change
+    // of it between two launches drains the SMs in between
+    if (st == cudaSuccess)
+      st = cudaFuncSetAttribute(dg_rhs_eo_kernel<double, N, P>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     if (st == cudaSuccess)
       st = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, dg_rhs_eo_kernel<double, N, P>, C::kThreads, C::kSmem);
   });
@@ -27,14 +31,14 @@ static cudaError_t rhs_f64(const RhsParams& p, int sm, cudaStream_t s, LaunchInf
     info->blocks_per_sm = bps;
     return cudaSuccess;
   }
-  const int te = eo_tile<double, N, P>(p.K, sm), ntiles = (p.K + te - 1) / te;
+  const int ntiles = eo_tiles<double, N, P>(p.K, sm);
   // Overlapped launch only where the grid leaves SMs one CTA each: its prologue
   // then runs beside the previous stage (K = 2048, N = 4, advection: 6.0 us per
   // stage against 6.8 without).  A larger grid launched early is placed on the
   // SMs that have room at that moment, unevenly (K = 2048, N = 6, Maxwell TE:
   // 24.9 us against 17.3 launched plainly).
-  if (ntiles <= sm) return launch_stage(dg_rhs_eo_kernel<double, N, P>, ntiles, C::kThreads, C::kSmem, s, p, te);
-  dg_rhs_eo_kernel<double, N, P><<<ntiles, C::kThreads, C::kSmem, s>>>(p, te);
+  if (ntiles <= sm) return launch_stage(dg_rhs_eo_kernel<double, N, P>, ntiles, C::kThreads, C::kSmem, s, p);
+  dg_rhs_eo_kernel<double, N, P><<<ntiles, C::kThreads, C::kSmem, s>>>(p);
   return cudaGetLastError();
 }
 
