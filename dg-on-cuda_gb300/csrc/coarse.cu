@@ -53,12 +53,14 @@ struct CoarseSpace {
   int32_t* d_cells = nullptr;         // [K]
   int32_t* d_agg = nullptr;           // [K]
   double* d_ainv = nullptr;           // [nagg][nagg] A_c^-1
-  float* d_ainv32 = nullptr;          // FP32 copy of A_c^-1 (the FP32 coarse cycle)
+  float* d_ainv32 = nullptr;          // FP32 copy of A_c^-1 (the FP32 coarse cycle), rows padded to lda()
+  int lda() const { return (nagg + 3) / 4 * 4; }
   double* d_rc = nullptr;             // P^T r
   float* d_rc32 = nullptr;            // FP32 copy of P^T r
   double* d_xc = nullptr;             // A_c^-1 P^T r
   double* d_w[3] = {};                // work vectors (K x NpP)
   float* d_f[2] = {};                 // FP32 work vectors of the FP32 smoothing applies
+  float* d_q32 = nullptr;             // S p of the two-level PCG's FP32 operator
   double* d_pcg[3] = {};              // two-level PCG: z, p, q = S p (allocated on first use)
   double* d_dots = nullptr;           // [4] dot products of the current kernel pair, [3] a mean
   double* d_sc = nullptr;             // [8] device-resident CG scalars (k_coarse_step_dev)
@@ -70,7 +72,7 @@ void coarse_free(CoarseSpace* c) {
   for (void* p : {(void*)c->d_ptr, (void*)c->d_cells, (void*)c->d_agg, (void*)c->d_ainv, (void*)c->d_rc,
                   (void*)c->d_xc, (void*)c->d_w[0], (void*)c->d_w[1], (void*)c->d_w[2], (void*)c->d_f[0],
                   (void*)c->d_f[1], (void*)c->d_pcg[0], (void*)c->d_pcg[1], (void*)c->d_pcg[2],
-                  (void*)c->d_dots, (void*)c->d_sc, (void*)c->d_ainv32, (void*)c->d_rc32})
+                  (void*)c->d_dots, (void*)c->d_q32, (void*)c->d_sc, (void*)c->d_ainv32, (void*)c->d_rc32})
     cudaFree(p);
   cudaFreeHost(c->h_sc);
   delete c;
@@ -98,12 +100,6 @@ __global__ void k_coarse_axpy(int64_t n, const double* x, double w, const double
   }
 }
 
-// out = x - w z with z in FP32 (an FP32 operator's output, no FP64 round trip)
-__global__ void k_coarse_axpy_z32(int64_t n, const double* x, double w, const float* __restrict__ z, double* out) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    out[i] = x[i] - w * (double)z[i];
-}
-
 // FP32 copy of an FP64 vector, and back
 __global__ void k_coarse_to_f32(int64_t n, const double* __restrict__ x, float* __restrict__ y) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -112,6 +108,15 @@ __global__ void k_coarse_to_f32(int64_t n, const double* __restrict__ x, float* 
 __global__ void k_coarse_to_f64(int64_t n, const float* __restrict__ x, double* __restrict__ y) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     y[i] = (double)x[i];
+}
+
+// FP32 copy of an n x n matrix with rows padded to lda
+__global__ void k_coarse_pad32(int n, int lda, const double* __restrict__ x, float* __restrict__ y) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (int64_t)n * lda;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t r = i / lda, c = i - r * lda;
+    y[i] = c < n ? (float)x[r * n + c] : 0.0f;
+  }
 }
 
 // out[j] += a_j . b_j, j < 3 (FP64; unused pairs have a null a)
@@ -159,33 +164,22 @@ __device__ __forceinline__ void block_dots_add(const double (&s)[3], int used, d
     atomicAdd(&out[threadIdx.x], v);
   }
 }
-// q = x32 in FP64 and out[0] += p.q (the FP32 operator output of the two-level
-// iteration, and the dot product its step needs)
-__global__ void k_coarse_to_f64_dot(int64_t n, const float* __restrict__ x32, double* __restrict__ q,
-                                    const double* __restrict__ p, double* out) {
+// out[0] += p.x32 (the FP32 operator output of the two-level iteration), q = x32
+// in FP64 when q is given; zero3, when given, is cleared for the next kernels' sums
+__global__ void k_coarse_dot32(int64_t n, const float* __restrict__ x32, const double* __restrict__ p, double* out,
+                               double* __restrict__ q, double* zero3) {
+  if (zero3 && blockIdx.x == 0 && threadIdx.x < 3) zero3[threadIdx.x] = 0.0;
   double s[3] = {0.0, 0.0, 0.0};
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const double v = (double)x32[i];
-    q[i] = v;
-    s[0] += p[i] * v;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n / 2; i += (int64_t)gridDim.x * blockDim.x) {
+    const float2 x = reinterpret_cast<const float2*>(x32)[i];
+    const double2 pv = reinterpret_cast<const double2*>(p)[i];
+    const double a = (double)(x.x), b = (double)(x.y);
+    if (q) reinterpret_cast<double2*>(q)[i] = make_double2(a, b);
+    s[0] += pv.x * a;
+    s[1] += pv.y * b;
   }
+  s[0] += s[1];
   block_dots_add(s, 1, out);
-}
-// z += x - w y, then out += (r.r, z.r, z.q) with the new z (the last kernel of the
-// two-level preconditioner and the dot products of the direction update)
-__global__ void k_coarse_axpy_dots(int64_t n, const double* __restrict__ x, double w, const double* __restrict__ y,
-                                   double* __restrict__ z, const double* __restrict__ r,
-                                   const double* __restrict__ q, double* out) {
-  double s[3] = {0.0, 0.0, 0.0};
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const double zi = z[i] + (x[i] - w * y[i]);
-    z[i] = zi;
-    const double ri = r[i];
-    s[0] += ri * ri;
-    s[1] += zi * ri;
-    s[2] += zi * q[i];
-  }
-  block_dots_add(s, 3, out);
 }
 
 // out += sum of z over the valid nodes; z -= *out / count on the valid nodes
@@ -208,33 +202,6 @@ __global__ void k_coarse_sub_mean(int64_t n, int npp, int np, const double* __re
 // back to back: sc[0], sc[1] = z.r by iteration parity, sc[3] = r.r, sc[5] =
 // alpha, sc[6] = stop flag (positivity lost); t = the dot products of the kernel
 // just before.
-// x += alpha p, r -= alpha q with alpha = z.r / p.q (t[0] = p.q)
-__global__ void k_coarse_step_dev(int64_t n, const double* __restrict__ p, const double* __restrict__ q,
-                                  double* __restrict__ x, double* __restrict__ r, double* sc,
-                                  const double* __restrict__ t, int cur) {
-  // one FP64 division per block, not per thread (GB300's FP64 rate is low)
-  __shared__ double s_alpha;
-  __shared__ int s_ok;
-  if (threadIdx.x == 0) {
-    const double rz = sc[cur], pq = t[0];
-    // at the rounding floor p.Sp or z.r can lose their sign: stop, the caller
-    // checks the true residual
-    const bool ok = pq > 0.0 && rz > 0.0 && sc[6] == 0.0;
-    s_alpha = ok ? rz / pq : 0.0;
-    s_ok = ok;
-    if (blockIdx.x == 0) {
-      sc[5] = s_alpha;
-      if (!ok) sc[6] = 1.0;
-    }
-  }
-  __syncthreads();
-  const double alpha = s_alpha;
-  if (!s_ok) return;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    x[i] += alpha * p[i];
-    r[i] -= alpha * q[i];
-  }
-}
 // p = z + beta p, beta = -alpha z.q / (z.r)_old (Polak-Ribiere, robust to the FP32
 // rounding inside the coarse term); t = (r.r, z.r, z.q) of the new residual.  The
 // new z.r goes to the other parity slot: no block reads what another writes.
@@ -247,10 +214,15 @@ __global__ void k_coarse_dir_dev(int64_t n, const double* __restrict__ z, double
   }
   __syncthreads();
   const double beta = s_beta;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const double v = first ? z[i] : z[i] + beta * p[i];
-    p[i] = v;
-    if (p32) p32[i] = (float)v;  // the next FP32 operator apply's input
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n / 2; i += (int64_t)gridDim.x * blockDim.x) {
+    double2 v = reinterpret_cast<const double2*>(z)[i];
+    if (!first) {
+      const double2 o = reinterpret_cast<const double2*>(p)[i];
+      v = make_double2(v.x + beta * o.x, v.y + beta * o.y);
+    }
+    reinterpret_cast<double2*>(p)[i] = v;
+    // the next FP32 operator apply's input
+    if (p32) reinterpret_cast<float2*>(p32)[i] = make_float2((float)v.x, (float)v.y);
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     sc[nxt] = t[1];
@@ -277,16 +249,42 @@ __global__ void k_gj_elim(int n, int i, double* __restrict__ A, const double* __
   A[(size_t)r * n + c] = v - col[r] * A[(size_t)i * n + c];
 }
 
-// rc[a] = sum of r over the valid nodes of the cells of aggregate a (fixed order)
+// rc[a] = sum of r (f32 given: r - w f32) over the valid nodes of the cells of
+// aggregate a, in a fixed order.  One warp per aggregate; up to 16 nodes per cell
+// its halves take alternate cells, four cells' loads in flight (one cell at a time:
+// 19 us at K = 131072, N = 4, after an 11 us pass forming r - w f32; 22 us so, the
+// FP64 conversions and sums).  zero1, when given, is cleared.
 __global__ void k_coarse_restrict(int nagg, int npp, int np, const int32_t* __restrict__ ptr,
                                   const int32_t* __restrict__ cells, const double* __restrict__ r,
-                                  double* __restrict__ rc, float* __restrict__ rc32) {
+                                  const float* __restrict__ f32, double w, double* __restrict__ rc,
+                                  float* __restrict__ rc32, double* zero1) {
+  if (zero1 && blockIdx.x == 0 && threadIdx.x == 0) *zero1 = 0.0;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= nagg) return;
+  const int q0 = ptr[warp], cnt = ptr[warp + 1] - q0;
+  const int half = np <= 16 ? lane >> 4 : 0, step = np <= 16 ? 2 : 1, j0 = np <= 16 ? lane & 15 : lane;
   double s = 0.0;
-  for (int q = ptr[warp]; q < ptr[warp + 1]; ++q) {
-    const double* rk = r + (size_t)cells[q] * npp;
-    for (int j = lane; j < np; j += 32) s += rk[j];
+  for (int b = 0; b < cnt; b += 32) {
+    const int m = min(32, cnt - b);
+    const int mine = lane < m ? cells[q0 + b + lane] : 0;
+    for (int jb = 0; jb < np; jb += 32 / step) {
+      const int j = jb + j0;
+      for (int c = 0; c < m; c += 4 * step) {
+        double rv[4];
+        float fv[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int q = c + u * step + half;
+          const int cell = __shfl_sync(0xffffffffu, mine, q & 31);
+          const bool ok = q < m && j < np;
+          const size_t o = (size_t)cell * npp + j;
+          rv[u] = ok ? r[o] : 0.0;
+          fv[u] = ok && f32 ? f32[o] : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) s += rv[u] - w * (double)(fv[u]);
+      }
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
@@ -311,16 +309,40 @@ __global__ void k_coarse_gemv(int n, const double* __restrict__ A, const double*
 
 // the same product with the FP32 copy of A_c^-1 and of x, FP32 sums (inside the
 // FP32 coarse cycle): half the bytes and no FP64 arithmetic
-__global__ void k_coarse_gemv32(int n, const float* __restrict__ A, const float* __restrict__ x,
+// (rows of A and x padded with zeros to lda, a multiple of 4: 16-byte loads)
+__global__ void k_coarse_gemv32(int n, int lda, const float* __restrict__ A, const float* __restrict__ x,
                                 double* __restrict__ y) {
   const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (row >= n) return;
-  const float* a = A + (size_t)row * n;
-  float s = 0.0f;
-  for (int c = lane; c < n; c += 32) s = fmaf(a[c], x[c], s);
+  const float4* a = reinterpret_cast<const float4*>(A + (size_t)row * lda);
+  const float4* x4 = reinterpret_cast<const float4*>(x);
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+  for (int c = lane; c < lda / 4; c += 32) {
+    const float4 aa = __ldg(a + c), xx = __ldg(x4 + c);
+    v.x = fmaf(aa.x, xx.x, v.x);
+    v.y = fmaf(aa.y, xx.y, v.y);
+    v.z = fmaf(aa.z, xx.z, v.z);
+    v.w = fmaf(aa.w, xx.w, v.w);
+  }
+  float s = (v.x + v.y) + (v.z + v.w);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if (lane == 0) y[row] = (double)s;
+}
+
+// z32[k][j] = xc[agg[k]] on the valid nodes, 0 on the others: the FP32 operator
+// apply's input (the correction takes xc itself); one thread per 4 nodes
+__global__ void k_coarse_prolong32(int64_t nq, int npp, int np, const int32_t* __restrict__ agg,
+                                   const double* __restrict__ xc, float* __restrict__ z32) {
+  const int q4 = npp / 4;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nq; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t k = i / q4;
+    const int j = 4 * (int)(i - k * q4);
+    const float v = (float)xc[agg[k]];
+    reinterpret_cast<float4*>(z32)[i] = make_float4(j < np ? v : 0.f, j + 1 < np ? v : 0.f, j + 2 < np ? v : 0.f,
+                                                    j + 3 < np ? v : 0.f);
+  }
 }
 
 // z[k][j] (+)= xc[agg[k]] on the valid nodes
@@ -615,10 +637,11 @@ extern "C" int dgc_coarse_build(dgc_handle h, int cells_per_aggregate, void* str
     dgk::k_gj_row<<<(nagg + 127) / 128, 128, 0, s>>>(nagg, i, c->d_ainv, c->d_rc);
     dgk::k_gj_elim<<<eg, 128, 0, s>>>(nagg, i, c->d_ainv, c->d_rc);
   }
-  if ((e = cudaMalloc(&c->d_ainv32, (size_t)nagg * nagg * 4)) != cudaSuccess ||
-      (e = cudaMalloc(&c->d_rc32, (size_t)nagg * 4)) != cudaSuccess)
+  if ((e = cudaMalloc(&c->d_ainv32, (size_t)nagg * c->lda() * 4)) != cudaSuccess ||
+      (e = cudaMalloc(&c->d_rc32, (size_t)c->lda() * 4)) != cudaSuccess ||
+      (e = cudaMemsetAsync(c->d_rc32, 0, (size_t)c->lda() * 4, s)) != cudaSuccess)
     return fail(cfail(e, "allocation"));
-  dgk::k_coarse_to_f32<<<grid1((int64_t)nagg * nagg), 256, 0, s>>>((int64_t)nagg * nagg, c->d_ainv, c->d_ainv32);
+  dgk::k_coarse_pad32<<<grid1((int64_t)nagg * c->lda()), 256, 0, s>>>(nagg, c->lda(), c->d_ainv, c->d_ainv32);
   if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaStreamSynchronize(s)) != cudaSuccess)
     return fail(cfail(e, "inversion"));
   h->launches += 3 * (int64_t)ncol + 3 * (int64_t)nagg + 1;
@@ -641,7 +664,7 @@ int dgc::coarse_apply(dgc_handle_s* h, const double* r, const double* binv_r, do
     // kernels: each conversion happens once, inside the kernel that produces
     // or consumes the value (same values as converting through FP64 vectors)
     if (!binv_r) {
-      if (int rc = ipdg_block_jacobi_apply_f32(h, r, nullptr, w0, f0, s)) return rc;
+      if (int rc = ipdg_block_jacobi_apply_f32(h, r, w0, f0, s)) return rc;
       binv_r = w0;
     } else if (!binv_r32_ready) {
       dgk::k_coarse_to_f32<<<grid1(n), 256, 0, s>>>(n, binv_r, f0);
@@ -649,24 +672,32 @@ int dgc::coarse_apply(dgc_handle_s* h, const double* r, const double* binv_r, do
     }
     // P^T r = P0^T (r - w S Binv r)
     if (int rc = ipdg_spd_apply_f32(h, f0, f1, s)) return rc;
-    dgk::k_coarse_axpy_z32<<<grid1(n), 256, 0, s>>>(n, r, om, f1, w1);
-    dgk::k_coarse_restrict<<<(c->nagg * 32 + 255) / 256, 256, 0, s>>>(c->nagg, h->NpP, h->Np, c->d_ptr, c->d_cells,
-                                                                    w1, c->d_rc, c->d_rc32);
-    dgk::k_coarse_gemv32<<<(c->nagg * 32 + 255) / 256, 256, 0, s>>>(c->nagg, c->d_ainv32, c->d_rc32, c->d_xc);
+    const int gw = (c->nagg * 32 + 255) / 256;
+    const int64_t nq = n / 4;
+    // the dot product of the step before has been read: cleared for the next one
+    CKC(dgk::launch_plain(dgk::k_coarse_restrict, gw, 256, 0, s, c->nagg, h->NpP, h->Np, (const int32_t*)c->d_ptr,
+                          (const int32_t*)c->d_cells, r, (const float*)f1, om, c->d_rc, c->d_rc32,
+                          c->d_dots ? c->d_dots + 4 : nullptr), "apply");
+    CKC(dgk::launch_plain(dgk::k_coarse_gemv32, gw, 256, 0, s, c->nagg, c->lda(), (const float*)c->d_ainv32,
+                          (const float*)c->d_rc32, c->d_xc), "apply");
     // y = P0 x_c;  z (+)= y - w Binv S y
-    dgk::k_coarse_prolong<<<grid1(n), 256, 0, s>>>(n, h->NpP, h->Np, c->d_agg, c->d_xc, 0, w1, f0);
-    CKC(cudaGetLastError(), "apply");
+    CKC(dgk::launch_plain(dgk::k_coarse_prolong32, grid1(nq), 256, 0, s, nq, h->NpP, h->Np, (const int32_t*)c->d_agg,
+                          (const double*)c->d_xc, f0), "apply");
+    h->launches += 3;
     if (int rc = ipdg_spd_apply_f32(h, f0, f1, s)) return rc;
-    if (int rc = ipdg_block_jacobi_apply_f32(h, nullptr, f1, w0, nullptr, s)) return rc;
+    BjFused io;
+    io.f = f1;
+    io.xc = c->d_xc;
+    io.agg = c->d_agg;
+    io.om = om;
+    io.add = add ? 1 : 0;
     if (dots && add) {
-      CKC(cudaMemsetAsync(dots->out, 0, 3 * 8, s), "dots");
-      dgk::k_coarse_axpy_dots<<<dots->grid, 256, 0, s>>>(n, w1, om, w0, z, dots->r, dots->q, dots->out);
-    } else {
-      dgk::k_coarse_axpy<<<grid1(n), 256, 0, s>>>(n, w1, om, w0, z, add ? 1 : 0);
+      io.dots = dots->out;
+      io.r = const_cast<double*>(dots->r);
+      io.q = dots->q;
+      io.q32 = dots->q32;
     }
-    CKC(cudaGetLastError(), "apply");
-    h->launches += 5;
-    return DGC_OK;
+    return ipdg_block_jacobi_correct(h, io, z, s);
   }
   // P^T r = P0^T (r - w S Binv r)
   if (!binv_r) {
@@ -676,7 +707,7 @@ int dgc::coarse_apply(dgc_handle_s* h, const double* r, const double* binv_r, do
   if (int rc = dgc_laplace_spd_apply(h, binv_r, w1, s)) return rc;
   dgk::k_coarse_axpy<<<grid1(n), 256, 0, s>>>(n, r, om, w1, w1, 0);
   dgk::k_coarse_restrict<<<(c->nagg * 32 + 255) / 256, 256, 0, s>>>(c->nagg, h->NpP, h->Np, c->d_ptr, c->d_cells, w1,
-                                                                  c->d_rc, nullptr);
+                                                                  nullptr, 0.0, c->d_rc, nullptr, nullptr);
   dgk::k_coarse_gemv<<<(c->nagg * 32 + 255) / 256, 256, 0, s>>>(c->nagg, c->d_ainv, c->d_rc, c->d_xc);
   // y = P0 x_c;  z (+)= y - w Binv S y
   dgk::k_coarse_prolong<<<grid1(n), 256, 0, s>>>(n, h->NpP, h->Np, c->d_agg, c->d_xc, 0, w1, nullptr);
@@ -699,7 +730,11 @@ int dgc::two_level_pcg(dgc_handle_s* h, double* x, double* r, double tol2, int m
       CKC(cudaMalloc(&v, n * 8), "allocation");
       CKC(cudaMemset(v, 0, n * 8), "clear");
     }
-    CKC(cudaMalloc(&c->d_dots, 4 * 8), "allocation");
+    // [0..2] dot products, [3] sums of the singular system, [4] p.q of the FP32 operator
+    CKC(cudaMalloc(&c->d_dots, 5 * 8), "allocation");
+    CKC(cudaMemset(c->d_dots, 0, 5 * 8), "clear");
+    CKC(cudaMalloc(&c->d_q32, n * 4), "allocation");
+    CKC(cudaMemset(c->d_q32, 0, n * 4), "clear");
     CKC(cudaMalloc(&c->d_sc, 8 * 8), "allocation");
     CKC(cudaMallocHost(&c->h_sc, 8 * 8), "allocation");
   }
@@ -708,6 +743,8 @@ int dgc::two_level_pcg(dgc_handle_s* h, double* x, double* r, double tol2, int m
   const int gd = grid1(n);
   // reductions end in one atomic per block on the same few addresses: 2 blocks per SM
   const int gr = std::max(1, std::min(gd, 2 * h->sm_count));
+  // kernels with a set-up per CTA (an FP64 division): 8 blocks per SM
+  const int gv = std::max(1, std::min(gd, 8 * h->sm_count));
   // dots of up to three pairs into t, left on the device
   auto dots = [&](dgk::Dot3 d) -> int {
     CKC(cudaMemsetAsync(t, 0, 3 * 8, s), "dots");
@@ -720,11 +757,11 @@ int dgc::two_level_pcg(dgc_handle_s* h, double* x, double* r, double tol2, int m
   // FP32 smoothing leaks a little of them into the coarse term; unchecked, x drifts
   // along them until S x loses its accuracy, so z is kept at zero mean.
   const bool singular = !h->desc.dirichlet && c->shift == 0.0;
-  // with `fused`, the preconditioner's last kernel also forms (r.r, z.r, z.q)
-  // in t (not for the singular system, whose z changes once more afterwards)
-  auto precondition = [&](bool fused) -> int {  // z = Binv r + P A_c^-1 P^T r, Binv and the coarse term in FP32
-    if (int rc = ipdg_block_jacobi_apply_f32(h, r, nullptr, z, c->d_f[0], s)) return rc;
-    const CoarseDots cd{t, r, q, gr};
+  // z = Binv r + P A_c^-1 P^T r, Binv and the coarse term in FP32.  With `fused`, the
+  // last kernel also forms (r.r, z.r, z.q) in t, cleared before (not for the
+  // singular system, whose z changes once more afterwards)
+  auto finish = [&](bool fused) -> int {  // z holds Binv r, the first FP32 work vector its FP32 copy
+    const CoarseDots cd{t, r, op32 ? nullptr : q, op32 ? c->d_q32 : nullptr};
     if (int rc = coarse_apply(h, r, z, z, true, true, s, true, fused && !singular ? &cd : nullptr)) return rc;
     if (singular) {
       CKC(cudaMemsetAsync(t + 3, 0, 8, s), "mean");
@@ -741,11 +778,11 @@ int dgc::two_level_pcg(dgc_handle_s* h, double* x, double* r, double tol2, int m
   float* p32 = op32 ? c->d_f[0] : nullptr;
   auto apply = [&]() -> int {
     if (!op32) return dgc_laplace_spd_apply(h, p, q, s);
-    if (int rc = ipdg_spd_apply_f32(h, p32, c->d_f[1], s)) return rc;
-    // q back in FP64, with t[0] = p.q for the step
-    CKC(cudaMemsetAsync(t, 0, 3 * 8, s), "dots");
-    dgk::k_coarse_to_f64_dot<<<gr, 256, 0, s>>>(n, c->d_f[1], q, p, t);
-    CKC(cudaGetLastError(), "apply");
+    if (int rc = ipdg_spd_apply_f32(h, p32, c->d_q32, s)) return rc;
+    // p.q for the step; q stays in FP32 (its readers convert), except for the dot
+    // products of the singular system
+    CKC(dgk::launch_plain(dgk::k_coarse_dot32, gr, 256, 0, s, n, (const float*)c->d_q32, (const double*)p, t + 4,
+                          singular ? q : nullptr, t), "apply");
     h->launches += 1;
     return DGC_OK;
   };
@@ -759,10 +796,12 @@ int dgc::two_level_pcg(dgc_handle_s* h, double* x, double* r, double tol2, int m
     return DGC_OK;
   };
   CKC(cudaMemsetAsync(sc, 0, 8 * 8, s), "scalars");
-  if (int rc = precondition(false)) return rc;
+  if (int rc = ipdg_block_jacobi_apply_f32(h, r, z, c->d_f[0], s)) return rc;
+  if (int rc = finish(false)) return rc;  // clears t[4] for the first p.q
   if (int rc = dots({{r, z, nullptr}, {r, r, nullptr}})) return rc;
-  dgk::k_coarse_dir_dev<<<gd, 256, 0, s>>>(n, z, p, sc, t, 0, 0, 1, p32);  // p = z, sc[0] = z.r, sc[3] = r.r
-  CKC(cudaGetLastError(), "start");
+  // p = z, sc[0] = z.r, sc[3] = r.r
+  CKC(dgk::launch_plain(dgk::k_coarse_dir_dev, gv, 256, 0, s, n, (const double*)z, p, sc, (const double*)t, 0, 0, 1,
+                        p32), "start");
   double rr = 0.0;
   bool stop = false;
   if (int rc = check(&rr, &stop)) return rc;
@@ -775,13 +814,24 @@ int dgc::two_level_pcg(dgc_handle_s* h, double* x, double* r, double tol2, int m
     if (int rc = apply()) return rc;
     if (!op32)  // the FP32 apply forms p.q while it converts q
       if (int rc = dots({{p, nullptr, nullptr}, {q, nullptr, nullptr}})) return rc;
-    dgk::k_coarse_step_dev<<<gd, 256, 0, s>>>(n, p, q, x, r, sc, t, cur);
-    if (int rc = precondition(true)) return rc;
+    // x += alpha p, r -= alpha q, z = Binv r
+    BjFused st;
+    st.x = x;
+    st.r = r;
+    st.p = p;
+    st.q = q;
+    st.q32 = op32 ? c->d_q32 : nullptr;
+    st.sc = sc;
+    st.pq = op32 ? t + 4 : t;
+    st.cur = cur;
+    if (int rc = ipdg_block_jacobi_step(h, st, z, c->d_f[0], s)) return rc;
+    if (!op32) CKC(cudaMemsetAsync(t, 0, 3 * 8, s), "dots");
+    if (int rc = finish(true)) return rc;
     if (singular)
       if (int rc = dots({{r, z, z}, {r, r, q}})) return rc;
-    dgk::k_coarse_dir_dev<<<gd, 256, 0, s>>>(n, z, p, sc, t, cur, cur ^ 1, 0, p32);
-    CKC(cudaGetLastError(), "update");
-    h->launches += 2;
+    CKC(dgk::launch_plain(dgk::k_coarse_dir_dev, gv, 256, 0, s, n, (const double*)z, p, sc, (const double*)t, cur,
+                          cur ^ 1, 0, p32), "update");
+    ++h->launches;
     ++it;
     if (it % kCheck == 0 || it == maxit)
       if (int rc = check(&rr, &stop)) return rc;

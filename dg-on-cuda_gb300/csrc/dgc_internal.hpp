@@ -71,10 +71,32 @@ void ipdg_operators_changed(dgc_handle_s* h);
 // (FP64 vectors; the blocks and sums in FP32 with fp32)
 int ipdg_build_preconditioner(dgc_handle_s* h, cudaStream_t s);
 int ipdg_block_jacobi_apply(dgc_handle_s* h, const double* r, double* z, cudaStream_t s);
-// z = Binv r with the FP32 blocks, r given in FP64 (r64) or FP32 (r32, used when
-// non-null); z32, when non-null, receives an FP32 copy of z
-int ipdg_block_jacobi_apply_f32(dgc_handle_s* h, const double* r64, const float* r32, double* z, float* z32,
-                                cudaStream_t s);
+// z = Binv r with the FP32 blocks; z32, when non-null, receives an FP32 copy of z
+int ipdg_block_jacobi_apply_f32(dgc_handle_s* h, const double* r, double* z, float* z32, cudaStream_t s);
+// the same as part of the two-level cycle, fused with the vector updates around it
+struct BjFused {
+  // step: x += alpha p, r -= alpha q first, alpha = sc[cur] / *pq (not when the
+  // positivity of either is lost: then sc[6] = 1); q in FP64 (q) or FP32 (q32)
+  double* x = nullptr;
+  double* r = nullptr;
+  const double* p = nullptr;
+  const double* q = nullptr;
+  const float* q32 = nullptr;
+  double* sc = nullptr;
+  const double* pq = nullptr;
+  int cur = 0;
+  // correction: z (+)= y - om Binv f, y = xc[agg] on the valid nodes; with dots
+  // (zero before) also dots += (r.r, z.r, z.q) with the new z
+  const float* f = nullptr;
+  const double* xc = nullptr;
+  const int32_t* agg = nullptr;
+  double om = 0.0;
+  int add = 0;
+  double* dots = nullptr;
+};
+// z = Binv r after the step
+int ipdg_block_jacobi_step(dgc_handle_s* h, const BjFused& io, double* z, float* z32, cudaStream_t s);
+int ipdg_block_jacobi_correct(dgc_handle_s* h, const BjFused& io, double* z, cudaStream_t s);
 // the SPD form's shift, and whether the boundary types are the handle's uniform ones
 double ipdg_shift(const dgc_handle_s* h);
 bool ipdg_uniform_bc(const dgc_handle_s* h);
@@ -83,12 +105,12 @@ bool ipdg_uniform_bc(const dgc_handle_s* h);
 // binv_r32, when non-null, an FP32 copy of binv_r the caller already holds in
 // the coarse space's first FP32 work vector); freeing
 // dots, when non-null (FP32 path with add), makes the last kernel also form
-// out = (r.r, z.r, z.q) with the new z, on `grid` blocks
+// out = (r.r, z.r, z.q) with the new z
 struct CoarseDots {
-  double* out;
+  double* out;  // zero before
   const double* r;
-  const double* q;
-  int grid;
+  const double* q;    // one of the two
+  const float* q32;
 };
 int coarse_apply(dgc_handle_s* h, const double* r, const double* binv_r, double* z, bool add, bool fp32,
                  cudaStream_t s, bool binv_r32_ready = false, const CoarseDots* dots = nullptr);

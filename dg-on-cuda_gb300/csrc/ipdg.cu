@@ -468,74 +468,174 @@ int ipdg_build_preconditioner(dgc_handle_s* h, cudaStream_t s) {
 }
 
 // z = Binv r elementwise (FP64 vectors, native layout; padding nodes of z set to
-// 0), the blocks and the sums in B's type (FP64 here; the FP32 cycle of the
-// two-level preconditioner uses the packed blocks below).  A CTA holds whole
-// elements (blockDim = E * NpP) and stages r once per node in shared memory, in
-// B's type.
-// The residual may also come as an FP32 vector (RIn = float: the two-level
-// cycle's FP32 operator output, no FP64 round trip), and z32, when given,
-// receives an FP32 copy of z (the input of the next FP32 operator apply).
-template <typename B, typename RIn = double>
-__global__ void k_bj_apply(int K, int Np, int NpP, int bstr, const B* __restrict__ binv,
-                           const RIn* __restrict__ r, double* __restrict__ z, float* __restrict__ z32) {
-  __shared__ B rs[256];
+// 0), FP64 blocks and sums.  A CTA holds whole elements (blockDim = E * NpP) and
+// stages r once per node in shared memory.
+__global__ void k_bj_apply(int K, int Np, int NpP, int bstr, const double* __restrict__ binv,
+                           const double* __restrict__ r, double* __restrict__ z) {
+  __shared__ double rs[256];
   const int E = blockDim.x / NpP;
   const int t = threadIdx.x, e = t / NpP, i = t - e * NpP;
   const int64_t k = (int64_t)blockIdx.x * E + e;
   const bool live = k < K;
-  rs[t] = live ? (B)r[k * NpP + i] : (B)0;
+  rs[t] = live ? r[k * NpP + i] : 0.0;
   __syncthreads();
   if (!live) return;
-  B s = 0;
+  double s = 0;
   if (i < Np) {
-    const B* Bk = binv + (size_t)k * bstr;
-    const B* rk = rs + e * NpP;
+    const double* Bk = binv + (size_t)k * bstr;
+    const double* rk = rs + e * NpP;
     for (int j = 0; j < Np; ++j) s += Bk[j * Np + i] * rk[j];
   }
-  z[k * NpP + i] = (double)s;
-  if (z32) z32[k * NpP + i] = (float)s;
+  z[k * NpP + i] = s;
 }
 
-// z = Binv r with the packed FP32 blocks (upper triangles row by row, PK floats
-// per element: the layout the register-blocked CG update stages), for the
-// two-level cycle: 496 instead of 900 bytes of blocks per element at N = 4.
-// A CTA holds whole elements; it copies their packed blocks (contiguous) and
-// residuals into shared memory, and thread (element, node i) sums over j with
-// B(i, j) = B(min, max) through a per-CTA table of packed indices.
-template <int N, typename RIn>
-__global__ void k_bj_apply_pk(int K, const float* __restrict__ bpk, const RIn* __restrict__ r,
-                              double* __restrict__ z, float* __restrict__ z32) {
+enum BjMode : int { BJ_APPLY = 0, BJ_STEP = 1, BJ_CORRECT = 2 };
+
+// Binv applied with the packed FP32 blocks (upper triangles row by row, PK floats
+// per element: the layout the register-blocked CG update stages), fused with the
+// vector updates before or after it in the two-level cycle (BjFused).  CTAs of
+// whole elements loop over the mesh: packed blocks (contiguous) and the FP32
+// input go to shared memory, thread (element, node i) sums over j with
+// B(i, j) = B(min, max) through a per-CTA table of packed indices.  Bound by DRAM
+// and the FP64 pipe; the fusions save the vectors between the kernels: at K =
+// 131072, N = 4 step + apply 50 -> 39 us, apply + correction 55 ->
+// 42 us.
+template <int N, int MODE, typename Q>
+__global__ void __launch_bounds__(256) k_bj_apply_pk(int K, const float* __restrict__ bpk, const double* r,
+                                                     double* __restrict__ z, float* __restrict__ z32,
+                                                     const BjFused io, const Q* __restrict__ qv) {
   // compile-time sizes: the j loop unrolls, so the block and residual reads of
   // a thread are independent loads issued back to back
   constexpr int Np = dgk::IpdgBlk<N>::Np, NpP = dgk::IpdgBlk<N>::NpP, PK = dgk::IpdgBlk<N>::PK;
+  constexpr int E = 256 / NpP;
   extern __shared__ __align__(16) float sm_pk[];
-  const int E = blockDim.x / NpP;
+  __shared__ double red[3][8];
+  __shared__ double s_alpha;
+  __shared__ int s_ok;
   float* sB = sm_pk;                  // [E][PK]
   float* sR = sB + E * PK;            // [E][NpP]
   uint16_t* tab = reinterpret_cast<uint16_t*>(sR + E * NpP);  // [Np][NpP]
   const int t = threadIdx.x, e = t / NpP, i = t - e * NpP;
-  const int64_t k0 = (int64_t)blockIdx.x * E;
-  const int ne = (int)min((int64_t)E, (int64_t)K - k0);
-  const float4* src = reinterpret_cast<const float4*>(bpk + k0 * PK);
-  for (int x = t; x < ne * PK / 4; x += blockDim.x) reinterpret_cast<float4*>(sB)[x] = src[x];
-  if (e < ne) sR[t] = (float)r[(k0 + e) * NpP + i];
-  for (int q = t; q < Np * NpP; q += blockDim.x) {
+  for (int q = t; q < Np * NpP; q += 256) {
     const int j = q / NpP, ii = q - j * NpP;
     const int lo = ii < j ? ii : j, hi = ii < j ? j : ii;
     tab[q] = (uint16_t)(ii >= Np ? 0 : lo * Np - lo * (lo - 1) / 2 + (hi - lo));
   }
-  __syncthreads();
-  if (e >= ne) return;
-  float acc = 0.0f;
-  if (i < Np) {
-    const float* Bk = sB + e * PK;
-    const float* rk = sR + e * NpP;
-#pragma unroll
-    for (int j = 0; j < Np; ++j) acc += Bk[tab[j * NpP + i]] * rk[j];
+  if (MODE == BJ_STEP) {
+    // one FP64 division per CTA
+    if (t == 0) {
+      const double rz = io.sc[io.cur], pq = *io.pq;
+      // at the rounding floor p.Sp or z.r can lose their sign: stop, the caller
+      // checks the true residual
+      const bool ok = pq > 0.0 && rz > 0.0 && io.sc[6] == 0.0;
+      s_alpha = ok ? rz / pq : 0.0;
+      s_ok = ok;
+      if (blockIdx.x == 0) {
+        io.sc[5] = s_alpha;
+        if (!ok) io.sc[6] = 1.0;
+      }
+    }
+    __syncthreads();
   }
-  const int64_t o = (k0 + e) * NpP + i;
-  z[o] = (double)acc;
-  if (z32) z32[o] = acc;
+  double d0 = 0.0, d1 = 0.0, d2 = 0.0;
+  const int ngroups = (K + E - 1) / E;
+  // the next group's loads are in flight while the current one is computed
+  constexpr int kV = (E * PK / 4 + 255) / 256;
+  float4 nb[kV];
+  double nz = 0.0, nr = 0.0, nx = 0.0, np = 0.0, ny = 0.0;
+  float nf = 0.0f;
+  Q nq = Q(0);
+  auto fetch = [&](int g) {
+    if (g >= ngroups) return;
+    const int64_t k0 = (int64_t)g * E;
+    const int ne = (int)min((int64_t)E, (int64_t)K - k0);
+    const float4* src = reinterpret_cast<const float4*>(bpk + k0 * PK);
+#pragma unroll
+    for (int v = 0; v < kV; ++v)
+      if (t + 256 * v < ne * PK / 4) nb[v] = src[t + 256 * v];
+    if (e < ne) {
+      const int64_t o = (k0 + e) * NpP + i;
+      if (MODE == BJ_CORRECT) {
+        nf = io.f[o];
+        ny = i < Np ? io.xc[io.agg[k0 + e]] : 0.0;
+        if (io.add) nz = z[o];
+        if (io.dots) {
+          nr = r[o];
+          nq = qv[o];
+        }
+      } else {
+        nr = r[o];
+        if (MODE == BJ_STEP && s_ok) {
+          nq = qv[o];
+          np = io.p[o];
+          nx = io.x[o];
+        }
+      }
+    }
+  };
+  fetch(blockIdx.x);
+  for (int g = blockIdx.x; g < ngroups; g += gridDim.x) {
+    const int64_t k0 = (int64_t)g * E;
+    const int ne = (int)min((int64_t)E, (int64_t)K - k0);
+    const bool live = e < ne;
+    const int64_t o = (k0 + e) * NpP + i;
+#pragma unroll
+    for (int v = 0; v < kV; ++v)
+      if (t + 256 * v < ne * PK / 4) reinterpret_cast<float4*>(sB)[t + 256 * v] = nb[v];
+    double rv = nr, zv = nz;
+    const double qd = (double)nq, yv = ny;
+    if (live) {
+      if (MODE == BJ_CORRECT) {
+        sR[t] = nf;
+      } else {
+        if (MODE == BJ_STEP && s_ok) {
+          rv -= s_alpha * qd;
+          io.r[o] = rv;
+          io.x[o] = nx + s_alpha * np;
+        }
+        sR[t] = (float)rv;
+      }
+    }
+    __syncthreads();
+    fetch(g + gridDim.x);
+    if (live) {
+      float acc = 0.0f;
+      if (i < Np) {
+        const float* Bk = sB + e * PK;
+        const float* rk = sR + e * NpP;
+#pragma unroll
+        for (int j = 0; j < Np; ++j) acc += Bk[tab[j * NpP + i]] * rk[j];
+      }
+      if (MODE == BJ_CORRECT) {
+        zv += yv - io.om * (double)(acc);
+        z[o] = zv;
+        if (io.dots) {
+          d0 += rv * rv;
+          d1 += zv * rv;
+          d2 += zv * qd;
+        }
+      } else {
+        z[o] = (double)(acc);
+        if (z32) z32[o] = acc;
+      }
+    }
+    __syncthreads();
+  }
+  if (MODE == BJ_CORRECT && io.dots) {
+    double d[3] = {d0, d1, d2};
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+#pragma unroll
+      for (int s = 16; s > 0; s >>= 1) d[j] += __shfl_xor_sync(0xffffffffu, d[j], s);
+      if ((t & 31) == 0) red[j][t >> 5] = d[j];
+    }
+    __syncthreads();
+    if (t < 3) {
+      double v = 0.0;
+      for (int w = 0; w < 8; ++w) v += red[t][w];
+      atomicAdd(io.dots + t, v);
+    }
+  }
 }
 
 int ipdg_block_jacobi_apply(dgc_handle_s* h, const double* r, double* z, cudaStream_t s) {
@@ -543,41 +643,66 @@ int ipdg_block_jacobi_apply(dgc_handle_s* h, const double* r, double* z, cudaStr
   const IpdgState* st = h->ipdg;
   const int E = 256 / h->NpP;  // whole elements per CTA (NpP <= 48)
   const unsigned grid = (unsigned)((h->K + E - 1) / E), block = (unsigned)(E * h->NpP);
-  k_bj_apply<double><<<grid, block, 0, s>>>(h->K, h->Np, h->NpP, st->bstr, st->binv64, r, z, nullptr);
+  k_bj_apply<<<grid, block, 0, s>>>(h->K, h->Np, h->NpP, st->bstr, st->binv64, r, z);
   CKI(cudaGetLastError());
   ++h->launches;
   return DGC_OK;
 }
 
-int ipdg_block_jacobi_apply_f32(dgc_handle_s* h, const double* r64, const float* r32, double* z, float* z32,
-                                cudaStream_t s) {
+namespace {
+
+template <int MODE, typename Q>
+int bj_pk(dgc_handle_s* h, const double* r, double* z, float* z32, const BjFused& io, const Q* q, cudaStream_t s) {
   if (int rc = ipdg_build_preconditioner(h, s)) return rc;
   const IpdgState* st = h->ipdg;
-  const int E = 256 / h->NpP;
-  const unsigned grid = (unsigned)((h->K + E - 1) / E), block = (unsigned)(E * h->NpP);
-  auto go = [&](auto nc) {
+  auto go = [&](auto nc) -> cudaError_t {
     constexpr int N = decltype(nc)::value;
-    constexpr int PK = dgk::IpdgBlk<N>::PK, Np = dgk::IpdgBlk<N>::Np, NpP = dgk::IpdgBlk<N>::NpP;
-    const size_t smem = (size_t)E * PK * 4 + (size_t)E * NpP * 4 + (size_t)Np * NpP * 2;
-    if (r32)
-      k_bj_apply_pk<N, float><<<grid, block, smem, s>>>(h->K, st->binv_pk32, r32, z, z32);
-    else
-      k_bj_apply_pk<N, double><<<grid, block, smem, s>>>(h->K, st->binv_pk32, r64, z, z32);
+    constexpr int PK = dgk::IpdgBlk<N>::PK, Np = dgk::IpdgBlk<N>::Np, NpP = dgk::IpdgBlk<N>::NpP, E = 256 / NpP;
+    constexpr size_t smem = (size_t)E * PK * 4 + (size_t)E * NpP * 4 + (size_t)Np * NpP * 2;
+    auto kern = k_bj_apply_pk<N, MODE, Q>;
+    static std::once_flag once;
+    static cudaError_t st0 = cudaSuccess;
+    static int bps = 1;
+    std::call_once(once, [&] {
+      st0 = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (st0 == cudaSuccess) st0 = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+      if (st0 == cudaSuccess) st0 = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, 256, smem);
+    });
+    if (st0 != cudaSuccess) return st0;
+    const int grid = std::min((h->K + E - 1) / E, h->sm_count * std::max(bps, 1));
+    return dgk::launch_plain(kern, grid, 256, smem, s, h->K, (const float*)st->binv_pk32, r, z, z32, io, q);
   };
+  cudaError_t e = cudaErrorInvalidValue;
   switch (h->N) {
-    case 1: go(std::integral_constant<int, 1>{}); break;
-    case 2: go(std::integral_constant<int, 2>{}); break;
-    case 3: go(std::integral_constant<int, 3>{}); break;
-    case 4: go(std::integral_constant<int, 4>{}); break;
-    case 5: go(std::integral_constant<int, 5>{}); break;
-    case 6: go(std::integral_constant<int, 6>{}); break;
-    case 7: go(std::integral_constant<int, 7>{}); break;
-    case 8: go(std::integral_constant<int, 8>{}); break;
-    default: return set_error(DGC_ERR_ARG, "order outside 1..8");
+    case 1: e = go(std::integral_constant<int, 1>{}); break;
+    case 2: e = go(std::integral_constant<int, 2>{}); break;
+    case 3: e = go(std::integral_constant<int, 3>{}); break;
+    case 4: e = go(std::integral_constant<int, 4>{}); break;
+    case 5: e = go(std::integral_constant<int, 5>{}); break;
+    case 6: e = go(std::integral_constant<int, 6>{}); break;
+    case 7: e = go(std::integral_constant<int, 7>{}); break;
+    case 8: e = go(std::integral_constant<int, 8>{}); break;
+    default: break;
   }
-  CKI(cudaGetLastError());
+  if (e != cudaSuccess) return cuda_err(e, "block-Jacobi apply");
   ++h->launches;
   return DGC_OK;
+}
+
+}  // namespace
+
+int ipdg_block_jacobi_apply_f32(dgc_handle_s* h, const double* r, double* z, float* z32, cudaStream_t s) {
+  return bj_pk<BJ_APPLY, double>(h, r, z, z32, BjFused{}, nullptr, s);
+}
+
+int ipdg_block_jacobi_step(dgc_handle_s* h, const BjFused& io, double* z, float* z32, cudaStream_t s) {
+  return io.q32 ? bj_pk<BJ_STEP, float>(h, io.r, z, z32, io, io.q32, s)
+                : bj_pk<BJ_STEP, double>(h, io.r, z, z32, io, io.q, s);
+}
+
+int ipdg_block_jacobi_correct(dgc_handle_s* h, const BjFused& io, double* z, cudaStream_t s) {
+  return io.q32 ? bj_pk<BJ_CORRECT, float>(h, io.r, z, nullptr, io, io.q32, s)
+                : bj_pk<BJ_CORRECT, double>(h, io.r, z, nullptr, io, io.q, s);
 }
 
 int upload_ipdg_matrices(dgc_handle_s* h) {

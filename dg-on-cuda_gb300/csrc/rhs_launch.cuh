@@ -31,6 +31,13 @@ inline bool stage_overlap_enabled() {
   return on;
 }
 
+// a plain launch with the same argument conversions
+template <typename... Args, typename... Act>
+cudaError_t launch_plain(void (*kern)(Args...), int grid, int threads, size_t smem, cudaStream_t s, Act&&... args) {
+  kern<<<grid, threads, smem, s>>>(static_cast<Args>(std::forward<Act>(args))...);
+  return cudaGetLastError();
+}
+
 template <typename... Args, typename... Act>
 cudaError_t launch_stage(void (*kern)(Args...), int grid, int threads, size_t smem, cudaStream_t s, Act&&... args) {
   cudaLaunchConfig_t cfg = {};
