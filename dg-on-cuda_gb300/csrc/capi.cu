@@ -170,6 +170,30 @@ int upload_operators(dgc_handle_s* h, int form) {
     CK(cudaMemcpy(h->d_eo64[form], eo.data(), eo.size() * sizeof(double), cudaMemcpyHostToDevice));
     h->d_eo_tab[form] = reinterpret_cast<const uint8_t*>(h->d_eo64[form] + nops);
   }
+  if (form == 0 && h->prec == DGC_F32 && h->desc.physics != DGC_LAPLACE) {
+    // the FP32 stage kernel's even / odd operators: rows in groups of G of one
+    // parity, each padded to GP values
+    const dgk::EoDims d(re.N);
+    const int G = dgk::sym_rows(re.N), GP = dgk::sym_pad(G), gE = (d.nE + G - 1) / G, gO = (d.nO + G - 1) / G,
+              KS = (gE + gO) * GP;
+    std::vector<double> eo = dgc::eo_pack(re.N, Dr, Ds, L, nullptr);
+    h->eo_ok[0] = dgc::eo_symmetric(re.N, Dr, Ds, L, nullptr);
+    if (!h->eo_ok[0]) std::fill(eo.begin(), eo.end(), std::nan(""));
+    const std::vector<uint8_t> tab = dgc::eo_tables(re.N);
+    const size_t nops = ((size_t)(d.Np + d.fE) * KS + 3) / 4 * 4;
+    std::vector<float> sy(nops + tab.size() / sizeof(float), 0.0f);
+    for (int c = 0; c < d.Np + d.fE; ++c)
+      for (int r = 0; r < d.Np; ++r) {
+        const bool odd = r >= d.nE;
+        const int q = odd ? r - d.nE : r, col = ((odd ? gE : 0) + q / G) * GP + q % G;
+        const double v = c < d.Np ? eo[(size_t)c * d.Np + r] : eo[(size_t)d.kK() + (size_t)(c - d.Np) * d.Np + r];
+        sy[(size_t)c * KS + col] = (float)v;
+      }
+    std::memcpy(sy.data() + nops, tab.data(), tab.size());
+    if (!h->d_sym32) CK(cudaMalloc(&h->d_sym32, sy.size() * sizeof(float)));
+    CK(cudaMemcpy(h->d_sym32, sy.data(), sy.size() * sizeof(float), cudaMemcpyHostToDevice));
+    h->d_sym_tab = reinterpret_cast<const uint8_t*>(h->d_sym32 + nops);
+  }
   if (form == 0) {
     // register-blocked kernel operand: rows j of Dr^T, Ds^T (j < Np) and m of
     // LIFT^T (m < 3 Nfp), each padded with zeros to NpP columns
@@ -393,6 +417,7 @@ void device_free(dgc_handle_s* h) {
     cudaFree(h->d_mats32[f]);
     cudaFree(h->d_eo64[f]);
   }
+  cudaFree(h->d_sym32);
   cudaFree(h->d_tc_b);
   cudaFree(h->d_blk_b);
   cudaFree(h->d_blk_bs);
@@ -537,7 +562,8 @@ dgk::RhsParams base_params(dgc_handle h) {
   p.bxy = h->d_bxy;
   p.mats = h->prec == DGC_F64 ? h->d_mats64[0] : h->d_mats32[0];
   p.mats_eo = h->prec == DGC_F64 && h->eo_ok[0] ? h->d_eo64[0] : nullptr;
-  p.tab_eo = h->d_eo_tab[0];
+  p.tab_eo = h->prec == DGC_F32 ? h->d_sym_tab : h->d_eo_tab[0];
+  p.mats_sym = h->prec == DGC_F32 && h->eo_ok[0] ? h->d_sym32 : nullptr;
   p.mats_tc = h->prec == DGC_F32 ? h->d_tc_b : nullptr;
   p.mats_blk = h->prec == DGC_F32 ? h->d_blk_b : (h->prec == DGC_F32C ? h->d_blk_bs : nullptr);
   p.ax = h->desc.ax;

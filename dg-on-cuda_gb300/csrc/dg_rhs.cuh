@@ -48,7 +48,8 @@ struct RhsParams {
   const void* mats;   // DrT | DsT | LT, each padded to 16 bytes
   const void* mats_tc;// FP32 tensor-core operand [Dr | Ds | LIFT] (split TF32, core-matrix layout)
   const void* mats_eo; // even / odd operators (eo.hpp) in the kernel type, NULL: no reflection symmetry
-  const uint8_t* tab_eo;  // their pair tables
+  const uint8_t* tab_eo;  // the pair tables of the even / odd operators
+  const void* mats_sym;   // FP32 even / odd operators in row groups (dg_rhs_sym.cuh), NULL: not symmetric
   const void* mats_blk;// FP32 rows of Dr^T | Ds^T | LIFT^T, each padded to NpP columns (weak form)
   double t, dt;       // time of the operator evaluation (offset when t_dev is set), step size
   const double* t_dev;// optional device-resident base time: operator time = *t_dev + t

@@ -101,6 +101,7 @@ cudaError_t rhs_x2_dispatch(int N, int P, const RhsParams& p, int sm_count, cuda
 #include "dg_rhs_tc.cuh"
 #include "dg_rhs_tct.cuh"
 #include "dg_rhs_tcp.cuh"
+#include "dg_rhs_sym.cuh"
 #include "dg_rhs_v2.cuh"
 #include "dg_rhs_x2.cuh"
 
@@ -251,6 +252,29 @@ cudaError_t rhs_tcp(const RhsParams* p, int sm_count, cudaStream_t s, LaunchInfo
   }
 }
 
+// one tile per CTA
+template <int N, int P>
+cudaError_t rhs_sym(const RhsParams* p, cudaStream_t s, LaunchInfo* info) {
+  using C = SymConfig<N, P>;
+  static std::once_flag once;
+  static cudaError_t st = cudaSuccess;
+  static int bps = 0;
+  std::call_once(once, [] {
+    st = cudaFuncSetAttribute(dg_rhs_sym_kernel<N, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
+    if (st == cudaSuccess)
+      st = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, dg_rhs_sym_kernel<N, P>, C::kThreads, C::kSmem);
+  });
+  if (st != cudaSuccess) return st;
+  if (info) {
+    info->threads = C::kThreads;
+    info->tile = C::TE;
+    info->smem = C::kSmem;
+    info->blocks_per_sm = bps;
+    return cudaSuccess;
+  }
+  return launch_stage(dg_rhs_sym_kernel<N, P>, (p->K + C::TE - 1) / C::TE, C::kThreads, C::kSmem, s, *p);
+}
+
 template <int N, int P, int EPT, int MAP>
 cudaError_t rhs_blk(const RhsParams* p, int sm_count, cudaStream_t s, LaunchInfo* info) {
   using C = BlkConfig<N, P, EPT, MAP>;
@@ -280,14 +304,22 @@ cudaError_t rhs_blk(const RhsParams* p, int sm_count, cudaStream_t s, LaunchInfo
 
 // FP32 variants at orders 1..6: 0 = one thread per element-node (dg_rhs_kernel),
 // 1..3 = register-blocked-by-node tile shapes (dg_rhs_v2_kernel), 4 = tensor
-// cores (dg_rhs_tc_kernel), 5, 6 = 4-node x 1 or 2 element blocks
-// (dg_rhs_blk_kernel, mapping 0), 7 = 4-node x 1 element blocks with
-// warp-uniform operator loads (mapping 1), 8 = tensor cores with the A operand
-// in TMEM (dg_rhs_tct_kernel), 9 = its warp-specialized pipelined form
-// (dg_rhs_tcp_kernel, Maxwell; advection runs variant 8).  Orders 7, 8: 0 =
-// dg_rhs_kernel, 1, 2, 3 = dg_rhs_blk_kernel (EPT 1, EPT 2, mapping 1).
+// cores (dg_rhs_tc_kernel), 5 = 4-node x 1 element blocks (dg_rhs_blk_kernel,
+// mapping 0), 6 = even / odd operators with one element per lane
+// (dg_rhs_sym_kernel), 7 = 4-node x 1 element blocks with warp-uniform operator
+// loads (mapping 1), 8 = tensor cores with the A operand in TMEM
+// (dg_rhs_tct_kernel), 9 = its warp-specialized pipelined form (dg_rhs_tcp_kernel,
+// Maxwell; advection runs variant 8).  Orders 7, 8: 0 = dg_rhs_kernel, 1 =
+// dg_rhs_blk_kernel, 2 = dg_rhs_sym_kernel, 3 = dg_rhs_blk_kernel with mapping 1.
 constexpr int kF32Variants = 10;
 constexpr int kF32VariantsHigh = 4;
+
+// variant 6 (2 at orders 7, 8): operators without the reflection symmetry run the
+// blocked kernel
+template <int N, int P>
+cudaError_t rhs_sym_or_blk(const RhsParams* p, int sm, cudaStream_t s, LaunchInfo* info) {
+  return info || p->mats_sym ? rhs_sym<N, P>(p, s, info) : rhs_blk<N, P, 1, 0>(p, sm, s, info);
+}
 
 template <int N, int P>
 cudaError_t rhs_f32_variant(int v, const RhsParams* p, int sm, cudaStream_t s, LaunchInfo* info) {
@@ -296,13 +328,13 @@ cudaError_t rhs_f32_variant(int v, const RhsParams* p, int sm, cudaStream_t s, L
     if (v >= 1 && v <= 3) return rhs_v2<N, P>(v - 1, p, sm, s, info);
     if (v == 4) return rhs_tc<N, P>(p, sm, s, info);
     if (v == 5) return rhs_blk<N, P, 1, 0>(p, sm, s, info);
-    if (v == 6) return rhs_blk<N, P, 2, 0>(p, sm, s, info);
+    if (v == 6) return rhs_sym_or_blk<N, P>(p, sm, s, info);
     if (v == 7) return rhs_blk<N, P, 1, 1>(p, sm, s, info);
     if (v == 8) return rhs_tct<N, P>(p, sm, s, info);
     if (v == 9) return rhs_tcp<N, P>(p, sm, s, info);
   } else {
     if (v == 1) return rhs_blk<N, P, 1, 0>(p, sm, s, info);
-    if (v == 2) return rhs_blk<N, P, 2, 0>(p, sm, s, info);
+    if (v == 2) return rhs_sym_or_blk<N, P>(p, sm, s, info);
     if (v == 3) return rhs_blk<N, P, 1, 1>(p, sm, s, info);
   }
   return cudaErrorInvalidValue;

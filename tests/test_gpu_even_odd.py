@@ -82,6 +82,48 @@ def test_grad_div(N, n):
     D.check()
 
 
+@pytest.mark.parametrize("n", [1, 4, 9])
+@pytest.mark.parametrize("N", range(1, 9))
+def test_fp32_stage(N, n):
+    """dg_rhs_sym_kernel (variant 6, 2 at orders 7 and 8): less than a tile, whole
+    tiles and a ragged last one; RHS, LSERK4 stage and classical RK4."""
+    m = dg.meshes.jittered_square(n, seed=30 + N)
+    o = oracle.Oracle(m.xy, m.cells, N)
+    rng = np.random.default_rng(N)
+    for name, kind in PHYS:
+        D = dg.Discretization(m, name, N, dg.F32, ax=-0.7, ay=0.4)
+        D.set_variant(6 if N <= 6 else 2)
+        p = oracle.problem(kind, ax=-0.7, ay=0.4)
+        q0 = rng.standard_normal(D.Nf * D.K * D.Np).astype(np.float32).astype(np.float64)
+        q = D.upload(q0)
+        ref = o.rhs(p, 0.3, q0)
+        # FP32 rounding (6e-8) through sums of up to 100 terms of one magnitude
+        assert rel(D.download(D.rhs(q, 0.3)), ref) < 2e-5
+        dt = 0.1 * D.info.min_edge / (N + 1) ** 2
+        qb, res = D.empty_state(), D.empty_state()
+        D.lserk4_stage(0, q, qb, res, 0.3, dt)
+        assert rel(D.download(res), dt * ref) < 2e-5
+        work = [D.empty_state() for _ in range(3)]
+        D.rk4_step(q, 0.3, dt, work)
+        assert rel(D.download(q), o.rk4_step(p, 0.3, dt, q0)) < 2e-5
+        D.check()
+
+
+def test_fp32_operators_without_the_symmetry():
+    """The blocked kernel takes over."""
+    N = 6
+    m = dg.meshes.jittered_square(6, seed=2)
+    D = dg.Discretization(m, "maxwell_te", N, dg.F32)
+    q = D.upload(np.random.default_rng(0).standard_normal(D.Nf * D.K * D.Np))
+    Dr, Ds, L = (D.operator(w).copy() for w in (dg.OP_DR_WEAK, dg.OP_DS_WEAK, dg.OP_LIFT))
+    Dr[3, 7] += 0.5
+    D.set_operators(0, Dr, Ds, L)
+    D.set_variant(5)
+    want = D.rhs(q, 0.0).clone()
+    D.set_variant(6)
+    assert torch.equal(D.rhs(q, 0.0), want)
+
+
 def test_operators_without_the_symmetry():
     """The node-by-node kernels take over, and give the caller's operators."""
     N = 4
