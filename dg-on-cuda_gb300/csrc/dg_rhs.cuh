@@ -26,6 +26,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "eo.hpp"
 
 namespace dgk {
 
@@ -38,6 +39,7 @@ struct PhysTraits { static constexpr int Nf = (P == PHYS_ADV) ? 1 : 3; };
 
 struct RhsParams {
   int K;
+  int ntiles;         // tiles of the blocked and compensated kernels, cut evenly (TileCut)
   const void* q_in;   // operator input state
   void* out;          // RHS: rhs | LSERK: next state | RK4: next stage input
   void* aux;          // LSERK: residual | RK4: stage accumulator
@@ -208,9 +210,13 @@ __device__ __forceinline__ bool rhs_v1_tile(const RhsParams& p, const V1Smem<R, 
         for (int c = 0; c < NF; ++c) b[c] = ldg(qb + c * NpP + nd2);
       }
     } else if (P == PHYS_ADV) {
-      const int bf = -1 - nb;
-      const double x = p.bxy[((size_t)bf * Nfp + d) * 2], y = p.bxy[((size_t)bf * Nfp + d) * 2 + 1];
-      b[0] = (R)adv_exact(p, p.t_dev ? *p.t_dev + p.t : p.t, x, y);
+      // the boundary value enters the flux only where the wind blows in
+      b[0] = (R)0;
+      if (!(cax * nx + cay * ny >= (R)0)) {
+        const int bf = -1 - nb;
+        const double x = p.bxy[((size_t)bf * Nfp + d) * 2], y = p.bxy[((size_t)bf * Nfp + d) * 2 + 1];
+        b[0] = (R)adv_exact(p, p.t_dev ? *p.t_dev + p.t : p.t, x, y);
+      }
     } else if (P == PHYS_TM) {  // PEC: H+ = H-, Ez+ = -Ez-
       b[0] = a[0]; b[1] = a[1]; b[2] = -a[2];
     } else {                    // PEC: E+ = -E-, Hz+ = Hz-

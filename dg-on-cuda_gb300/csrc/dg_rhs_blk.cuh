@@ -61,7 +61,13 @@ struct BlkConfig {
   static constexpr uint32_t oMats = 32;
   static constexpr uint32_t oBuf = oMats + kMat;
   static constexpr uint32_t oFlux = oBuf + 2 * kBuf;
-  static constexpr uint32_t kSmem = oFlux + TE * Nf * FSTR * 4;
+  // advection: list of a tile's inflow boundary nodes (count, indices, values).
+  // Their values (FP64 exp or sin) are evaluated by consecutive threads: the nodes
+  // of a boundary row lie in a few lanes of every warp, and the FP64 pipe pays per
+  // warp.  Nodes past the list's end are evaluated where they are used.
+  static constexpr int kBnd = P == PHYS_ADV ? 256 : 0;
+  static constexpr uint32_t oBnd = oFlux + TE * Nf * FSTR * 4;
+  static constexpr uint32_t kSmem = oBnd + kBnd * 8 + (P == PHYS_ADV ? 16 : 0);
   static_assert(NpP % 4 == 0 && kMat % 16 == 0, "16-byte operator rows");
 };
 
@@ -73,12 +79,12 @@ __device__ __forceinline__ float f4c(const float4& v, int i) {
 // double-buffered tile loop.  smem holds BlkConfig's layout with its three
 // mbarriers (initialised by the caller) at offset 0; ph[0], ph[1] are the
 // phases of the tile-buffer barriers, ph[2] that of the operator barrier, kept
-// by the caller across calls.  Every thread must have finished with smem
+// by the caller across calls.  The elements are cut into ntiles tiles.  Every thread must have finished with smem
 // before the call; the call ends in a CTA barrier.  False if a wait expired
 // (uniform across the CTA).
 template <int N, int P, int EPT_, int MAP_>
 __device__ __forceinline__ bool blk_tiles(const RhsParams& p, unsigned char* smem, uint32_t (&ph)[3], int t0,
-                                          int tstep, int tend) {
+                                          int tstep, int tend, int ntiles) {
   using C = BlkConfig<N, P, EPT_, MAP_>;
   constexpr int Np = C::Np, NpP = C::NpP, NFACE = C::NFACE, Nfp = Order<N>::Nfp;
   constexpr int EPT = C::EPT, NG = C::NG, NTE = C::NTE, TE = C::TE, NF = C::Nf, ESTR = C::ESTR;
@@ -94,6 +100,10 @@ __device__ __forceinline__ bool blk_tiles(const RhsParams& p, unsigned char* sme
     return reinterpret_cast<int4*>(smem + C::oBuf + b * C::kBuf + C::kQ + C::kA + C::kG);
   };
   const bool aux_tile = C::kAuxTile && p.mode == MODE_LSERK;
+  const TileCut tiles(p.K, ntiles);
+  int* bcount = reinterpret_cast<int*>(smem + C::oBnd);
+  int* bnode = bcount + 4;
+  float* bval = reinterpret_cast<float*>(bnode + C::kBnd);
 
   const int tid = threadIdx.x;
   // element slot and 4-node group of this thread
@@ -104,10 +114,11 @@ __device__ __forceinline__ bool blk_tiles(const RhsParams& p, unsigned char* sme
 
   // the padding columns of the flux rows are never written by the face phase
   for (int x = tid; x < TE * NF * FSTR; x += NT) sF[x] = 0.0f;
+  if (P == PHYS_ADV && tid == 0) *bcount = 0;
   __syncthreads();
 
   auto issue = [&](int tile, int b) {
-    const int k0 = tile * TE, ne = min(TE, p.K - k0);
+    const int k0 = tiles.start(tile), ne = tiles.size(tile);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     const uint32_t bq = ne * ESTR * 4, bg = ne * 16 * 4, bn = ne * 16;
     mbar_arrive_expect_tx(&bar[b], bq + (aux_tile ? bq : 0) + bg + bn);
@@ -133,7 +144,7 @@ __device__ __forceinline__ bool blk_tiles(const RhsParams& p, unsigned char* sme
   int it = 0;
   for (int tile = t0; tile < tend; tile += tstep, ++it) {
     const int b = it & 1;
-    const int k0 = tile * TE, ne = min(TE, p.K - k0);
+    const int k0 = tiles.start(tile), ne = tiles.size(tile);
     const int nxt = tile + tstep;
     // buffer b^1 was last read in the previous iteration, which ended in a
     // CTA barrier, so it (and its mbarrier) can be refilled now
@@ -255,6 +266,32 @@ __device__ __forceinline__ bool blk_tiles(const RhsParams& p, unsigned char* sme
     // deep (it waits for this grid before its reads)
     if (tile + tstep >= tend) grid_dep_launch();
 
+    // ---- inflow boundary nodes (advection): listed, then evaluated; a flux entry
+    //      holds its node's place in the list until the flux replaces it
+    if constexpr (P == PHYS_ADV) {
+#pragma unroll
+      for (int s = 0; s < C::kFItems; ++s) {
+        const int x = tid + s * NT;
+        if (x >= ne * Nfp) break;
+        const int e = x / Nfp, d = x - e * Nfp;
+        const int4 nb4 = sN[e];
+#pragma unroll
+        for (int f = 0; f < 3; ++f) {
+          const int nb = f == 0 ? nb4.x : (f == 1 ? nb4.y : nb4.z);
+          if (nb < 0 && !(cax * sG[e * 16 + 8 + f] + cay * sG[e * 16 + 11 + f] >= 0.0f)) {
+            const int at = atomicAdd(bcount, 1);
+            if (at < C::kBnd) bnode[at] = (-1 - nb) * Nfp + d;
+            sF[e * FSTR + f * Nfp + d] = __int_as_float(at);
+          }
+        }
+      }
+      __syncthreads();
+      const int nlist = min(*bcount, C::kBnd);
+      for (int x = tid; x < nlist; x += NT)
+        bval[x] = (float)adv_exact(p, tnow, p.bxy[(size_t)bnode[x] * 2], p.bxy[(size_t)bnode[x] * 2 + 1]);
+      if (nlist > 0) __syncthreads();
+    }
+
     // ---- face nodes: item (element e, face-node index d) takes node d of the
     //      three faces of e; the own and neighbour values of all three are
     //      gathered first, then the three fluxes formed
@@ -282,9 +319,16 @@ __device__ __forceinline__ bool blk_tiles(const RhsParams& p, unsigned char* sme
             for (int c = 0; c < NF; ++c) bv[f][c] = __ldg(qb + c * NpP);
           }
         } else if (P == PHYS_ADV) {
-          const int bf = -1 - nb;
-          const double xx = p.bxy[((size_t)bf * Nfp + d) * 2], yy = p.bxy[((size_t)bf * Nfp + d) * 2 + 1];
-          bv[f][0] = (float)adv_exact(p, tnow, xx, yy);
+          bv[f][0] = 0.0f;  // enters only where the wind blows in
+          if (!(cax * sG[e * 16 + 8 + f] + cay * sG[e * 16 + 11 + f] >= 0.0f)) {
+            const int at = __float_as_int(sF[e * FSTR + f * Nfp + d]);
+            if (at < C::kBnd) {
+              bv[f][0] = bval[at];
+            } else {
+              const double* xy = p.bxy + ((size_t)(-1 - nb) * Nfp + d) * 2;
+              bv[f][0] = (float)adv_exact(p, tnow, xy[0], xy[1]);
+            }
+          }
         } else if (P == PHYS_TM) {  // PEC: H+ = H-, Ez+ = -Ez-
           bv[f][0] = av[f][0]; bv[f][1] = av[f][1]; bv[f][2] = -av[f][2];
         } else {                    // PEC: E+ = -E-, Hz+ = Hz-
@@ -317,6 +361,7 @@ __device__ __forceinline__ bool blk_tiles(const RhsParams& p, unsigned char* sme
       }
     }
     __syncthreads();
+    if (P == PHYS_ADV && tid == 0) *bcount = 0;
 
     // ---- lift + epilogue
     if (slot < NTE) {
@@ -416,7 +461,7 @@ __global__ void __launch_bounds__(BlkConfig<N, P, EPT_, MAP_>::kThreads, BlkConf
   }
   __syncthreads();
   uint32_t ph[3] = {0, 0, 0};
-  blk_tiles<N, P, EPT_, MAP_>(p, smem, ph, blockIdx.x, gridDim.x, (p.K + C::TE - 1) / C::TE);
+  blk_tiles<N, P, EPT_, MAP_>(p, smem, ph, blockIdx.x, gridDim.x, p.ntiles, p.ntiles);
 }
 
 }  // namespace dgk

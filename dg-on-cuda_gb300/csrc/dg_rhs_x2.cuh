@@ -104,7 +104,8 @@ __global__ void __launch_bounds__(X2Config<N, P>::kThreads, X2Config<N, P>::kMin
 
   const int tid = threadIdx.x;
   const int slot = tid / NG, grp = tid - (tid / NG) * NG;
-  const int ntiles = (p.K + TE - 1) / TE;
+  const int ntiles = p.ntiles;
+  const TileCut tiles(p.K, ntiles);
   const size_t nvec = (size_t)p.K * ESTR;
   const float* qhi = static_cast<const float*>(p.q_in);
   const float* qlo = qhi + nvec;
@@ -120,7 +121,7 @@ __global__ void __launch_bounds__(X2Config<N, P>::kThreads, X2Config<N, P>::kMin
   __syncthreads();
 
   auto issue = [&](int tile, int b) {
-    const int k0 = tile * TE, ne = min(TE, p.K - k0);
+    const int k0 = tiles.start(tile), ne = tiles.size(tile);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     const uint32_t bq = ne * ESTR * 4, bg = ne * 16 * 4, bn = ne * 16;
     mbar_arrive_expect_tx(&bar[b], 2 * bq + bg + bn);
@@ -145,7 +146,7 @@ __global__ void __launch_bounds__(X2Config<N, P>::kThreads, X2Config<N, P>::kMin
   int it = 0;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
     const int b = it & 1;
-    const int k0 = tile * TE, ne = min(TE, p.K - k0);
+    const int k0 = tiles.start(tile), ne = tiles.size(tile);
     const int nxt = tile + gridDim.x;
     if (tid == 0 && nxt < ntiles) issue(nxt, b ^ 1);
     if (!__syncthreads_and(mbar_wait(&bar[b], ph[b], p.status))) return;
@@ -291,9 +292,12 @@ __global__ void __launch_bounds__(X2Config<N, P>::kThreads, X2Config<N, P>::kMin
 #pragma unroll
           for (int c = 0; c < NF; ++c) d[f][c] = __fadd_rn(__fsub_rn(bh[c], ah[c]), __fsub_rn(bl[c], al[c]));
         } else if (P == PHYS_ADV) {
-          const int bf = -1 - nb;
-          const double xx = p.bxy[((size_t)bf * Nfp + dd) * 2], yy = p.bxy[((size_t)bf * Nfp + dd) * 2 + 1];
-          d[f][0] = (float)((adv_exact(p, tnow, xx, yy) - (double)ah[0]) - (double)al[0]);
+          d[f][0] = 0.0f;  // enters only where the wind blows in
+          if (cax * sG[e * 16 + 8 + f] + cay * sG[e * 16 + 11 + f] < 0.0f) {
+            const int bf = -1 - nb;
+            const double xx = p.bxy[((size_t)bf * Nfp + dd) * 2], yy = p.bxy[((size_t)bf * Nfp + dd) * 2 + 1];
+            d[f][0] = (float)((adv_exact(p, tnow, xx, yy) - (double)ah[0]) - (double)al[0]);
+          }
         } else if (P == PHYS_TM) {  // PEC: H+ = H-, Ez+ = -Ez-
           d[f][0] = 0.0f; d[f][1] = 0.0f; d[f][2] = -2.0f * ah[2] - 2.0f * al[2];
         } else {                    // PEC: E+ = -E-, Hz+ = Hz-

@@ -89,6 +89,17 @@ struct TileCut {
   DGC_HD int size(int i) const { return len + (i < rem ? 1 : 0); }
 };
 
+// Tiles of the register-blocked kernels (FP32 and compensated stages, FP32 CG), cut
+// evenly (TileCut): as many as full tiles make, at least one per SM.  On meshes with
+// fewer full tiles than SMs a launch is latency (FP32 stage, Maxwell TE, K = 128,
+// N = 3: 3.8 -> 3.0 us; CG iteration, K = 3200, N = 3: 19.8 -> 15.0 us with the
+// convergence test in the grad pass); rounding larger counts up to whole waves took
+// the CG iteration at K = 131072, N = 4 from 95 to 98 us.
+inline int blk_tiles_for(int K, int sm_count, int te_max) {
+  const int full = (K + te_max - 1) / te_max;
+  return full >= sm_count ? full : (K < sm_count ? K : sm_count);
+}
+
 }  // namespace dgk
 
 namespace dgc {

@@ -18,16 +18,6 @@
 
 namespace dgk {
 
-// Tiles of the register-blocked kernels, cut evenly (TileCut): as many as full
-// tiles make, at least one per SM.  On meshes with fewer full tiles than SMs an
-// iteration is latency (K = 3200, N = 3: 19.8 -> 15.0 us with one tile per SM and
-// the convergence test in the grad pass instead of a launch); rounding larger counts up to whole waves
-// took K = 131072, N = 4 from 95 to 98 us per iteration.
-inline int blk_tiles_for(int K, int sm_count, int te_max) {
-  const int full = (K + te_max - 1) / te_max;
-  return full >= sm_count ? full : (K < sm_count ? K : sm_count);
-}
-
 template <int N>
 struct IpdgBlk {
   using O = Order<N>;

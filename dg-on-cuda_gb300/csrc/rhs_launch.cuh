@@ -296,10 +296,10 @@ cudaError_t rhs_blk(const RhsParams* p, int sm_count, cudaStream_t s, LaunchInfo
     return cudaSuccess;
   }
   if (!p->mats_blk) return cudaErrorInvalidValue;
-  const int ntiles = (p->K + C::TE - 1) / C::TE;
-  int grid = sm_count * (bps > 0 ? bps : 1);
-  if (grid > ntiles) grid = ntiles;
-  return launch_stage(dg_rhs_blk_kernel<N, P, EPT, MAP>, grid, C::kThreads, C::kSmem, s, *p);
+  RhsParams q = *p;
+  q.ntiles = blk_tiles_for(p->K, sm_count, C::TE);
+  const int grid = std::min(q.ntiles, sm_count * (bps > 0 ? bps : 1));
+  return launch_stage(dg_rhs_blk_kernel<N, P, EPT, MAP>, grid, C::kThreads, C::kSmem, s, q);
 }
 
 // FP32 variants at orders 1..6: 0 = one thread per element-node (dg_rhs_kernel),

@@ -24,10 +24,10 @@ static cudaError_t rhs_x2(const RhsParams* p, int sm_count, cudaStream_t s, Laun
     return cudaSuccess;
   }
   if (!p->mats_blk) return cudaErrorInvalidValue;
-  const int ntiles = (p->K + C::TE - 1) / C::TE;
-  int grid = sm_count * (bps > 0 ? bps : 1);
-  if (grid > ntiles) grid = ntiles;
-  return launch_stage(dg_rhs_x2_kernel<N, P>, grid, C::kThreads, C::kSmem, s, *p);
+  RhsParams q = *p;
+  q.ntiles = blk_tiles_for(p->K, sm_count, C::TE);
+  const int grid = std::min(q.ntiles, sm_count * (bps > 0 ? bps : 1));
+  return launch_stage(dg_rhs_x2_kernel<N, P>, grid, C::kThreads, C::kSmem, s, q);
 }
 
 template <int N>
