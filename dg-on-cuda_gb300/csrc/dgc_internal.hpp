@@ -125,6 +125,9 @@ int two_level_pcg(dgc_handle_s* h, double* x, double* r, double tol2, int maxit,
 int ipdg_boundary_cells(const dgc_handle_s* h, const int** cells, int* n);
 // out = S u with the FP32 kernels (any laplace handle; one field, native layout)
 int ipdg_spd_apply_f32(dgc_handle_s* h, const float* u, float* out, cudaStream_t s);
+// the same for `fields` consecutive fields in one pair of launches (u 16-byte
+// aligned; q: workspace of 2 x fields fields)
+int ipdg_spd_apply_f32_many(dgc_handle_s* h, const float* u, float* out, int fields, float* q, cudaStream_t s);
 // stage-kernel parameters of a handle (geometry, operators, physics; no buffers)
 dgk::RhsParams rhs_base_params(dgc_handle_s* h);
 // LSERK4 (Carpenter-Kennedy) coefficients: 0 -> a_k, 1 -> b_k, 2 -> c_k (5 each)

@@ -107,18 +107,21 @@ cudaError_t ipdg_eo_launch(int N, int kind, const IpdgParams& p, int sm, cudaStr
 }
 
 // register-blocked FP32 CG kernels
-enum IpdgBlkKernel : int { IB_GRAD = 0, IB_DIV = 1, IB_UPDATE = 2 };
+enum IpdgBlkKernel : int { IB_GRAD = 0, IB_DIV = 1, IB_UPDATE = 2, IB_GRAD_MULTI = 3, IB_DIV_MULTI = 4 };
 
 template <int N>
 cudaError_t ipdg_blk_launch_n(int kind, const IpdgParams& p, int sm, cudaStream_t s, bool graph) {
   using B = IpdgBlk<N>;
-  static std::once_flag once[3];
-  static int bps[3];
-  static cudaError_t st[3];
-  const void* fn = kind == IB_GRAD ? (const void*)ipdg_grad_blk_kernel<N>
-                   : kind == IB_DIV ? (const void*)ipdg_div_blk_kernel<N>
-                                    : (const void*)pcg_update_blk_kernel<N>;
-  const int smem = (int)(kind == IB_GRAD ? B::kSmemGrad : kind == IB_DIV ? B::kSmemDiv : B::kSmemUpd);
+  static std::once_flag once[5];
+  static int bps[5];
+  static cudaError_t st[5];
+  static const void* const fns[5] = {(const void*)ipdg_grad_blk_kernel<N, false>,
+                                     (const void*)ipdg_div_blk_kernel<N, false>, (const void*)pcg_update_blk_kernel<N>,
+                                     (const void*)ipdg_grad_blk_kernel<N, true>,
+                                     (const void*)ipdg_div_blk_kernel<N, true>};
+  const void* fn = fns[kind];
+  const int smem = (int)(kind == IB_UPDATE ? B::kSmemUpd
+                         : kind == IB_GRAD || kind == IB_GRAD_MULTI ? B::kSmemGrad : B::kSmemDiv);
   std::call_once(once[kind], [&] {
     st[kind] = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     // all of the unified L1 / shared storage as shared memory, so residency is
@@ -131,7 +134,8 @@ cudaError_t ipdg_blk_launch_n(int kind, const IpdgParams& p, int sm, cudaStream_
   if (st[kind] != cudaSuccess) return st[kind];
   IpdgParams q = p;
   q.ntiles = blk_tiles_for(p.K, sm, B::TE);
-  const int grid = std::min(q.ntiles, sm * (bps[kind] > 0 ? bps[kind] : 1));
+  const int64_t all = (int64_t)q.ntiles * (kind >= IB_GRAD_MULTI ? p.fields : 1);
+  const int grid = (int)std::min<int64_t>(all, sm * (bps[kind] > 0 ? bps[kind] : 1));
   // programmatic dependent launch (the kernels wait, grid_dep_wait, before their
   // first access to the CG scalars and vectors), but from a graph only where every
   // CTA has one tile: iteration at K = 32768, N = 4 35.1 us against 36.7 launched
@@ -191,6 +195,12 @@ cudaError_t bc_jump_launch(int N, int ncells, const IpdgParams& p, const int* ce
     default: return cudaErrorInvalidValue;
   }
 #undef DGK_BJ
+}
+
+// tiles of one field (ipdg_blk_launch_n)
+int64_t packed_tiles(int N, int K, int sm) {
+  const int npp = ((N + 1) * (N + 2) / 2 + 3) / 4 * 4;
+  return blk_tiles_for(K, sm, 256 / (npp / 4));
 }
 
 // floats per packed block (IpdgBlk<N>::PK) for the allocation on the host
@@ -993,6 +1003,29 @@ int true_residual(dgc_handle_s* h, const double* b64, const double* x64, double*
 }
 
 }  // namespace
+
+int ipdg_spd_apply_f32_many(dgc_handle_s* h, const float* u, float* out, int fields, float* q, cudaStream_t s) {
+  if (int rc = check_laplace(h)) return rc;
+  const int64_t all = (int64_t)fields * dgk::packed_tiles(h->N, h->K, h->sm_count);
+  if (h->ipdg->bcdir || fields == 1 || all > INT32_MAX / 2) {
+    for (int f = 0; f < fields; ++f)
+      if (int rc = ipdg_spd_apply_f32(h, u + f * nvec(h), out + f * nvec(h), s)) return rc;
+    return DGC_OK;
+  }
+  dgk::IpdgParams p = base<float>(h);
+  p.u = u;
+  p.fields = fields;
+  p.qx = q;
+  p.qy = q + fields * nvec(h);
+  cudaError_t e = dgk::ipdg_blk_launch(h->N, dgk::IB_GRAD_MULTI, p, h->sm_count, s, false);
+  if (e != cudaSuccess) return cuda_err(e, "ipdg blocked kernel launch");
+  p.du_src = u;
+  p.out = out;
+  e = dgk::ipdg_blk_launch(h->N, dgk::IB_DIV_MULTI, p, h->sm_count, s, false);
+  if (e != cudaSuccess) return cuda_err(e, "ipdg blocked kernel launch");
+  h->launches += 2;
+  return DGC_OK;
+}
 
 int ipdg_spd_apply_f32(dgc_handle_s* h, const float* u, float* out, cudaStream_t s) {
   if (int rc = check_laplace(h)) return rc;

@@ -85,6 +85,7 @@ struct IpdgParams {
   CgScalars* cg;
   double* dot_out;      // DIV_SPD_DOT / DIV_RESID: accumulated dot product
   int ntiles;           // register-blocked kernels: tiles, cut evenly (TileCut)
+  int fields;           // register-blocked applies of many fields: their number, K NpP values apart
   int slot;             // iteration slot (i mod 3)
   int first;            // first iteration: beta = 0
   int* status;

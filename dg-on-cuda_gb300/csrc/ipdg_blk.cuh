@@ -89,8 +89,11 @@ __device__ __forceinline__ float col_shfl(const float4& v, int j) {
 }
 
 // ---------------------------------------------------------------- grad pass
-// p = z + beta p_old (written), qx, qy = grad p (strong form, jumps lifted)
-template <int N>
+// p = z + beta p_old (written), qx, qy = grad p (strong form, jumps lifted).  MULTI:
+// p = z for p.fields fields, nothing read or written for the direction (a template:
+// the 64 registers that let 4 CTAs share an SM are all in use; as a run-time branch
+// the single-field pass took 29.6 instead of 24.3 us at K = 131072, N = 4)
+template <int N, bool MULTI>
 __global__ void __launch_bounds__(256, 4) ipdg_grad_blk_kernel(const IpdgParams p) {
   using B = IpdgBlk<N>;
   constexpr int Np = B::Np, NpP = B::NpP, Nfp = B::Nfp, NFACE = B::NFACE, NG = B::NG, TE = B::TE;
@@ -110,21 +113,21 @@ __global__ void __launch_bounds__(256, 4) ipdg_grad_blk_kernel(const IpdgParams 
   __shared__ int s_done;
   const int tid = threadIdx.x;
   const int slot = tid / NG, grp = tid - slot * NG;
-  const int ntiles = p.ntiles;
-  const TileCut tiles(p.K, ntiles);
-  const float* zin = static_cast<const float*>(p.u);
+  const int ntiles = MULTI ? p.ntiles * p.fields : p.ntiles;
+  const TileCut tiles(p.K, p.ntiles);
+  const size_t flen = (size_t)p.K * NpP;
   const float* pold = static_cast<const float*>(p.p_old);
   float* pv = static_cast<float*>(p.p);
-  float* qxo = static_cast<float*>(p.qx);
-  float* qyo = static_cast<float*>(p.qy);
 
   auto issue = [&](int tile, int b) {
-    const int k0 = tiles.start(tile), ne = tiles.size(tile);
+    const int fld = MULTI ? tile / p.ntiles : 0, ft = tile - fld * p.ntiles;
+    const int k0 = tiles.start(ft), ne = tiles.size(ft);
+    const float* zin = static_cast<const float*>(p.u) + fld * flen;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     const uint32_t bf = ne * NpP * 4, bg = ne * 64, bn = ne * 16;
-    mbar_arrive_expect_tx(&bar[b], 2 * bf + bg + bn);
+    mbar_arrive_expect_tx(&bar[b], (MULTI ? 1 : 2) * bf + bg + bn);
     bulk_g2s(bufZ(b), zin + (size_t)k0 * NpP, bf, &bar[b]);
-    bulk_g2s(bufP(b), pold + (size_t)k0 * NpP, bf, &bar[b]);
+    if (!MULTI) bulk_g2s(bufP(b), pold + (size_t)k0 * NpP, bf, &bar[b]);
     bulk_g2s(bufG(b), static_cast<const float*>(p.geom) + (size_t)k0 * 16, bg, &bar[b]);
     bulk_g2s(bufN(b), p.nbr + k0, bn, &bar[b]);
   };
@@ -145,16 +148,16 @@ __global__ void __launch_bounds__(256, 4) ipdg_grad_blk_kernel(const IpdgParams 
   // are set-up data (their copy is in flight already)
   grid_dep_wait();
   if (tid == 0) {
-    const int d = p.first ? p.cg->done : cg_decide(*p.cg, p.slot);
+    const int d = MULTI ? 0 : p.first ? p.cg->done : cg_decide(*p.cg, p.slot);
     s_done = d;
     if (!d) {
       if ((int)blockIdx.x < ntiles) issue(blockIdx.x, 0);  // in flight during the division
       s_beta = 0.0f;
-      if (!p.first) {
+      if (!MULTI && !p.first) {
         const int s = p.slot, sp = (s + 2) % 3;
         s_beta = (float)(p.cg->rz[s] / p.cg->rz[sp]);
       }
-      if (blockIdx.x == 0) p.cg->pAp = 0.0;
+      if (!MULTI && blockIdx.x == 0) p.cg->pAp = 0.0;
     } else if (blockIdx.x == 0) {
       p.cg->done = d;
     }
@@ -166,7 +169,9 @@ __global__ void __launch_bounds__(256, 4) ipdg_grad_blk_kernel(const IpdgParams 
   int it = 0;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
     const int b = it & 1;
-    const int k0 = tiles.start(tile), ne = tiles.size(tile);
+    const int fld = MULTI ? tile / p.ntiles : 0, ft = tile - fld * p.ntiles;
+    const int k0 = tiles.start(ft), ne = tiles.size(ft);
+    const float* zin = static_cast<const float*>(p.u) + fld * flen;
     const int nxt = tile + gridDim.x;
     if (tid == 0 && nxt < ntiles) issue(nxt, b ^ 1);
     if (!__syncthreads_and(mbar_wait(&bar[b], ph[b], p.status))) return;
@@ -176,7 +181,7 @@ __global__ void __launch_bounds__(256, 4) ipdg_grad_blk_kernel(const IpdgParams 
     const float* sG = bufG(b);
     const int4* sN = bufN(b);
     // p = z + beta p_old on the tile (in place over z), written out
-    if (slot < ne) {
+    if (!MULTI && slot < ne) {
       float4* u4 = reinterpret_cast<float4*>(sU) + slot * NG + grp;
       const float4 z4 = *u4, o4 = reinterpret_cast<const float4*>(sP)[slot * NG + grp];
       const float4 v = make_float4(fmaf(beta, o4.x, z4.x), fmaf(beta, o4.y, z4.y), fmaf(beta, o4.z, z4.z),
@@ -206,7 +211,7 @@ __global__ void __launch_bounds__(256, 4) ipdg_grad_blk_kernel(const IpdgParams 
             vz[q] = sU[(kn - k0) * NpP + nd2];
           } else {
             vz[q] = __ldg(zin + (size_t)kn * NpP + nd2);
-            vp[q] = __ldg(pold + (size_t)kn * NpP + nd2);
+            if (!MULTI) vp[q] = __ldg(pold + (size_t)kn * NpP + nd2);
           }
         } else {  // Dirichlet: u+ = -u- (du = 2 u-); Neumann: u+ = u- (du = 0)
           const float um = sU[e * NpP + fmask<N>(f, d)];
@@ -277,9 +282,9 @@ __global__ void __launch_bounds__(256, 4) ipdg_grad_blk_kernel(const IpdgParams 
       qy.z = ry * ur.z + sy * us.z + ly.z;
       qy.w = ry * ur.w + sy * us.w + ly.w;
       if (slot < ne) {
-        const size_t o = (size_t)(k0 + slot) * NpP;
-        reinterpret_cast<float4*>(qxo + o)[grp] = qx;  // padding columns of the operators are zero
-        reinterpret_cast<float4*>(qyo + o)[grp] = qy;
+        const size_t o = fld * flen + (size_t)(k0 + slot) * NpP;
+        reinterpret_cast<float4*>(static_cast<float*>(p.qx) + o)[grp] = qx;  // padding columns of the operators are zero
+        reinterpret_cast<float4*>(static_cast<float*>(p.qy) + o)[grp] = qy;
       }
     }
     __syncthreads();
@@ -287,8 +292,9 @@ __global__ void __launch_bounds__(256, 4) ipdg_grad_blk_kernel(const IpdgParams 
 }
 
 // ---------------------------------------------------------------- div pass
-// Ap = S p = -J M (div q + lifted penalty / flux jumps); pAp accumulated
-template <int N>
+// Ap = S p = -J M (div q + lifted penalty / flux jumps); pAp accumulated.  MULTI:
+// p.fields fields, no dot product
+template <int N, bool MULTI>
 __global__ void __launch_bounds__(256, 4) ipdg_div_blk_kernel(const IpdgParams p) {
   using B = IpdgBlk<N>;
   constexpr int Np = B::Np, NpP = B::NpP, Nfp = B::Nfp, NFACE = B::NFACE, NG = B::NG, TE = B::TE;
@@ -313,15 +319,16 @@ __global__ void __launch_bounds__(256, 4) ipdg_div_blk_kernel(const IpdgParams p
   };
   const int tid = threadIdx.x;
   const int slot = tid / NG, grp = tid - slot * NG;
-  const int ntiles = p.ntiles;
-  const TileCut tiles(p.K, ntiles);
-  const float* qx = static_cast<const float*>(p.qx);
-  const float* qy = static_cast<const float*>(p.qy);
-  const float* uj = static_cast<const float*>(p.du_src);
-  float* out = static_cast<float*>(p.out);
+  const int ntiles = MULTI ? p.ntiles * p.fields : p.ntiles;
+  const TileCut tiles(p.K, p.ntiles);
+  const size_t flen = (size_t)p.K * NpP;
 
   auto issue = [&](int tile, int b) {
-    const int k0 = tiles.start(tile), ne = tiles.size(tile);
+    const int fld = MULTI ? tile / p.ntiles : 0, ft = tile - fld * p.ntiles;
+    const int k0 = tiles.start(ft), ne = tiles.size(ft);
+    const float* qx = static_cast<const float*>(p.qx) + fld * flen;
+    const float* qy = static_cast<const float*>(p.qy) + fld * flen;
+    const float* uj = static_cast<const float*>(p.du_src) + fld * flen;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     const uint32_t bf = ne * NpP * 4, bg = ne * 64, bn = ne * 16, bt = ne * 16;
     mbar_arrive_expect_tx(&bar[b], 3 * bf + bg + bn + bt);
@@ -348,9 +355,9 @@ __global__ void __launch_bounds__(256, 4) ipdg_div_blk_kernel(const IpdgParams p
   // the CG scalars and vectors are earlier launches' output; the operators
   // are set-up data (their copy is in flight already)
   grid_dep_wait();
-  const bool done = p.cg->done != 0;
+  const bool done = !MULTI && p.cg->done != 0;
   if (tid == 0 && !done) {
-    if (blockIdx.x == 0) {
+    if (!MULTI && blockIdx.x == 0) {
       const int s1 = (p.slot + 1) % 3;
       p.cg->rz[s1] = 0.0;
       p.cg->rr[s1] = 0.0;
@@ -364,7 +371,12 @@ __global__ void __launch_bounds__(256, 4) ipdg_div_blk_kernel(const IpdgParams p
   int it = 0;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
     const int b = it & 1;
-    const int k0 = tiles.start(tile), ne = tiles.size(tile);
+    const int fld = MULTI ? tile / p.ntiles : 0, ft = tile - fld * p.ntiles;
+    const int k0 = tiles.start(ft), ne = tiles.size(ft);
+    const float* qx = static_cast<const float*>(p.qx) + fld * flen;
+    const float* qy = static_cast<const float*>(p.qy) + fld * flen;
+    const float* uj = static_cast<const float*>(p.du_src) + fld * flen;
+    float* out = static_cast<float*>(p.out) + fld * flen;
     const int nxt = tile + gridDim.x;
     if (tid == 0 && nxt < ntiles) issue(nxt, b ^ 1);
     if (!__syncthreads_and(mbar_wait(&bar[b], ph[b], p.status))) return;
@@ -383,7 +395,7 @@ __global__ void __launch_bounds__(256, 4) ipdg_div_blk_kernel(const IpdgParams p
         sm.w *= mJ;
         reinterpret_cast<float4*>(out + (size_t)(k0 + slot) * NpP)[grp] = sm;
         const float4 pu = reinterpret_cast<const float4*>(bufU(b) + slot * NpP)[grp];
-        dot += (double)pu.x * sm.x + (double)pu.y * sm.y + (double)pu.z * sm.z + (double)pu.w * sm.w;
+        if (!MULTI) dot += (double)pu.x * sm.x + (double)pu.y * sm.y + (double)pu.z * sm.z + (double)pu.w * sm.w;
       }
     };
     const float* sX = bufX(b);
@@ -499,8 +511,10 @@ __global__ void __launch_bounds__(256, 4) ipdg_div_blk_kernel(const IpdgParams p
     }
     __syncthreads();
   }
-  const double sdot = block_sum(dot, red);
-  if (tid == 0) atomicAdd(&p.cg->pAp, sdot);
+  if constexpr (!MULTI) {
+    const double sdot = block_sum(dot, red);
+    if (tid == 0) atomicAdd(&p.cg->pAp, sdot);
+  }
 }
 
 // ---------------------------------------------------------------- update

@@ -549,6 +549,7 @@ struct dgc_mpnn_s {
   std::vector<float*> as;        // a_1 .. a_L  [S K W]
   float *y = nullptr, *dy = nullptr, *dh0 = nullptr, *dh1 = nullptr, *g = nullptr;
   float *sd = nullptr, *tm = nullptr, *st = nullptr;  // energy loss: S d, masked t, S t
+  float* sq = nullptr;           // its S applies' gradient fields, x then y
   int loss_kind = DGC_MPNN_LOSS_ENERGY;
   int linear = 0;                // DGC_MPNN_ACT_LINEAR: no ReLU, biases held at zero
   int post = 0;                  // DGC_MPNN_CORR_RESIDUAL: the network acts on r - S z0
@@ -622,7 +623,7 @@ int ensure_train(dgc_mpnn m, int S) {
   for (auto& p : m->hs) fr(p);
   for (auto& p : m->as) fr(p);
   fr(m->y); fr(m->dy); fr(m->dh0); fr(m->dh1); fr(m->g);
-  fr(m->sd); fr(m->tm); fr(m->st);
+  fr(m->sd); fr(m->tm); fr(m->st); fr(m->sq);
   const size_t nW = (size_t)S * m->h->K * dgk::kW, nY = (size_t)S * field_len(m);
   m->hs.assign(m->lay.L + 1, nullptr);
   m->as.assign(m->lay.L, nullptr);
@@ -636,6 +637,7 @@ int ensure_train(dgc_mpnn m, int S) {
   CKM(zalloc(&m->sd, nY));
   CKM(zalloc(&m->tm, nY));
   CKM(zalloc(&m->st, nY));
+  CKM(zalloc(&m->sq, 2 * nY));
   m->cap = S;
   // [0] loss, [1..S] target norms (L2 loss), [1+S .. 1+3S) per-sample d.Sd, t.St (energy loss)
   return ensure_scal(m, 1 + 3 * S);
@@ -808,7 +810,7 @@ extern "C" int dgc_mpnn_create(dgc_handle h, int layers, uint64_t seed, dgc_mpnn
 
 extern "C" int dgc_mpnn_destroy(dgc_mpnn m) {
   if (!m) return DGC_OK;
-  for (float* p : {m->w, m->grad, m->am, m->av, m->y, m->dy, m->dh0, m->dh1, m->g, m->sd, m->tm, m->st,
+  for (float* p : {m->w, m->grad, m->am, m->av, m->y, m->dy, m->dh0, m->dh1, m->g, m->sd, m->tm, m->st, m->sq,
                    m->px, m->ph0, m->ph1,
                    m->py, m->pt})
     cudaFree(p);
@@ -919,10 +921,11 @@ extern "C" int dgc_mpnn_train_step(dgc_mpnn m, const float* x, const float* t, i
     const int64_t f = (int64_t)K * npi;
     dgk::k_mask_diff<<<grid_for(m, n * npi, 256), 256, 0, s>>>(n * npi, npi, np, m->y, t, m->dy, m->tm);
     CKM(cudaGetLastError());
-    for (int j = 0; j < S; ++j) {
-      if (int rc = dgc::ipdg_spd_apply_f32(m->h, m->dy + j * f, m->sd + j * f, s)) return rc;
-      if (int rc = dgc::ipdg_spd_apply_f32(m->h, m->tm + j * f, m->st + j * f, s)) return rc;
-    }
+    // all samples' fields in one pair of launches: a field of 32768 cells alone fills
+    // little more than one wave, and its partly empty last one is a third of its time
+    // (a step of 8 samples: 1.89 -> 1.81 ms)
+    if (int rc = dgc::ipdg_spd_apply_f32_many(m->h, m->dy, m->sd, S, m->sq, s)) return rc;
+    if (int rc = dgc::ipdg_spd_apply_f32_many(m->h, m->tm, m->st, S, m->sq, s)) return rc;
     double* dots = m->scal + 1 + S;
     const int per = (int)std::max<int64_t>(1, std::min<int64_t>((f + 255) / 256, (4 * m->sm_count + S - 1) / S));
     dgk::k_energy_dots<<<dim3(per, S), 256, 0, s>>>(f, m->dy, m->sd, m->tm, m->st, dots);

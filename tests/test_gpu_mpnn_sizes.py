@@ -46,3 +46,32 @@ def test_forward_and_gradients(n, N, S, offset):
     y = net.forward(dev(x[:K]))
     assert rel(y.cpu().numpy(), mpnn_ref.forward(w, x[:K].astype(np.float64), nbr, K, npi, L)[0]) < 5e-6
     D.check()
+
+
+@pytest.mark.parametrize("n,N,S", [(1, 1, 2), (3, 4, 3), (9, 8, 2), (20, 3, 5), (40, 4, 7)])
+def test_energy_loss_over_many_fields(n, N, S):
+    """The S applies of all samples go through one pair of launches, tiles field after
+    field: fields smaller than a tile, partly filled tiles, more tiles than CTAs."""
+    m = meshes.jittered_square(n, 40 + n)
+    D = dg.Discretization(m, "laplace", N, dg.F64, tau=dg.TAU_SCALED, dirichlet=True)
+    L = 2
+    net = dg.MPNN(D, layers=L, seed=1)
+    K, Np, npi = D.K, D.Np, D.NpP
+    rng = np.random.default_rng(n)
+    w = (rng.standard_normal(net.num_params) * 0.15).astype(np.float32)
+    net.set_weights(w)
+    x = rng.standard_normal((S * K, npi)).astype(np.float32)
+    t = rng.standard_normal((S * K, npi)).astype(np.float32)
+    loss, grad = net.train_step(torch.from_numpy(x).cuda().reshape(-1), torch.from_numpy(t).cuda().reshape(-1),
+                                lr=0.0, want_grad=True)
+
+    def spd(v):  # the FP64 form on one native-layout field
+        return D.spd(torch.from_numpy(np.ascontiguousarray(v).reshape(-1)).cuda()).cpu().numpy().reshape(K, npi)
+
+    lr, gr = mpnn_ref.loss_and_grad(w, x.astype(np.float64), t.astype(np.float64), dg.host_mesh(m, N)[1], K, npi, Np, L,
+                                    spd=spd)
+    # random fields load all modes, so S d carries FP32's own relative error: sums of
+    # at most 3 Np + 9 (N + 1) = 216 products, 216 x 6e-8 at worst
+    assert abs(loss - lr) < 1.3e-5 * lr
+    assert rel(grad.cpu().numpy(), gr) < 3e-5
+    D.check()
