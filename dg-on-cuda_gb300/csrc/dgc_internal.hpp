@@ -99,6 +99,8 @@ struct BjFused {
 // z = Binv r after the step
 int ipdg_block_jacobi_step(dgc_handle_s* h, const BjFused& io, double* z, float* z32, cudaStream_t s);
 int ipdg_block_jacobi_correct(dgc_handle_s* h, const BjFused& io, double* z, cudaStream_t s);
+// per-element constants of the FP64 even / odd passes (laplace handles, else NULL)
+const double* ipdg_consts(const dgc_handle_s* h);
 // the SPD form's shift, and whether the boundary types are the handle's uniform ones
 double ipdg_shift(const dgc_handle_s* h);
 bool ipdg_uniform_bc(const dgc_handle_s* h);

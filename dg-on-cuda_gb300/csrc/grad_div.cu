@@ -14,7 +14,7 @@
 //
 // FP64: even / odd form on the tile layout of ipdg_eo.cuh (k_grad_eo, k_div_eo),
 // bound by the FP64 pipe: at K = 131072, N = 4 a gradient and a divergence take
-// 373 us together, 522 us node by node (that pipe 94.6 % busy).  FP32, FP64
+// 338 us together on laplace handles, 522 us node by node (that pipe 94.6 % busy).  FP32, FP64
 // operators without the reflection symmetry and inputs off a 16-byte boundary:
 //
 // Kernel: one CTA of 256 threads holds E = 256 / NpP elements; their fields are
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(256) k_grad_eo(const IpdgParams p, const GradD
       }
     }
   }
-  t.template constants<EO_WEAK>(ne);
+  t.constants(p, ne);
   if (!__syncthreads_and(mbar_wait(t.bar() + 1, 0, p.status))) return;
   const double* sU = t.field(0);
   if (fact) {
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(256) k_grad_eo(const IpdgParams p, const GradD
   }
   t.sum_diff(sU, ne);
   __syncthreads();
-  t.grad_rows(ne, k0, static_cast<double*>(p.qx), static_cast<double*>(p.qy));
+  t.template grad_rows<true>(ne, k0, static_cast<double*>(p.qx), static_cast<double*>(p.qy));
 }
 
 // divergence of (p.qx, p.qy) into p.out
@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(256) k_div_eo(const IpdgParams p, const GradDi
       }
     }
   }
-  t.template constants<EO_WEAK>(ne);
+  t.constants(p, ne);
   if (!__syncthreads_and(mbar_wait(t.bar() + 1, 0, p.status))) return;
   const double *sX = t.field(0), *sY = t.field(1);
   if (fact) {
@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(256) k_div_eo(const IpdgParams p, const GradDi
   double* ro = t.in() + e * 2 * Np;
   if (act) ro[r] = au;
   __syncthreads();
-  if (act) static_cast<double*>(p.out)[(size_t)(k0 + e) * NpP + r] = t.node(ro, r);
+  if (act) static_cast<double*>(p.out)[(size_t)(k0 + e) * NpP + r] = t.template node<true>(ro, r);
 }
 
 template <int N, bool DIV>
@@ -289,8 +289,9 @@ cudaError_t launch_eo(const IpdgParams& p, const GradDivBc& bc, int sm, cudaStre
     st = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemGrad);
   });
   if (st != cudaSuccess) return st;
-  // the passes' cost, without the mass rows
-  const EoCost w = DIV ? EoCost{C::kCostDiv.row - C::nE, C::kCostDiv.flux, C::kCostDiv.in, C::kCostDiv.cst} : C::kCostGrad;
+  // the passes' cost, without the mass rows and with the constants formed here
+  EoCost w = DIV ? EoCost{C::kCostDiv.row - C::nE, C::kCostDiv.flux, C::kCostDiv.in, 0} : C::kCostGrad;
+  if (!p.consts) w.cst = 8;
   const int ntiles = eo_pick_tiles(C::D, p.K, sm, C::TE, w);
   if (ntiles <= sm) return launch_stage(kern, ntiles, 256, C::kSmemGrad, s, p, bc);
   kern<<<ntiles, 256, C::kSmemGrad, s>>>(p, bc);
@@ -340,6 +341,7 @@ int grad_div(dgc_handle h, const void* u0, const void* u1, const double* g0, con
     p.nbr = reinterpret_cast<const int4*>(h->d_nbr);
     p.mats_eo = h->d_eo64[0];
     p.tab_eo = h->d_eo_tab[0];
+    p.consts = ipdg_consts(h);
     p.status = h->d_status;
     p.u = u0;
     p.qx = DIV ? const_cast<void*>(u0) : out0;

@@ -348,6 +348,14 @@ __global__ void k_cg_start(CgScalars* cg, double tol2, int maxit) {
   if (cg->rr[0] == 0.0) cg->done = 1;
 }
 
+// the FP64 passes' per-element constants (ipdg_eo.cuh), out: [2 forms][K][16], strong first
+__global__ void k_eo_consts(int K, const double* __restrict__ geom, const double* __restrict__ tau,
+                            double* __restrict__ out) {
+  const int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t e = x >> 4;
+  if (e < K) eo_const((int)(x & 7), x & 8, geom + e * 16, tau + e * 4, out + (x & 8 ? (size_t)K * 16 : 0) + e * 16);
+}
+
 }  // namespace dgk
 
 namespace dgc {
@@ -371,6 +379,7 @@ struct IpdgState {
   void* qd = nullptr;          // lifted Dirichlet data q_d, 2 x K x NpP in the handle's precision
   void* mass64 = nullptr;      // padded M in FP64 / FP32
   void* mass32 = nullptr;
+  double* consts = nullptr;    // [2][K][16] per-element constants of the FP64 passes (ipdg_eo.cuh)
   double* dense64 = nullptr;   // row-major Dr | Ds | L | M (FP64) for the block set-up
   // workspace: FP64 and FP32 vector sets
   double* w64[10] = {};
@@ -420,6 +429,7 @@ dgk::IpdgParams base(const dgc_handle_s* h) {
   p.mass = sizeof(R) == 8 ? h->ipdg->mass64 : h->ipdg->mass32;
   p.mats_eo = sizeof(R) == 8 && h->eo_ok[1] ? h->d_eo64[1] : nullptr;
   p.tab_eo = h->d_eo_tab[1];
+  p.consts = h->ipdg->consts;
   p.binv = sizeof(R) == 8 ? (const void*)h->ipdg->binv64 : (const void*)h->ipdg->binv32;
   p.mats_blk = h->ipdg->ops_blk32;
   p.mass_blk = h->ipdg->mass_blk32;
@@ -765,6 +775,9 @@ int ipdg_init(dgc_handle_s* h) {
     CKI(cudaMemcpy(h->d_tau, ones.data(), ones.size() * 8, cudaMemcpyHostToDevice));
     CKI(cudaMemcpy(h->d_tau32, ones32.data(), ones32.size() * 4, cudaMemcpyHostToDevice));
   }
+  CKI(cudaMalloc(&st->consts, (size_t)h->K * 32 * 8));
+  dgk::k_eo_consts<<<(unsigned)(((int64_t)h->K * 16 + 255) / 256), 256>>>(h->K, h->d_kgeom64, h->d_tau, st->consts);
+  CKI(cudaGetLastError());
   CKI(cudaMalloc(&st->mass64, (size_t)st->bstr * 8));
   CKI(cudaMalloc(&st->mass32, (size_t)st->bstr * 4));
   CKI(cudaMalloc(&st->dense64, ((size_t)3 * Np * Np + (size_t)Np * NF) * 8));
@@ -835,6 +848,7 @@ void ipdg_free(dgc_handle_s* h) {
   cudaFree(st->mass64);
   cudaFree(st->mass32);
   cudaFree(st->dense64);
+  cudaFree(st->consts);
   for (int i = 0; i < W_COUNT; ++i) {
     cudaFree(st->w64[i]);
     cudaFree(st->w32[i]);
@@ -846,6 +860,8 @@ void ipdg_free(dgc_handle_s* h) {
   delete st;
   h->ipdg = nullptr;
 }
+
+const double* ipdg_consts(const dgc_handle_s* h) { return h->ipdg ? h->ipdg->consts : nullptr; }
 
 double ipdg_shift(const dgc_handle_s* h) { return h->ipdg ? h->ipdg->shift : 0.0; }
 

@@ -60,6 +60,7 @@ struct IpdgParams {
   const void* mass;     // M (Np x Np, R), symmetric
   const void* mats_eo;  // FP64: strong-form operators and M in the even / odd basis (ipdg_eo.cuh), NULL: not symmetric
   const uint8_t* tab_eo;  // their pair tables
+  const double* consts; // [2][K][16] their per-element constants, NULL: formed from the geometry
   // grad pass
   const void* u;        // input u (GRAD_PLAIN) or z (GRAD_PCG)
   void* p;              // GRAD_PCG: new search direction p (written); update: p (read)

@@ -10,7 +10,7 @@
 //     element's constant geometry: 2 Np^2 instead of 6 Np^2 for both passes, LIFT
 //     and M half of theirs;
 //   * -1/J (the SPD form: J (1/J) = 1), faceJ, normals and penalties are
-//     multiplied into per-element constants.
+//     multiplied into per-element constants, once per laplace handle.
 // One tile per CTA (eo_pick_tiles); set-up data are fetched
 // before the wait for the previous launch, exterior traces while the tile's own
 // fields arrive.
@@ -33,22 +33,41 @@ struct IpdgEo {
   static constexpr int CSTR = 16;
   static constexpr uint32_t kOpsG = (D.kK() + D.kL()) * 8, kOpsD = kOpsG + D.kM() * 8, kTab = D.tabBytes();
   static constexpr uint32_t kF = TE * NpP * 8;  // one field
-  static constexpr uint32_t oBar = 0, oTab = 32, oGeom = oTab + kTab, oNbr = oGeom + TE * 16 * 8, oTau = oNbr + TE * 16,
-                            oC = oTau + TE * 4 * 8, oFld = oC + TE * CSTR * 8, oIn = oFld + 3 * kF,
+  static constexpr uint32_t oBar = 0, oTab = 32, oGeom = oTab + kTab, oNbr = oGeom + TE * 16 * 8, oC = oNbr + TE * 16,
+                            oFld = oC + TE * CSTR * 8, oIn = oFld + 3 * kF,
                             oF = oIn + TE * 2 * Np * 8, oRed = (oF + TE * FSTR * 8 + 15) / 16 * 16, oOps = oRed + 16 * 8;
   static constexpr uint32_t kSmemGrad = oOps + kOpsG, kSmemDiv = oOps + kOpsD;
   static_assert(TE * fE <= 256, "one face-node pair per thread");
   static_assert(oGeom % 16 == 0 && oFld % 16 == 0 && kF % 16 == 0 && oRed % 16 == 0 && kOpsG % 16 == 0, "alignment");
   // FP64 instructions per item (eo_pick_tiles)
-  static constexpr EoCost kCostGrad{Np + 2 * fE + 6, 12, 2, 8}, kCostDiv{Np + fE + nE + 5, 14, 8, 8};
+  static constexpr EoCost kCostGrad{Np + 2 * fE + 6, 12, 2, 0}, kCostDiv{Np + fE + nE + 5, 14, 8, 0};
 };
 
-// volume + lift / J as the strong form has them (1, -1/J), the strong form times
-// -J, or the weak form's signs (-1, 1/J)
-enum IpdgEoForm : int { EO_STRONG = 0, EO_SPD = 1, EO_WEAK = 2 };
+// Per-element constants, in the strong form's signs or with the SPD form's rows
+// times -J: (rx +- sx, ry +- sy) s, then per face h nx, h ny and 2 tau h with
+// h = faceJ / 2 times -1/J (SPD: J (1/J) = 1), and -J.  The weak form is minus the strong one.
+// Laplace handles keep both forms (k_eo_consts), 128 bytes per element and form, read
+// in place of geometry and penalties: forming them in every launch was a tenth of a
+// pass's FP64 instructions (SPD apply, K = 65522, N = 5: 309 -> 294 us; gradient and
+// divergence, K = 131072, N = 4: 373 -> 338 us).
+enum IpdgEoConst : int { IC_P1 = 0, IC_P2 = 1, IC_Q1 = 2, IC_Q2 = 3, IC_F = 4, IC_MJ = 13 };
 
-// per-element constants: (rx +- sx, ry +- sy) s, then per face (cx, cy, ct)
-enum IpdgEoConst : int { IC_P1 = 0, IC_P2 = 1, IC_Q1 = 2, IC_Q2 = 3, IC_F = 4 };
+// value group v (0 .. 7: the volume factors, the faces, -J) of an element's constants
+__device__ __forceinline__ void eo_const(int v, bool spd, const double* g, const double* tau, double* c) {
+  const double sv = spd ? g[14] : 1.0, sf = spd ? 1.0 : g[4];  // g[14] = -J, g[4] = -1/J
+  if (v < 2) c[IC_P1 + v] = sv * (v ? g[0] - g[2] : g[0] + g[2]);
+  else if (v < 4) c[IC_Q1 + v - 2] = sv * (v == 3 ? g[1] - g[3] : g[1] + g[3]);
+  else if (v < 7) {
+    const int f = v - 4;
+    const double h = 0.5 * g[5 + f] * sf;
+    c[IC_F + 3 * f] = h * g[8 + f];
+    c[IC_F + 3 * f + 1] = h * g[11 + f];
+    c[IC_F + 3 * f + 2] = tau ? 2.0 * tau[f] * h : 0.0;
+  } else {
+    c[IC_MJ] = g[14];
+    c[IC_MJ + 1] = c[IC_MJ + 2] = 0.0;
+  }
+}
 
 // views of a CTA's shared memory, and the parts both passes share
 template <int N>
@@ -61,7 +80,6 @@ struct IpdgEoTile {
   __device__ const uint8_t* inverse() const { return smem + C::oTab + 2 * C::nE + 2 * C::fE; }
   __device__ const double* geom() const { return reinterpret_cast<const double*>(smem + C::oGeom); }
   __device__ const int4* nbr() const { return reinterpret_cast<const int4*>(smem + C::oNbr); }
-  __device__ const double* tau() const { return reinterpret_cast<const double*>(smem + C::oTau); }
   __device__ double* consts() const { return reinterpret_cast<double*>(smem + C::oC); }
   __device__ double* field(int i) const { return reinterpret_cast<double*>(smem + C::oFld + i * C::kF); }
   __device__ double* in() const { return reinterpret_cast<double*>(smem + C::oIn); }
@@ -72,40 +90,27 @@ struct IpdgEoTile {
   __device__ const double* M() const { return L() + C::D.kL(); }
 
   // set-up data of the elements k0 .. k0 + ne - 1; false if a wait expired
-  __device__ bool setup(const IpdgParams& p, int k0, int ne, uint32_t ops, bool tau) const {
+  __device__ bool setup(const IpdgParams& p, int k0, int ne, uint32_t ops, bool spd) const {
     if (threadIdx.x == 0) {
       mbar_init(bar(), 1);
       mbar_init(bar() + 1, 1);
       fence_barrier_init();
-      mbar_arrive_expect_tx(bar(), ops + C::kTab + ne * (16 * 8 + 16 + (tau ? 32 : 0)));
+      mbar_arrive_expect_tx(bar(), ops + C::kTab + ne * (16 * 8 + 16));
       bulk_g2s(smem + C::oOps, p.mats_eo, ops, bar());
       bulk_g2s(smem + C::oTab, p.tab_eo, C::kTab, bar());
-      bulk_g2s(smem + C::oGeom, static_cast<const double*>(p.geom) + (size_t)k0 * 16, ne * 16 * 8, bar());
+      // the constants, or the geometry they are formed from
+      if (p.consts) bulk_g2s(smem + C::oC, p.consts + ((size_t)(spd ? p.K : 0) + k0) * 16, ne * 16 * 8, bar());
+      else bulk_g2s(smem + C::oGeom, static_cast<const double*>(p.geom) + (size_t)k0 * 16, ne * 16 * 8, bar());
       bulk_g2s(smem + C::oNbr, p.nbr + k0, ne * 16, bar());
-      if (tau) bulk_g2s(smem + C::oTau, static_cast<const double*>(p.tau) + (size_t)k0 * 4, ne * 32, bar());
     }
     __syncthreads();
     return __syncthreads_and(mbar_wait(bar(), 0, p.status));
   }
-  // constants: volume factors times sv, face factors h n and 2 tau h, h = faceJ / 2 times sf
-  template <IpdgEoForm FORM, bool TAU = false>
-  __device__ void constants(int ne) const {
-    for (int x = 255 - (int)threadIdx.x; x < ne * 8; x += 256) {
-      const int e = x >> 3, v = x & 7;
-      const double* g = geom() + e * 16;
-      double* c = consts() + e * C::CSTR;
-      const double sv = FORM == EO_SPD ? g[14] : (FORM == EO_WEAK ? -1.0 : 1.0);      // g[14] = -J
-      const double sf = FORM == EO_SPD ? 1.0 : (FORM == EO_WEAK ? -g[4] : g[4]);      // g[4] = -1/J
-      if (v < 2) c[IC_P1 + v] = sv * (v ? g[0] - g[2] : g[0] + g[2]);
-      else if (v < 4) c[IC_Q1 + v - 2] = sv * (v == 3 ? g[1] - g[3] : g[1] + g[3]);
-      else if (v < 7) {
-        const int f = v - 4;
-        const double h = 0.5 * g[5 + f] * sf;
-        c[IC_F + 3 * f] = h * g[8 + f];
-        c[IC_F + 3 * f + 1] = h * g[11 + f];
-        if (TAU) c[IC_F + 3 * f + 2] = 2.0 * tau()[e * 4 + f] * h;
-      }
-    }
+  // the constants of handles that keep none (gradient and divergence of advection handles)
+  __device__ void constants(const IpdgParams& p, int ne) const {
+    if (p.consts) return;
+    for (int x = 255 - (int)threadIdx.x; x < ne * 8; x += 256)
+      eo_const(x & 7, false, geom() + (x >> 3) * 16, nullptr, consts() + (x >> 3) * C::CSTR);
   }
 
   // inputs of the gradient rows: sums and differences of the field u
@@ -149,15 +154,18 @@ struct IpdgEoTile {
     }
   }
   // node r's value from the sums and differences ro[Np] of its element's rows
+  // (NEG: minus it)
+  template <bool NEG = false>
   __device__ double node(const double* ro, int r) const {
     const int inv = inverse()[r], c = inv & 127;
-    const double v = ro[c];
+    const double v = NEG ? -ro[c] : ro[c];
     if (c >= C::nO) return v;
     const double o = ro[C::nE + c];
-    return inv & 128 ? v - o : v + o;
+    return ((inv & 128) != 0) != NEG ? v - o : v + o;
   }
   // gradient rows of the tile from sum_diff's inputs and the x | y flux sums and
   // differences, then both components by node
+  template <bool NEG = false>
   __device__ void grad_rows(int ne, int k0, double* ox, double* oy) const {
     constexpr int Np = C::Np, nE = C::nE, nO = C::nO, fE = C::fE;
     const int e = (int)threadIdx.x / Np, r = (int)threadIdx.x - e * Np;
@@ -196,8 +204,8 @@ struct IpdgEoTile {
     __syncthreads();
     if (act) {
       const size_t o = (size_t)(k0 + e) * C::NpP + r;
-      ox[o] = node(ro, r);
-      oy[o] = node(ro + Np, r);
+      ox[o] = node<NEG>(ro, r);
+      oy[o] = node<NEG>(ro + Np, r);
     }
   }
   // divergence row r of element e from combine's inputs and the flux sums and differences
@@ -275,7 +283,6 @@ __global__ void __launch_bounds__(256) ipdg_grad_eo_kernel(const IpdgParams p) {
       }
     }
   }
-  t.template constants<EO_STRONG>(ne);
   if (!__syncthreads_and(mbar_wait(t.bar() + 1, 0, p.status))) return;
   double* sU = t.field(0);
   const double beta = s_beta;
@@ -326,7 +333,7 @@ __global__ void __launch_bounds__(256) ipdg_div_eo_kernel(const IpdgParams p) {
   const int tid = threadIdx.x;
   const TileCut tiles(p.K, gridDim.x);
   const int k0 = tiles.start(blockIdx.x), ne = tiles.size(blockIdx.x);
-  if (!t.setup(p, k0, ne, SPD ? C::kOpsD : C::kOpsG, true)) return;
+  if (!t.setup(p, k0, ne, SPD ? C::kOpsD : C::kOpsG, SPD)) return;
   const double* qx = static_cast<const double*>(p.qx);
   const double* qy = static_cast<const double*>(p.qy);
   const double* uj = static_cast<const double*>(p.du_src);
@@ -371,7 +378,6 @@ __global__ void __launch_bounds__(256) ipdg_div_eo_kernel(const IpdgParams p) {
   const size_t o = (size_t)(k0 + e) * NpP + r;
   double bv = 0.0;
   if (MODE == DIV_RESID && act) bv = static_cast<const double*>(p.b)[o];
-  t.template constants<SPD ? EO_SPD : EO_STRONG, true>(ne);
   if (!__syncthreads_and(mbar_wait(t.bar() + 1, 0, p.status))) return;
   const double *sX = t.field(0), *sY = t.field(1), *sU = t.field(2);
   if (fact) {
@@ -405,7 +411,7 @@ __global__ void __launch_bounds__(256) ipdg_div_eo_kernel(const IpdgParams p) {
       const int c = sum ? r : r - nE;
       const double ua = sU[e * NpP + t.nodes()[2 * c]], ub = sU[e * NpP + t.nodes()[2 * c + 1]];
       const double uh = sum ? (c < nO ? 0.5 * (ua + ub) : ua) : 0.5 * (ua - ub);
-      au = fma(-p.shift * t.geom()[e * 16 + 14], uh, au);
+      au = fma(-p.shift * t.consts()[e * C::CSTR + IC_MJ], uh, au);
     }
   }
   __syncthreads();

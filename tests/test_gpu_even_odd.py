@@ -82,6 +82,20 @@ def test_grad_div(N, n):
     D.check()
 
 
+@pytest.mark.parametrize("N,n", [(1, 9), (2, 1), (4, 23), (5, 40), (8, 7)])
+def test_grad_div_without_kept_constants(N, n):
+    """Advection handles keep no per-element constants: the same ones formed in the
+    kernel, so the same bits as on a laplace handle."""
+    m = dg.meshes.jittered_square(n, seed=3 + n)
+    A, B = dg.Discretization(m, "laplace", N, dg.F64), dg.Discretization(m, "advection", N, dg.F64, ax=1.0, ay=0.5)
+    u = torch.randn(A.K * A.NpP, dtype=torch.float64, device="cuda")
+    gx, gy = A.grad(u)
+    hx, hy = B.grad(u)
+    valid = torch.arange(A.K * A.NpP, device="cuda") % A.NpP < A.Np
+    for a, b in ((gx, hx), (gy, hy), (A.div(gx, gy), B.div(hx, hy))):
+        assert torch.equal(a.reshape(-1)[valid], b.reshape(-1)[valid])
+
+
 @pytest.mark.parametrize("n", [1, 4, 9])
 @pytest.mark.parametrize("N", range(1, 9))
 def test_fp32_stage(N, n):
