@@ -309,26 +309,44 @@ __global__ void k_coarse_gemv(int n, const double* __restrict__ A, const double*
 
 // the same product with the FP32 copy of A_c^-1 and of x, FP32 sums (inside the
 // FP32 coarse cycle): half the bytes and no FP64 arithmetic
-// (rows of A and x padded with zeros to lda, a multiple of 4: 16-byte loads)
-__global__ void k_coarse_gemv32(int n, int lda, const float* __restrict__ A, const float* __restrict__ x,
-                                double* __restrict__ y) {
+// (rows of A and x padded with zeros to lda, a multiple of 4: 16-byte loads).
+// Bound by the latency of a warp's row, which leaves L2 between two cycles: eight
+// loads per lane are in flight, the first ones before x has reached shared memory
+// (4057 rows: 16 us; x read from L1 beside A, 22 us)
+constexpr int kGemvX = 1024;  // float4 of x per pass
+__global__ void __launch_bounds__(256) k_coarse_gemv32(int n, int lda, const float* __restrict__ A,
+                                                       const float* __restrict__ x, double* __restrict__ y) {
+  __shared__ float4 sx[kGemvX];
   const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (row >= n) return;
-  const float4* a = reinterpret_cast<const float4*>(A + (size_t)row * lda);
+  const bool live = row < n;
+  const float4* a = reinterpret_cast<const float4*>(A + (size_t)(live ? row : 0) * lda);
   const float4* x4 = reinterpret_cast<const float4*>(x);
   float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-  for (int c = lane; c < lda / 4; c += 32) {
-    const float4 aa = __ldg(a + c), xx = __ldg(x4 + c);
-    v.x = fmaf(aa.x, xx.x, v.x);
-    v.y = fmaf(aa.y, xx.y, v.y);
-    v.z = fmaf(aa.z, xx.z, v.z);
-    v.w = fmaf(aa.w, xx.w, v.w);
+  for (int b = 0; b < lda / 4; b += kGemvX) {
+    const int m = min(kGemvX, lda / 4 - b);
+    if (b) __syncthreads();
+    for (int c = threadIdx.x; c < m; c += 256) sx[c] = x4[b + c];
+    for (int c0 = lane; c0 < kGemvX; c0 += 256) {
+      float4 aa[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (c0 + 32 * u < m) aa[u] = __ldg(a + b + c0 + 32 * u);
+      if (c0 == lane) __syncthreads();
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (c0 + 32 * u < m) {
+          const float4 xx = sx[c0 + 32 * u];
+          v.x = fmaf(aa[u].x, xx.x, v.x);
+          v.y = fmaf(aa[u].y, xx.y, v.y);
+          v.z = fmaf(aa[u].z, xx.z, v.z);
+          v.w = fmaf(aa[u].w, xx.w, v.w);
+        }
+    }
   }
   float s = (v.x + v.y) + (v.z + v.w);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) y[row] = (double)s;
+  if (live && lane == 0) y[row] = (double)s;
 }
 
 // z32[k][j] = xc[agg[k]] on the valid nodes, 0 on the others: the FP32 operator

@@ -29,3 +29,19 @@ def test_two_level_modes_solve_every_order(N, n, cells, dirichlet):
         assert (torch.linalg.norm(u - ref) / torch.linalg.norm(ref)).item() < 1e-6
         assert st["final_relres"] <= 1e-11
     D.check()
+
+
+@pytest.mark.parametrize("n,cells", [(80, 2), (33, 1)])
+def test_coarse_product_across_passes(n, cells):
+    """More aggregates than one pass of the FP32 coarse product holds of its vector
+    (4096), and fewer: against the FP64 product."""
+    D = dg.Discretization(meshes.jittered_square(n, 3), "laplace", 1, dg.F64, tau=dg.TAU_SCALED, dirichlet=True)
+    D.coarse_build(cells)
+    na = D.coarse_info()[1]
+    assert na > 4096 if n == 80 else 0 < na < 4096
+    r = D.upload(np.random.default_rng(n).standard_normal(D.K * D.Np))
+    a, b = D.coarse_apply(r, precision=dg.F32), D.coarse_apply(r)
+    # FP32 rounding (6e-8) of a random r, whose modes the inverse scales like the
+    # result's own, over sums of a few hundred roundings
+    assert (torch.linalg.norm(a - b) / torch.linalg.norm(b)).item() < 1e-4
+    D.check()
