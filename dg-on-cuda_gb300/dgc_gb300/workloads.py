@@ -13,15 +13,15 @@ skip count can be read off.
 
     stage_x2     dg_rhs_x2_kernel<6, TE>: Maxwell TE, jittered 128x128 (K = 32768),
                  N = 6, compensated FP32 state, one LSERK4 stage per launch
-    stage_fp64   dg_rhs_kernel<double, 6, TE>: the same workload in FP64
+    stage_fp64   dg_rhs_eo_kernel<6, TE>: the same workload in FP64
     stage_fp32   the autotuned FP32 stage kernel of the same workload
     batch        dg_batch_kernel: 24 seeded instances (advection / Maxwell TE / TM,
                  n in [8, 160], N in 2..8), each on its faster batch tile code
     mpnn_fwd     k_layer_tc: the 4-layer, width-64 network over a jittered
                  128x128 mesh (K = 32768), N = 4
-    bj_apply     k_bj_apply<float>: block-Jacobi application inside the two-level
+    bj_apply     k_bj_apply_pk: block-Jacobi application inside the two-level
                  mixed PCG, jittered 256x256 mesh (K = 131072), N = 4
-    grad_div     k_grad_div: weak-form gradient and divergence, K = 131072, N = 4, FP64
+    grad_div     k_grad_eo, k_div_eo: weak-form gradient and divergence, K = 131072, N = 4, FP64
 """
 from __future__ import annotations
 
@@ -120,7 +120,7 @@ def bj_apply(reps: int):
     D.block_jacobi()
     D.coarse_build(32)
     b = D.mass(D.upload((2 * np.pi ** 2 * np.sin(np.pi * x) * np.sin(np.pi * y)).reshape(-1)))
-    print(f"kernel: k_bj_apply (two-level mixed PCG iterations), solves 1 + {reps}", flush=True)
+    print(f"kernel: k_bj_apply_pk (two-level mixed PCG iterations), solves 1 + {reps}", flush=True)
     D.pcg(b, mode=dg.SOLVE_TWO_LEVEL_MIXED, rtol=1e-10, maxit=40, check=False)
     _sync()
     for _ in range(reps):
@@ -136,7 +136,7 @@ def grad_div(reps: int):
                           dirichlet=True)
     x, y = D.node_xy()
     u = D.upload((np.sin(np.pi * x) * np.cos(np.pi * y)).reshape(-1))
-    print(f"kernel: k_grad_div, warm-up launches 4, measured {2 * reps}", flush=True)
+    print(f"kernel: k_grad_eo and k_div_eo, warm-up launches 4, measured {2 * reps}", flush=True)
     for _ in range(2):
         gx, gy = D.grad(u)
         D.div(gx, gy)
