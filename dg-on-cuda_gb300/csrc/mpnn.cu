@@ -923,7 +923,7 @@ extern "C" int dgc_mpnn_train_step(dgc_mpnn m, const float* x, const float* t, i
     CKM(cudaGetLastError());
     // all samples' fields in one pair of launches: a field of 32768 cells alone fills
     // little more than one wave, and its partly empty last one is a third of its time
-    // (a step of 8 samples: 1.89 -> 1.81 ms)
+    // (a step of 8 samples: 1.89 -> 1.77 ms)
     if (int rc = dgc::ipdg_spd_apply_f32_many(m->h, m->dy, m->sd, S, m->sq, s)) return rc;
     if (int rc = dgc::ipdg_spd_apply_f32_many(m->h, m->tm, m->st, S, m->sq, s)) return rc;
     double* dots = m->scal + 1 + S;
