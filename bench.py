@@ -167,7 +167,8 @@ class ClockSampler:
 
 
 # committed ncu summaries of the stage-kernel variants on this workload
-PROFILES = {5: "dg_rhs_blk_maxwell_te_n6_fp32.md", 9: "dg_rhs_tcp_maxwell_te_n6_fp32.md",
+PROFILES = {5: "dg_rhs_blk_maxwell_te_n6_fp32.md", 6: "dg_rhs_sym_maxwell_te_n6_fp32.md",
+            9: "dg_rhs_tcp_maxwell_te_n6_fp32.md",
             "x2": "dg_rhs_x2_maxwell_te_n6_fp32c.md"}
 
 
