@@ -61,13 +61,14 @@ struct BlkConfig {
   static constexpr uint32_t oMats = 32;
   static constexpr uint32_t oBuf = oMats + kMat;
   static constexpr uint32_t oFlux = oBuf + 2 * kBuf;
-  // advection: list of a tile's inflow boundary nodes (count, indices, values).
-  // Their values (FP64 exp or sin) are evaluated by consecutive threads: the nodes
-  // of a boundary row lie in a few lanes of every warp, and the FP64 pipe pays per
-  // warp.  Nodes past the list's end are evaluated where they are used.
+  // advection: list of a tile's inflow boundary nodes (count, then each one's
+  // 3 item + face).  Their values (FP64 exp or sin) are evaluated by consecutive
+  // threads: the nodes of a boundary row lie in a few lanes of every warp, and the
+  // FP64 pipe pays per warp.  Nodes past the list's end are evaluated where found.
   static constexpr int kBnd = P == PHYS_ADV ? 256 : 0;
   static constexpr uint32_t oBnd = oFlux + TE * Nf * FSTR * 4;
-  static constexpr uint32_t kSmem = oBnd + kBnd * 8 + (P == PHYS_ADV ? 16 : 0);
+  static constexpr uint32_t kSmem = oBnd + kBnd * 2 + (P == PHYS_ADV ? 16 : 0);
+  static_assert(3 * TE * O::Nfp <= 65536, "16-bit list entries");
   static_assert(NpP % 4 == 0 && kMat % 16 == 0, "16-byte operator rows");
 };
 
@@ -102,8 +103,7 @@ __device__ __forceinline__ bool blk_tiles(const RhsParams& p, unsigned char* sme
   const bool aux_tile = C::kAuxTile && p.mode == MODE_LSERK;
   const TileCut tiles(p.K, ntiles);
   int* bcount = reinterpret_cast<int*>(smem + C::oBnd);
-  int* bnode = bcount + 4;
-  float* bval = reinterpret_cast<float*>(bnode + C::kBnd);
+  uint16_t* blist = reinterpret_cast<uint16_t*>(bcount + 4);
 
   const int tid = threadIdx.x;
   // element slot and 4-node group of this thread
@@ -266,9 +266,15 @@ __device__ __forceinline__ bool blk_tiles(const RhsParams& p, unsigned char* sme
     // deep (it waits for this grid before its reads)
     if (tile + tstep >= tend) grid_dep_launch();
 
-    // ---- inflow boundary nodes (advection): listed, then evaluated; a flux entry
-    //      holds its node's place in the list until the flux replaces it
+    // ---- exterior values of the boundary nodes (advection), each in its node's
+    //      flux entry until the flux replaces it: 0 where the wind blows out (it
+    //      does not enter the flux), listed and then evaluated where it blows in.
+    //      Whether it does is asked here only: the face phase takes the value.
     if constexpr (P == PHYS_ADV) {
+      auto exact = [&](int nb, int d) {
+        const double* xy = p.bxy + ((size_t)(-1 - nb) * Nfp + d) * 2;
+        return (float)adv_exact(p, tnow, xy[0], xy[1]);
+      };
 #pragma unroll
       for (int s = 0; s < C::kFItems; ++s) {
         const int x = tid + s * NT;
@@ -278,17 +284,23 @@ __device__ __forceinline__ bool blk_tiles(const RhsParams& p, unsigned char* sme
 #pragma unroll
         for (int f = 0; f < 3; ++f) {
           const int nb = f == 0 ? nb4.x : (f == 1 ? nb4.y : nb4.z);
-          if (nb < 0 && !(cax * sG[e * 16 + 8 + f] + cay * sG[e * 16 + 11 + f] >= 0.0f)) {
+          if (nb >= 0) continue;
+          float v = 0.0f;
+          if (!(cax * sG[e * 16 + 8 + f] + cay * sG[e * 16 + 11 + f] >= 0.0f)) {
             const int at = atomicAdd(bcount, 1);
-            if (at < C::kBnd) bnode[at] = (-1 - nb) * Nfp + d;
-            sF[e * FSTR + f * Nfp + d] = __int_as_float(at);
+            if (at < C::kBnd) blist[at] = (uint16_t)(3 * x + f);
+            else v = exact(nb, d);
           }
+          sF[e * FSTR + f * Nfp + d] = v;
         }
       }
       __syncthreads();
       const int nlist = min(*bcount, C::kBnd);
-      for (int x = tid; x < nlist; x += NT)
-        bval[x] = (float)adv_exact(p, tnow, p.bxy[(size_t)bnode[x] * 2], p.bxy[(size_t)bnode[x] * 2 + 1]);
+      for (int q = tid; q < nlist; q += NT) {
+        const int x = blist[q] / 3, f = blist[q] - 3 * x, e = x / Nfp, d = x - e * Nfp;
+        const int4 nb4 = sN[e];
+        sF[e * FSTR + f * Nfp + d] = exact(f == 0 ? nb4.x : (f == 1 ? nb4.y : nb4.z), d);
+      }
       if (nlist > 0) __syncthreads();
     }
 
@@ -319,16 +331,7 @@ __device__ __forceinline__ bool blk_tiles(const RhsParams& p, unsigned char* sme
             for (int c = 0; c < NF; ++c) bv[f][c] = __ldg(qb + c * NpP);
           }
         } else if (P == PHYS_ADV) {
-          bv[f][0] = 0.0f;  // enters only where the wind blows in
-          if (!(cax * sG[e * 16 + 8 + f] + cay * sG[e * 16 + 11 + f] >= 0.0f)) {
-            const int at = __float_as_int(sF[e * FSTR + f * Nfp + d]);
-            if (at < C::kBnd) {
-              bv[f][0] = bval[at];
-            } else {
-              const double* xy = p.bxy + ((size_t)(-1 - nb) * Nfp + d) * 2;
-              bv[f][0] = (float)adv_exact(p, tnow, xy[0], xy[1]);
-            }
-          }
+          bv[f][0] = sF[e * FSTR + f * Nfp + d];
         } else if (P == PHYS_TM) {  // PEC: H+ = H-, Ez+ = -Ez-
           bv[f][0] = av[f][0]; bv[f][1] = av[f][1]; bv[f][2] = -av[f][2];
         } else {                    // PEC: E+ = -E-, Hz+ = Hz-
