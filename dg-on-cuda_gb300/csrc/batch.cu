@@ -65,8 +65,8 @@ template <int N, int P>
 __device__ __noinline__ bool batch_item_blk(const RhsParams& p, unsigned char* smem, uint32_t* ph, int tile0,
                                             int ntile) {
   uint32_t loc[3] = {ph[0], ph[1], ph[2]};
-  const bool ok = blk_tiles<N, P, 1, 0>(p, smem, loc, tile0, 1, tile0 + ntile,
-                                         (p.K + BlkConfig<N, P, 1, 0>::TE - 1) / BlkConfig<N, P, 1, 0>::TE);
+  const bool ok = blk_tiles<N, P, 1, 0, false>(p, smem, loc, tile0, 1, tile0 + ntile,
+                                               TileRun{p.K, BlkConfig<N, P, 1, 0>::TE});
   ph[0] = loc[0];
   ph[1] = loc[1];
   ph[2] = loc[2];

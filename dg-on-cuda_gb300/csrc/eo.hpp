@@ -89,6 +89,13 @@ struct TileCut {
   DGC_HD int size(int i) const { return len + (i < rem ? 1 : 0); }
 };
 
+// K elements cut into tiles of len elements, the last one shorter
+struct TileRun {
+  int K, len;
+  DGC_HD int start(int i) const { return i * len; }
+  DGC_HD int size(int i) const { return K - i * len < len ? K - i * len : len; }
+};
+
 // Tiles of the register-blocked kernels (FP32 and compensated stages, FP32 CG), cut
 // evenly (TileCut): as many as full tiles make, at least one per SM.  On meshes with
 // fewer full tiles than SMs a launch is latency (FP32 stage, Maxwell TE, K = 128,

@@ -275,17 +275,17 @@ cudaError_t rhs_sym(const RhsParams* p, cudaStream_t s, LaunchInfo* info) {
   return launch_stage(dg_rhs_sym_kernel<N, P>, (p->K + C::TE - 1) / C::TE, C::kThreads, C::kSmem, s, *p);
 }
 
-template <int N, int P, int EPT, int MAP>
+template <int N, int P, int EPT, int MAP, bool LIST = true>
 cudaError_t rhs_blk(const RhsParams* p, int sm_count, cudaStream_t s, LaunchInfo* info) {
   using C = BlkConfig<N, P, EPT, MAP>;
+  auto kern = dg_rhs_blk_kernel<N, P, EPT, MAP, LIST>;
   static std::once_flag once;
   static cudaError_t st = cudaSuccess;
   static int bps = 0;
-  std::call_once(once, [] {
-    st = cudaFuncSetAttribute(dg_rhs_blk_kernel<N, P, EPT, MAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
+  std::call_once(once, [&] {
+    st = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
     if (st == cudaSuccess)
-      st = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, dg_rhs_blk_kernel<N, P, EPT, MAP>, C::kThreads,
-                                                         C::kSmem);
+      st = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, C::kThreads, C::kSmem);
   });
   if (st != cudaSuccess) return st;
   if (info) {
@@ -299,7 +299,13 @@ cudaError_t rhs_blk(const RhsParams* p, int sm_count, cudaStream_t s, LaunchInfo
   RhsParams q = *p;
   q.ntiles = blk_tiles_for(p->K, sm_count, C::TE);
   const int grid = std::min(q.ntiles, sm_count * (bps > 0 ? bps : 1));
-  return launch_stage(dg_rhs_blk_kernel<N, P, EPT, MAP>, grid, C::kThreads, C::kSmem, s, q);
+  // the inflow list at orders 7, 8 only where every CTA has one tile (us per step,
+  // list / no list / as it was without either: N = 7, K = 3200 34.1 / 36.8 / 40.8,
+  // K = 9800 64.9 / 68.0 / 70.4, but K = 29768 146.9 / 142.5 / 140.4; N = 6 60.1 / 61.3 /
+  // 67.7 at K = 20000 and 104.0 / 104.7 / 106.5 at K = 45000, lower orders more)
+  if constexpr (P == PHYS_ADV && N >= 7 && LIST)
+    if (grid < q.ntiles) return rhs_blk<N, P, EPT, MAP, false>(p, sm_count, s, info);
+  return launch_stage(kern, grid, C::kThreads, C::kSmem, s, q);
 }
 
 // FP32 variants at orders 1..6: 0 = one thread per element-node (dg_rhs_kernel),
