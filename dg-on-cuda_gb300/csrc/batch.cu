@@ -14,9 +14,11 @@
 //   code 1: the register-blocked tiles of dg_rhs_blk_kernel with one element
 //           per thread slot (blk_tiles, variant 5 at orders 1..6 and 1 at
 //           orders 7, 8), double-buffered within each work item.
-// An instance runs code 1 when its handle is set to that variant (e.g. by
-// dgc_autotune) and code 0 otherwise, so a batched step is bitwise equal to
-// the handle's own dgc_lserk4_step with either of those two variants.  The
+// An instance runs code 1 when its handle is set to that variant or to the even /
+// odd one (6, 2 at orders 7, 8: it has no batch form, and dgc_autotune picks it
+// where the blocked tiles are the next best), and code 0 otherwise, so a batched
+// step is bitwise equal to the handle's own dgc_lserk4_step with variant 0 or the
+// blocked variant.  The
 // launch's dynamic shared memory is the largest layout among the batch's
 // instances, which sets the resident CTAs per SM.
 #include <cuda_runtime.h>
@@ -189,6 +191,8 @@ int physics_kind(int phys) {
 // the FP32 variant that runs the register-blocked tiles with one element per
 // thread slot (batch tile code 1)
 int blk_variant(int N) { return N <= 6 ? 5 : 1; }
+// whether a handle set to variant v runs tile code 1 in a batch
+bool blk_in_batch(int N, int v) { return v == blk_variant(N) || v == blk_variant(N) + 1; }
 
 // tile size and shared memory of an (order, physics, variant) stage kernel
 bool tile_info(int N, int phys, int variant, dgk::LaunchInfo* li) {
@@ -267,7 +271,7 @@ extern "C" int dgc_batch_create(const dgc_handle* handles, int n, dgc_batch* out
     if (h->prec != DGC_F32) return fail(berr(DGC_ERR_UNSUPPORTED, "batches run FP32 handles"));
     if (h->desc.physics == DGC_LAPLACE) return fail(berr(DGC_ERR_UNSUPPORTED, "batches run time-dependent handles"));
     const int P = physics_kind(h->desc.physics);
-    const int code = h->rhs_variant == blk_variant(h->N) ? 1 : 0;
+    const int code = blk_in_batch(h->N, h->rhs_variant) ? 1 : 0;
     kinds[i] = ((h->N - 1) * 3 + P) * 2 + code;
     dgk::LaunchInfo li;
     if (!tile_info(h->N, h->desc.physics, code ? blk_variant(h->N) : 0, &li) || li.tile <= 0)

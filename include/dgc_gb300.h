@@ -219,9 +219,11 @@ int dgc_lserk4_run(dgc_handle h, void* qa, void* qb, void* res, double t0, doubl
 /* A batch over existing FP32 advection / Maxwell handles (any mix of orders
  * and mesh sizes).  Every LSERK4 stage of every instance runs in ONE launch:
  * persistent CTAs take work items (instance, run of tiles) from a device
- * queue ordered by decreasing cost, and evaluate them with the same tile code
- * as the handles' variant-0 stage kernel, so a batched step is bitwise equal
- * to per-instance dgc_lserk4_step calls with that variant.  The handles must
+ * queue ordered by decreasing cost, and evaluate them with one of two tile
+ * codes: that of the blocked variant (5; 1 at orders 7, 8) for handles set to it
+ * or to the even / odd variant (6; 2) when the batch is created, e.g. by
+ * dgc_autotune, that of variant 0 for all others.  A batched step is bitwise
+ * equal to dgc_lserk4_step with the variant whose tiles run.  The handles must
  * outlive the batch.  No reference counterpart (the reference integrates one
  * problem per process). */
 typedef struct dgc_batch_s* dgc_batch;
