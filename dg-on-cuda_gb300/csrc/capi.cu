@@ -177,7 +177,9 @@ int upload_operators(dgc_handle_s* h, int form) {
     const int G = dgk::sym_rows(re.N), GP = dgk::sym_pad(G), gE = (d.nE + G - 1) / G, gO = (d.nO + G - 1) / G,
               KS = (gE + gO) * GP;
     std::vector<double> eo = dgc::eo_pack(re.N, Dr, Ds, L, nullptr);
-    h->eo_ok[0] = dgc::eo_symmetric(re.N, Dr, Ds, L, nullptr);
+    // that kernel also takes the state relative to a constant
+    h->eo_ok[0] = h->straight && dgc::eo_symmetric(re.N, Dr, Ds, L, nullptr) &&
+                  dgc::eo_constants_cancel(re.N, Dr, Ds, L);
     if (!h->eo_ok[0]) std::fill(eo.begin(), eo.end(), std::nan(""));
     const std::vector<uint8_t> tab = dgc::eo_tables(re.N);
     const size_t nops = ((size_t)(d.Np + d.fE) * KS + 3) / 4 * 4;
@@ -388,6 +390,7 @@ int device_init(dgc_handle_s* h) {
   CK(cudaMemset(h->d_status, 0, 64));
   CK(cudaMalloc(&h->d_time, 64));
   CK(cudaMemset(h->d_time, 0, 64));
+  h->straight = h->prec == DGC_F32 && h->desc.physics != DGC_LAPLACE && straight_sided(m);
   int rc = upload_operators(h, 0);
   if (rc != DGC_OK) return rc;
   rc = upload_operators(h, 1);

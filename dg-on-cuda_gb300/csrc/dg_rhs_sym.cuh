@@ -82,6 +82,18 @@ __device__ __forceinline__ void sym_ops(const float* k, float (&o)[G]) {
   }
 }
 
+// Each element's state is taken relative to its value at node 0 (c below), and so
+// are the exterior values on its faces: a constant state has no right-hand side
+// (volume and flux terms cancel on a straight-sided element), so c drops out, and
+// with it the part of the operators' FP32 rounding that acts on the state's
+// magnitude.  Without it that part, larger here than in the node basis because the
+// operators are rounded after the change of basis, grew with the time integrated:
+// error against FP64 after the same run, blocked kernel / here without / here with:
+// Maxwell TE to T = 1, K = 32768, N = 6 5.8e-6 / 6.6e-6 / 3.9e-6, to T = 0.5, K = 4608,
+// N = 7 9.2e-6 / 1.2e-5 / 2.5e-6, advection to T = 0.5, K = 8192, N = 4 1.1e-6 / 2.0e-6 /
+// 1.1e-6.  It costs the Maxwell stage 1-3 % (K = 32768, N = 6: 17.4 -> 17.7 us).
+// Operators or geometry without that cancellation run the blocked kernel.
+//
 // The tile of ne elements from k0.  Operators, geometry and neighbours are in
 // shared memory; the state arrives on `bar`, phase 0.
 template <int N, int P>
@@ -171,12 +183,17 @@ __device__ __forceinline__ void sym_tile(const RhsParams& p, unsigned char* smem
         if (P == PHYS_ADV) {
           const float an = cax * nx + cay * ny;
           const float bx = bs[q][w] >= 0 ? bval[bs[q][w]] : bb[0];
-          fl[w][0] = ((an >= 0.0f) ? a[0] : bx) * an * sc;
+          fl[w][0] = (((an >= 0.0f) ? a[0] : bx) - qa[0]) * an * sc;
         } else {
           if (bs[q][w] == -2) {  // PEC: E+ = -E-, Hz+ = Hz- | H+ = H-, Ez+ = -Ez-
             bb[0] = P == PHYS_TE ? -a[0] : a[0];
             bb[1] = P == PHYS_TE ? -a[1] : a[1];
             bb[2] = P == PHYS_TE ? a[2] : -a[2];
+          }
+#pragma unroll
+          for (int i = 0; i < NF; ++i) {
+            a[i] -= qa[i * NpP];
+            bb[i] -= qa[i * NpP];
           }
           if (P == PHYS_TM) {
             const float w3 = (a[2] + bb[2]) + ny * (a[0] - bb[0]) - nx * (a[1] - bb[1]);
@@ -209,7 +226,7 @@ __device__ __forceinline__ void sym_tile(const RhsParams& p, unsigned char* smem
     const bool two = c < nO;
     float* in = sI + e * ISTR;
     if (P == PHYS_ADV) {
-      const float u = qa[na], v = qa[nb];
+      const float u = qa[na] - qa[0], v = qa[nb] - qa[0];
       in[c] = two ? u + v : u;
       if (two) in[nE + c] = u - v;
       if (c == 0) {
@@ -220,9 +237,10 @@ __device__ __forceinline__ void sym_tile(const RhsParams& p, unsigned char* smem
     } else {
       const float sg = P == PHYS_TE ? 1.0f : -1.0f;
       const float p1 = sg * (g.x + g.z), p2 = sg * (g.x - g.z), q1 = -sg * (g.y + g.w), q2 = -sg * (g.y - g.w);
-      const float u0 = qa[na], u1 = qa[NpP + na], u2 = qa[2 * NpP + na];
+      const float c0 = qa[0], c1 = qa[NpP], c2 = qa[2 * NpP];
+      const float u0 = qa[na] - c0, u1 = qa[NpP + na] - c1, u2 = qa[2 * NpP + na] - c2;
       if (two) {
-        const float v0 = qa[nb], v1 = qa[NpP + nb], v2 = qa[2 * NpP + nb];
+        const float v0 = qa[nb] - c0, v1 = qa[NpP + nb] - c1, v2 = qa[2 * NpP + nb] - c2;
         const float s0 = u0 + v0, s1 = u1 + v1, d0 = u0 - v0, d1 = u1 - v1;
         in[c] = u2 + v2;
         in[nE + c] = u2 - v2;

@@ -34,6 +34,7 @@ struct dgc_handle_s {
   double* d_eo64[2] = {nullptr, nullptr};  // the same, FP64, in the even / odd basis (eo.hpp), then its pair tables
   float* d_sym32 = nullptr;                // FP32, weak form, in row groups (dg_rhs_sym.cuh), then the tables
   const uint8_t* d_sym_tab = nullptr;
+  bool straight = false;                   // straight_sided(mesh), asked for FP32 stage handles
   bool eo_ok[2] = {false, false};          // the operators have the symmetry that basis needs
   const uint8_t* d_eo_tab[2] = {nullptr, nullptr};
   void* d_tc_b = nullptr;     // FP32 tensor-core operand [Dr | Ds | LIFT] (strong form, split TF32)

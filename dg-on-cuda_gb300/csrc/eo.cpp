@@ -76,6 +76,27 @@ bool eo_symmetric(int N, const std::vector<double>& Dr, const std::vector<double
   return true;
 }
 
+bool eo_constants_cancel(int N, const std::vector<double>& Dr, const std::vector<double>& Ds,
+                         const std::vector<double>& L) {
+  const dgk::EoDims d(N);
+  double big = 0.0, off = 0.0;
+  auto see = [&](double x) {
+    off = std::isfinite(x) ? std::max(off, std::fabs(x)) : INFINITY;
+  };
+  for (int i = 0; i < d.Np; ++i) {
+    double vr = 0.0, vs = 0.0, l[3] = {0.0, 0.0, 0.0};
+    for (int j = 0; j < d.Np; ++j) {
+      vr += Dr[(size_t)i * d.Np + j];
+      vs += Ds[(size_t)i * d.Np + j];
+    }
+    for (int m = 0; m < 3 * d.Nfp; ++m) l[m / d.Nfp] += L[(size_t)i * 3 * d.Nfp + m];
+    for (double v : l) big = std::max(big, std::fabs(v));
+    see(vr - (l[1] - l[2]));
+    see(vs - (l[1] - l[0]));
+  }
+  return off <= 1e-10 * big;
+}
+
 std::vector<double> eo_pack(int N, const std::vector<double>& Dr, const std::vector<double>& Ds,
                             const std::vector<double>& L, const std::vector<double>* M) {
   const dgk::EoDims d(N);

@@ -122,6 +122,13 @@ std::vector<uint8_t> eo_tables(int N);
 bool eo_symmetric(int N, const std::vector<double>& Dr, const std::vector<double>& Ds, const std::vector<double>& L,
                   const std::vector<double>* M);
 
+// Whether the weak form's volume and flux terms cancel for a constant state (to
+// 1e-10 of the largest face row sum): Dr 1 = l1 - l2 and Ds 1 = l1 - l0 with l_f the
+// sums of LIFT's columns of face f.  With straight-sided geometry (straight_sided)
+// the right-hand side of q then equals that of q - c, element by element.
+bool eo_constants_cancel(int N, const std::vector<double>& Dr, const std::vector<double>& Ds,
+                         const std::vector<double>& L);
+
 // The K, L and M parts of the blob (M left out when null), in FP64.
 std::vector<double> eo_pack(int N, const std::vector<double>& Dr, const std::vector<double>& Ds,
                             const std::vector<double>& L, const std::vector<double>* M);

@@ -320,7 +320,8 @@ cudaError_t rhs_blk(const RhsParams* p, int sm_count, cudaStream_t s, LaunchInfo
 constexpr int kF32Variants = 10;
 constexpr int kF32VariantsHigh = 4;
 
-// variant 6 (2 at orders 7, 8): operators without the reflection symmetry run the
+// variant 6 (2 at orders 7, 8): operators without the reflection symmetry, and
+// operators or geometry under which a constant state has a right-hand side, run the
 // blocked kernel
 template <int N, int P>
 cudaError_t rhs_sym_or_blk(const RhsParams* p, int sm, cudaStream_t s, LaunchInfo* info) {

@@ -432,6 +432,24 @@ void fill_penalty(MeshData& m, const RefElement& re) {
     }
 }
 
+bool straight_sided(const MeshData& m) {
+  for (int k = 0; k < m.K; ++k) {
+    const double* g = &m.geom[(size_t)k * kGeomStride];
+    double big = 0.0, off = 0.0;
+    for (int x = 0; x < 2; ++x) {
+      const double r = g[G_RX + x], s = g[G_SX + x], want[3] = {-s, r + s, -r};
+      for (int f = 0; f < 3; ++f) {
+        const double have = g[(x ? G_NY0 : G_NX0) + f] * g[G_FJ0 + f] / g[G_J];
+        big = std::max(big, std::fabs(want[f]));
+        off = std::max(off, std::fabs(have - want[f]));
+        if (!std::isfinite(have - want[f])) return false;
+      }
+    }
+    if (!(off <= 1e-10 * big)) return false;
+  }
+  return true;
+}
+
 bool build_mesh_from_arrays(int K, const RefElement& re, const double* invJ, const double* J, const double* faceJ,
                             const int32_t* nb_cell, const int32_t* nb_face, int num_boundary_nodes, const double* bx,
                             const double* by, const double* nx, const double* ny, MeshData& m, std::string& err) {

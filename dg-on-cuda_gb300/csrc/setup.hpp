@@ -86,6 +86,12 @@ std::vector<R> kernel_geometry(const std::vector<double>& geom, int K) {
   return g;
 }
 
+struct MeshData;
+// Whether every element's face normals, times faceJ / J, are -grad s, grad (r + s) and
+// -grad r (to 1e-10), as on straight-sided triangles: meshes always, arrays a
+// caller gives only if they describe such elements.
+bool straight_sided(const MeshData& m);
+
 struct MeshData {
   int K = 0, nv = 0, N = 0, Np = 0, Nfp = 0;
   std::vector<double> vx, vy;
