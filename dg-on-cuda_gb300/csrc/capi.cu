@@ -2,7 +2,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -154,43 +153,46 @@ int upload_operators(dgc_handle_s* h, int form) {
   CK(cudaMemcpy(h->d_mats64[form], m64.data(), m64.size() * sizeof(double), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(h->d_mats32[form], m32.data(), m32.size() * sizeof(float), cudaMemcpyHostToDevice));
   // even / odd form for the FP64 kernels: the weak operators of FP64 handles and
-  // the strong ones of laplace handles.  Operators without the reflection
-  // symmetry run the node-by-node kernels; NaN in its place then, so that a graph
-  // a caller captured with symmetric operators cannot quietly go on with those.
+  // the strong ones of laplace handles, then tables and rest (eo.hpp).  Operators
+  // without the reflection symmetry run the node-by-node kernels; the rest is for
+  // graphs that a caller captured before.
   if (form == 0 ? h->prec == DGC_F64 : h->desc.physics == DGC_LAPLACE) {
     const std::vector<double>* M = form == 1 ? &re.M : nullptr;
-    const std::vector<uint8_t> tab = dgc::eo_tables(re.N);
-    std::vector<double> eo = dgc::eo_pack(re.N, Dr, Ds, L, M);
     h->eo_ok[form] = dgc::eo_symmetric(re.N, Dr, Ds, L, M);
-    if (!h->eo_ok[form]) std::fill(eo.begin(), eo.end(), std::nan(""));
+    const std::vector<uint8_t> tab = dgc::eo_tables(re.N, !h->eo_ok[form]);
+    std::vector<double> eo = dgc::eo_pack(re.N, Dr, Ds, L, M);
+    const std::vector<double> rest = dgc::eo_pack(re.N, Dr, Ds, L, nullptr, true);
     const size_t nops = eo.size();
     eo.resize(nops + tab.size() / sizeof(double));
     std::memcpy(eo.data() + nops, tab.data(), tab.size());
+    eo.insert(eo.end(), rest.begin(), rest.end());
     if (!h->d_eo64[form]) CK(cudaMalloc(&h->d_eo64[form], eo.size() * sizeof(double)));
     CK(cudaMemcpy(h->d_eo64[form], eo.data(), eo.size() * sizeof(double), cudaMemcpyHostToDevice));
     h->d_eo_tab[form] = reinterpret_cast<const uint8_t*>(h->d_eo64[form] + nops);
   }
   if (form == 0 && h->prec == DGC_F32 && h->desc.physics != DGC_LAPLACE) {
     // the FP32 stage kernel's even / odd operators: rows in groups of G of one
-    // parity, each padded to GP values
+    // parity, each padded to GP values; then tables and rest
     const dgk::EoDims d(re.N);
     const int G = dgk::sym_rows(re.N), GP = dgk::sym_pad(G), gE = (d.nE + G - 1) / G, gO = (d.nO + G - 1) / G,
               KS = (gE + gO) * GP;
-    std::vector<double> eo = dgc::eo_pack(re.N, Dr, Ds, L, nullptr);
     // that kernel also takes the state relative to a constant
     h->eo_ok[0] = h->straight && dgc::eo_symmetric(re.N, Dr, Ds, L, nullptr) &&
                   dgc::eo_constants_cancel(re.N, Dr, Ds, L);
-    if (!h->eo_ok[0]) std::fill(eo.begin(), eo.end(), std::nan(""));
-    const std::vector<uint8_t> tab = dgc::eo_tables(re.N);
-    const size_t nops = ((size_t)(d.Np + d.fE) * KS + 3) / 4 * 4;
-    std::vector<float> sy(nops + tab.size() / sizeof(float), 0.0f);
-    for (int c = 0; c < d.Np + d.fE; ++c)
-      for (int r = 0; r < d.Np; ++r) {
-        const bool odd = r >= d.nE;
-        const int q = odd ? r - d.nE : r, col = ((odd ? gE : 0) + q / G) * GP + q % G;
-        const double v = c < d.Np ? eo[(size_t)c * d.Np + r] : eo[(size_t)d.kK() + (size_t)(c - d.Np) * d.Np + r];
-        sy[(size_t)c * KS + col] = (float)v;
-      }
+    const std::vector<uint8_t> tab = dgc::eo_tables(re.N, !h->eo_ok[0]);
+    const size_t nops = ((size_t)(d.Np + d.fE) * KS + 3) / 4 * 4, ntab = tab.size() / sizeof(float);
+    std::vector<float> sy(2 * nops + ntab, 0.0f);
+    for (int part = 0; part < 2; ++part) {
+      const std::vector<double> eo = dgc::eo_pack(re.N, Dr, Ds, L, nullptr, part == 1);
+      float* to = sy.data() + part * (nops + ntab);
+      for (int c = 0; c < d.Np + d.fE; ++c)
+        for (int r = 0; r < d.Np; ++r) {
+          const bool odd = r >= d.nE;
+          const int q = odd ? r - d.nE : r, col = ((odd ? gE : 0) + q / G) * GP + q % G;
+          const double v = c < d.Np ? eo[(size_t)c * d.Np + r] : eo[(size_t)d.kK() + (size_t)(c - d.Np) * d.Np + r];
+          to[(size_t)c * KS + col] = (float)v;
+        }
+    }
     std::memcpy(sy.data() + nops, tab.data(), tab.size());
     if (!h->d_sym32) CK(cudaMalloc(&h->d_sym32, sy.size() * sizeof(float)));
     CK(cudaMemcpy(h->d_sym32, sy.data(), sy.size() * sizeof(float), cudaMemcpyHostToDevice));

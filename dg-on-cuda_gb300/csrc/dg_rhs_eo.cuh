@@ -309,6 +309,8 @@ __global__ void __launch_bounds__(256) dg_rhs_eo_kernel(const RhsParams p) {
   __syncthreads();
 
   // ---- rows: sum row (r < nE) or difference row of element e
+  const bool rest = nt[C::D.flag()] != 0;  // operators without the symmetry (eo.hpp)
+  auto rest_row = [&] { return reinterpret_cast<const R*>(p.tab_eo + C::kTab) + r; };
   R rr[NF];
   if (act) {
     const bool sum = r < nE;
@@ -323,6 +325,12 @@ __global__ void __launch_bounds__(256) dg_rhs_eo_kernel(const RhsParams p) {
       x += nE;
 #pragma unroll 4
       for (int c = 0; c < nO; ++c) s2 = fma(k[c * Np], x[c], s2);
+      if (rest) {
+        const R* k2 = rest_row();
+        x = sI + e * C::ISTR;
+#pragma unroll 1
+        for (int c = 0; c < Np; ++c) (c < nE ? s2 : s1) = fma(k2[c * Np], x[c], c < nE ? s2 : s1);
+      }
       const R p1 = cc[EC_P1], p2 = cc[EC_P2];
       rr[0] = sum ? fma(p1, s1, p2 * s2) : fma(p2, s1, p1 * s2);
     } else {
@@ -344,6 +352,17 @@ __global__ void __launch_bounds__(256) dg_rhs_eo_kernel(const RhsParams p) {
         s2 = fma(kk, x[c], s2);
         cv = fma(kk, v[c], cv);
       }
+      if (rest) {
+        const R* k2 = rest_row();
+        x = sI + e * C::ISTR;
+#pragma unroll 1
+        for (int c = 0; c < Np; ++c) {
+          const R kk = k2[c * Np];
+          (c < nE ? s2 : s1) = fma(kk, x[c], c < nE ? s2 : s1);
+          // sum rows: m's sums and p's differences, difference rows the others
+          cu = fma(kk, x[((c < nE) == sum ? 2 * Np : Np) + c], cu);
+        }
+      }
       const int ia = sum ? 0 : 1;  // D+ q2 is s1 in a sum row, s2 in a difference row
       rr[0] = fma(cc[EC_Q1 + ia], s1, cc[EC_Q2 - ia] * s2);
       rr[1] = fma(cc[EC_P1 + ia], s1, cc[EC_P2 - ia] * s2);
@@ -356,6 +375,13 @@ __global__ void __launch_bounds__(256) dg_rhs_eo_kernel(const RhsParams p) {
       const R ll = l[m * Np];
 #pragma unroll
       for (int i = 0; i < NF; ++i) rr[i] = fma(ll, f[i * 2 * fE + m], rr[i]);
+    }
+    if (rest) {
+      l = rest_row() + C::D.kK();
+      f = sF + e * C::FSTR + (sum ? fE : 0);
+#pragma unroll 1
+      for (int m = 0; m < (sum ? fO : fE); ++m)
+        for (int i = 0; i < NF; ++i) rr[i] = fma(l[m * Np], f[i * 2 * fE + m], rr[i]);
     }
   }
   __syncthreads();

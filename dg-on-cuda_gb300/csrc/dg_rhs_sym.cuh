@@ -27,6 +27,8 @@
 // and K = 2048, N = 6 5.4 / 4.5: the autotuner decides.
 #pragma once
 
+#include <type_traits>
+
 #include "dg_rhs.cuh"
 #include "eo.hpp"
 
@@ -119,6 +121,9 @@ __device__ __forceinline__ void sym_tile(const RhsParams& p, unsigned char* smem
   const int tid = threadIdx.x;
   const float* qin = static_cast<const float*>(p.q_in);
   const float cax = p.fax, cay = p.fay;
+  // operators that have lost the symmetry (eo.hpp) or the cancellation
+  const bool rest = nt[C::D.flag()] != 0;
+  auto rest_ops = [&] { return reinterpret_cast<const float*>(p.tab_eo + C::kTab); };
 
   // ---- exterior values of the face-node pairs
   float b[kItems][2][NF];
@@ -161,106 +166,114 @@ __device__ __forceinline__ void sym_tile(const RhsParams& p, unsigned char* smem
   }
   if (!__syncthreads_and(mbar_wait(bar, 0, p.status))) return;
 
-  // ---- fluxes of the pairs, scaled by -faceJ / J, as sums and differences
+  // the two phases that take the constant off (compiled twice: a test at each value
+  // cost up to 5 % of the stage)
+  auto prepare = [&](auto cancels) {
+    // the element's constant
+    auto level = [&](const float* qa, int i) { return decltype(cancels)::value ? qa[i * NpP] : 0.0f; };
+    // ---- fluxes of the pairs, scaled by -faceJ / J, as sums and differences
 #pragma unroll
-  for (int q = 0; q < kItems; ++q) {
-    const int x = tid + q * NT;
-    if (x < ne * fE) {
-      const int e = x / fE, c = x - e * fE;
-      const float* g = sG + e * 16;
-      const float* qa = sQ + e * ESTR;
-      const bool two = c < fO;
-      float fl[2][NF];
+    for (int q = 0; q < kItems; ++q) {
+      const int x = tid + q * NT;
+      if (x < ne * fE) {
+        const int e = x / fE, c = x - e * fE;
+        const float* g = sG + e * 16;
+        const float* qa = sQ + e * ESTR;
+        const bool two = c < fO;
+        float fl[2][NF];
 #pragma unroll
-      for (int w = 0; w < 2; ++w) {
-        if (w && !two) break;
-        const int m = ft[2 * c + w], f = m / Nfp, d = m - f * Nfp, nd = fmask<N>(f, d);
-        const float nx = g[8 + f], ny = g[11 + f], sc = g[5 + f] * g[4];  // g[4] = -1/J
-        float a[NF];
+        for (int w = 0; w < 2; ++w) {
+          if (w && !two) break;
+          const int m = ft[2 * c + w], f = m / Nfp, d = m - f * Nfp, nd = fmask<N>(f, d);
+          const float nx = g[8 + f], ny = g[11 + f], sc = g[5 + f] * g[4];  // g[4] = -1/J
+          float a[NF];
 #pragma unroll
-        for (int i = 0; i < NF; ++i) a[i] = qa[i * NpP + nd];
-        float* bb = b[q][w];
-        if (P == PHYS_ADV) {
-          const float an = cax * nx + cay * ny;
-          const float bx = bs[q][w] >= 0 ? bval[bs[q][w]] : bb[0];
-          fl[w][0] = (((an >= 0.0f) ? a[0] : bx) - qa[0]) * an * sc;
-        } else {
-          if (bs[q][w] == -2) {  // PEC: E+ = -E-, Hz+ = Hz- | H+ = H-, Ez+ = -Ez-
-            bb[0] = P == PHYS_TE ? -a[0] : a[0];
-            bb[1] = P == PHYS_TE ? -a[1] : a[1];
-            bb[2] = P == PHYS_TE ? a[2] : -a[2];
-          }
-#pragma unroll
-          for (int i = 0; i < NF; ++i) {
-            a[i] -= qa[i * NpP];
-            bb[i] -= qa[i * NpP];
-          }
-          if (P == PHYS_TM) {
-            const float w3 = (a[2] + bb[2]) + ny * (a[0] - bb[0]) - nx * (a[1] - bb[1]);
-            fl[w][0] = 0.5f * ny * w3 * sc;
-            fl[w][1] = -0.5f * nx * w3 * sc;
-            fl[w][2] = 0.5f * (ny * (a[0] + bb[0]) - nx * (a[1] + bb[1]) + a[2] - bb[2]) * sc;
+          for (int i = 0; i < NF; ++i) a[i] = qa[i * NpP + nd];
+          float* bb = b[q][w];
+          if (P == PHYS_ADV) {
+            const float an = cax * nx + cay * ny;
+            const float bx = bs[q][w] >= 0 ? bval[bs[q][w]] : bb[0];
+            fl[w][0] = (((an >= 0.0f) ? a[0] : bx) - level(qa, 0)) * an * sc;
           } else {
-            const float w3 = (a[2] + bb[2]) - ny * (a[0] - bb[0]) + nx * (a[1] - bb[1]);
-            fl[w][0] = -0.5f * ny * w3 * sc;
-            fl[w][1] = 0.5f * nx * w3 * sc;
-            fl[w][2] = 0.5f * (nx * (a[1] + bb[1]) - ny * (a[0] + bb[0]) + a[2] - bb[2]) * sc;
+            if (bs[q][w] == -2) {  // PEC: E+ = -E-, Hz+ = Hz- | H+ = H-, Ez+ = -Ez-
+              bb[0] = P == PHYS_TE ? -a[0] : a[0];
+              bb[1] = P == PHYS_TE ? -a[1] : a[1];
+              bb[2] = P == PHYS_TE ? a[2] : -a[2];
+            }
+#pragma unroll
+            for (int i = 0; i < NF; ++i) {
+              a[i] -= level(qa, i);
+              bb[i] -= level(qa, i);
+            }
+            if (P == PHYS_TM) {
+              const float w3 = (a[2] + bb[2]) + ny * (a[0] - bb[0]) - nx * (a[1] - bb[1]);
+              fl[w][0] = 0.5f * ny * w3 * sc;
+              fl[w][1] = -0.5f * nx * w3 * sc;
+              fl[w][2] = 0.5f * (ny * (a[0] + bb[0]) - nx * (a[1] + bb[1]) + a[2] - bb[2]) * sc;
+            } else {
+              const float w3 = (a[2] + bb[2]) - ny * (a[0] - bb[0]) + nx * (a[1] - bb[1]);
+              fl[w][0] = -0.5f * ny * w3 * sc;
+              fl[w][1] = 0.5f * nx * w3 * sc;
+              fl[w][2] = 0.5f * (nx * (a[1] + bb[1]) - ny * (a[0] + bb[0]) + a[2] - bb[2]) * sc;
+            }
           }
         }
-      }
-      float* fo = sF + e * FSTR + c;
+        float* fo = sF + e * FSTR + c;
 #pragma unroll
-      for (int i = 0; i < NF; ++i) {
-        fo[i * (fE + fO)] = two ? fl[0][i] + fl[1][i] : fl[0][i];
-        if (two) fo[i * (fE + fO) + fE] = fl[0][i] - fl[1][i];
+        for (int i = 0; i < NF; ++i) {
+          fo[i * (fE + fO)] = two ? fl[0][i] + fl[1][i] : fl[0][i];
+          if (two) fo[i * (fE + fO) + fE] = fl[0][i] - fl[1][i];
+        }
       }
     }
-  }
-  // ---- inputs of the node pairs: Maxwell [q2 | p | m], advection [q], each [sums | differences];
-  //      the element's constants behind them
-  for (int x = tid; x < ne * nE; x += NT) {
-    const int e = x / nE, c = x - e * nE;
-    const float* qa = sQ + e * ESTR;
-    const float4 g = *reinterpret_cast<const float4*>(sG + e * 16);  // rx ry sx sy
-    const int na = nt[2 * c], nb = nt[2 * c + 1];
-    const bool two = c < nO;
-    float* in = sI + e * ISTR;
-    if (P == PHYS_ADV) {
-      const float u = qa[na] - qa[0], v = qa[nb] - qa[0];
-      in[c] = two ? u + v : u;
-      if (two) in[nE + c] = u - v;
-      if (c == 0) {
-        const float al = cax * g.x + cay * g.y, be = cax * g.z + cay * g.w;
-        in[C::IN] = al + be;
-        in[C::IN + 1] = al - be;
-      }
-    } else {
-      const float sg = P == PHYS_TE ? 1.0f : -1.0f;
-      const float p1 = sg * (g.x + g.z), p2 = sg * (g.x - g.z), q1 = -sg * (g.y + g.w), q2 = -sg * (g.y - g.w);
-      const float c0 = qa[0], c1 = qa[NpP], c2 = qa[2 * NpP];
-      const float u0 = qa[na] - c0, u1 = qa[NpP + na] - c1, u2 = qa[2 * NpP + na] - c2;
-      if (two) {
-        const float v0 = qa[nb] - c0, v1 = qa[NpP + nb] - c1, v2 = qa[2 * NpP + nb] - c2;
-        const float s0 = u0 + v0, s1 = u1 + v1, d0 = u0 - v0, d1 = u1 - v1;
-        in[c] = u2 + v2;
-        in[nE + c] = u2 - v2;
-        in[Np + c] = p1 * s1 + q1 * s0;
-        in[Np + nE + c] = p1 * d1 + q1 * d0;
-        in[2 * Np + c] = p2 * s1 + q2 * s0;
-        in[2 * Np + nE + c] = p2 * d1 + q2 * d0;
+    // ---- inputs of the node pairs: Maxwell [q2 | p | m], advection [q], each [sums | differences];
+    //      the element's constants behind them
+    for (int x = tid; x < ne * nE; x += NT) {
+      const int e = x / nE, c = x - e * nE;
+      const float* qa = sQ + e * ESTR;
+      const float4 g = *reinterpret_cast<const float4*>(sG + e * 16);  // rx ry sx sy
+      const int na = nt[2 * c], nb = nt[2 * c + 1];
+      const bool two = c < nO;
+      float* in = sI + e * ISTR;
+      if (P == PHYS_ADV) {
+        const float c0 = level(qa, 0), u = qa[na] - c0, v = qa[nb] - c0;
+        in[c] = two ? u + v : u;
+        if (two) in[nE + c] = u - v;
+        if (c == 0) {
+          const float al = cax * g.x + cay * g.y, be = cax * g.z + cay * g.w;
+          in[C::IN] = al + be;
+          in[C::IN + 1] = al - be;
+        }
       } else {
-        in[c] = u2;
-        in[Np + c] = p1 * u1 + q1 * u0;
-        in[2 * Np + c] = p2 * u1 + q2 * u0;
-      }
-      if (c == 0) {
-        in[C::IN] = p1;
-        in[C::IN + 1] = p2;
-        in[C::IN + 2] = q1;
-        in[C::IN + 3] = q2;
+        const float sg = P == PHYS_TE ? 1.0f : -1.0f;
+        const float p1 = sg * (g.x + g.z), p2 = sg * (g.x - g.z), q1 = -sg * (g.y + g.w), q2 = -sg * (g.y - g.w);
+        const float c0 = level(qa, 0), c1 = level(qa, 1), c2 = level(qa, 2);
+        const float u0 = qa[na] - c0, u1 = qa[NpP + na] - c1, u2 = qa[2 * NpP + na] - c2;
+        if (two) {
+          const float v0 = qa[nb] - c0, v1 = qa[NpP + nb] - c1, v2 = qa[2 * NpP + nb] - c2;
+          const float s0 = u0 + v0, s1 = u1 + v1, d0 = u0 - v0, d1 = u1 - v1;
+          in[c] = u2 + v2;
+          in[nE + c] = u2 - v2;
+          in[Np + c] = p1 * s1 + q1 * s0;
+          in[Np + nE + c] = p1 * d1 + q1 * d0;
+          in[2 * Np + c] = p2 * s1 + q2 * s0;
+          in[2 * Np + nE + c] = p2 * d1 + q2 * d0;
+        } else {
+          in[c] = u2;
+          in[Np + c] = p1 * u1 + q1 * u0;
+          in[2 * Np + c] = p2 * u1 + q2 * u0;
+        }
+        if (c == 0) {
+          in[C::IN] = p1;
+          in[C::IN + 1] = p2;
+          in[C::IN + 2] = q1;
+          in[C::IN + 3] = q2;
+        }
       }
     }
-  }
+  };
+  if (rest) prepare(std::false_type{});
+  else prepare(std::true_type{});
   __syncthreads();
 
   // ---- rows: warp = (block of 32 elements, row group), lane = element
@@ -292,6 +305,20 @@ __device__ __forceinline__ void sym_tile(const RhsParams& p, unsigned char* smem
         const float xv = x[c];
 #pragma unroll
         for (int g = 0; g < G; ++g) s2[g] = fmaf(o[g], xv, s2[g]);
+      }
+      if (rest) {
+        const float* k2 = rest_ops() + grp * GP;
+#pragma unroll 1
+        for (int c = 0; c < Np; ++c) {
+          float o[G];
+          sym_ops<G, GP>(k2 + c * KS, o);
+          const float xe = c < nE ? x[c] : 0.0f, xo = c < nE ? 0.0f : x[c];
+#pragma unroll
+          for (int g = 0; g < G; ++g) {
+            s2[g] = fmaf(o[g], xe, s2[g]);
+            s1[g] = fmaf(o[g], xo, s1[g]);
+          }
+        }
       }
       const float p1 = x[C::IN], p2 = x[C::IN + 1];
       const float ca = sum ? p1 : p2, cb = sum ? p2 : p1;
@@ -326,6 +353,23 @@ __device__ __forceinline__ void sym_tile(const RhsParams& p, unsigned char* smem
           cu[g] = fmaf(o[g], vv, cu[g]);
         }
       }
+      if (rest) {
+        const float* k2 = rest_ops() + grp * GP;
+#pragma unroll 1
+        for (int c = 0; c < Np; ++c) {
+          float o[G];
+          sym_ops<G, GP>(k2 + c * KS, o);
+          // sum rows: m's sums and p's differences, difference rows the others
+          const float xv = x[c], uv = x[((c < nE) == sum ? 2 * Np : Np) + c];
+          const float xe = c < nE ? xv : 0.0f, xo = c < nE ? 0.0f : xv;
+#pragma unroll
+          for (int g = 0; g < G; ++g) {
+            s2[g] = fmaf(o[g], xe, s2[g]);
+            s1[g] = fmaf(o[g], xo, s1[g]);
+            cu[g] = fmaf(o[g], uv, cu[g]);
+          }
+        }
+      }
       const float p1 = x[C::IN], p2 = x[C::IN + 1], q1 = x[C::IN + 2], q2 = x[C::IN + 3];
       // D+ q2 is s1 in a sum row, s2 in a difference row
       const float pa = sum ? p1 : p2, pb = sum ? p2 : p1, qa = sum ? q1 : q2, qb = sum ? q2 : q1;
@@ -348,6 +392,19 @@ __device__ __forceinline__ void sym_tile(const RhsParams& p, unsigned char* smem
         const float fv = f[i * (fE + fO) + m];
 #pragma unroll
         for (int g = 0; g < G; ++g) rr[i][g] = fmaf(o[g], fv, rr[i][g]);
+      }
+    }
+    if (rest) {
+      l = rest_ops() + Np * KS + grp * GP;
+      f = sF + re * FSTR + (sum ? fE : 0);
+#pragma unroll 1
+      for (int m = 0; m < (sum ? fO : fE); ++m) {
+        float o[G];
+        sym_ops<G, GP>(l + m * KS, o);
+#pragma unroll
+        for (int i = 0; i < NF; ++i)
+#pragma unroll
+          for (int g = 0; g < G; ++g) rr[i][g] = fmaf(o[g], f[i * (fE + fO) + m], rr[i][g]);
       }
     }
   }

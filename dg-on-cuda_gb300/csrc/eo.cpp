@@ -26,7 +26,7 @@ std::vector<int> node_image(int N) {
 
 }  // namespace
 
-std::vector<uint8_t> eo_tables(int N) {
+std::vector<uint8_t> eo_tables(int N, bool rest) {
   const dgk::EoDims d(N);
   std::vector<uint8_t> t;
   for (int i = 0; i <= N; ++i)
@@ -49,6 +49,7 @@ std::vector<uint8_t> eo_tables(int N) {
         t.push_back((uint8_t)(c | (t[2 * c] == i ? 0 : 128)));
         break;
       }
+  t.push_back(rest ? 1 : 0);
   t.resize((size_t)d.tabBytes(), 0);
   return t;
 }
@@ -98,7 +99,7 @@ bool eo_constants_cancel(int N, const std::vector<double>& Dr, const std::vector
 }
 
 std::vector<double> eo_pack(int N, const std::vector<double>& Dr, const std::vector<double>& Ds,
-                            const std::vector<double>& L, const std::vector<double>* M) {
+                            const std::vector<double>& L, const std::vector<double>* M, bool rest) {
   const dgk::EoDims d(N);
   const std::vector<uint8_t> t = eo_tables(N);
   const int NF = 3 * d.Nfp;
@@ -118,7 +119,7 @@ std::vector<double> eo_pack(int N, const std::vector<double>& Dr, const std::vec
   for (int c = 0; c < d.Np; ++c)
     for (int r = 0; r < d.Np; ++r) {
       const bool co = c >= d.nE, ro = r >= d.nE;
-      const double sg = co == ro ? 1.0 : -1.0;  // D+ keeps the parity, D- flips it
+      const double sg = (co == ro) != rest ? 1.0 : -1.0;  // D+ keeps the parity, D- flips it
       auto D = [&](int i, int j) {
         return 0.5 * (Dr[(size_t)i * d.Np + j] + sg * Ds[(size_t)i * d.Np + j]);
       };
@@ -128,9 +129,9 @@ std::vector<double> eo_pack(int N, const std::vector<double>& Dr, const std::vec
   double* l = out.data() + d.kK();
   auto Lf = [&](int i, int m) { return L[(size_t)i * NF + m]; };
   for (int r = 0; r < d.Np; ++r) {
-    const bool ro = r >= d.nE;
-    for (int c = 0; c < (ro ? d.fO : d.fE); ++c)
-      l[(size_t)c * d.Np + r] = coef(Lf, nt + 2 * (ro ? r - d.nE : r), ro, ft + 2 * c, ro);
+    const bool ro = r >= d.nE, co = ro != rest;
+    for (int c = 0; c < (co ? d.fO : d.fE); ++c)
+      l[(size_t)c * d.Np + r] = coef(Lf, nt + 2 * (ro ? r - d.nE : r), ro, ft + 2 * c, co);
   }
   if (M) {
     double* m = out.data() + d.kK() + d.kL();

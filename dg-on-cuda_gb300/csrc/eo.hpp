@@ -19,6 +19,13 @@
 // and columns are [nE sums | nO differences], nE = nP + nF, nO = nP.  Face-node
 // pairs: c < Nfp pairs node c of face 0 with node N - c of face 2, then the
 // pairs (d, N - d) of face 1, then its middle node (N even).
+//
+// Operators without the symmetry (dgc_set_operators) go to the node-by-node
+// kernels.  A graph that a caller captured before still holds the kernels of this
+// form: for it the tables carry a flag, and the blob the operators' rest, which
+// maps where the parts above do not (D+ sums to differences, LIFT difference
+// columns to sum rows, ...), in the same layout.  A kernel that finds the flag adds
+// it from global memory.
 #pragma once
 
 #include <cstdint>
@@ -44,9 +51,11 @@ struct EoDims {
   DGC_HD constexpr int kK() const { return (Np * Np + 3) / 4 * 4; }
   DGC_HD constexpr int kL() const { return (fE * Np + 3) / 4 * 4; }
   DGC_HD constexpr int kM() const { return (nE * Np + 3) / 4 * 4; }
-  // tables: pair (a, b) per sum column, pair (m1, m2) per face sum column, and
-  // per node its pair | 128 for the second member
-  DGC_HD constexpr int tabBytes() const { return (2 * nE + 2 * fE + Np + 15) / 16 * 16; }
+  // tables: pair (a, b) per sum column, pair (m1, m2) per face sum column, per node
+  // its pair | 128 for the second member, then the flag: 1 with a rest (which
+  // follows the tables in memory)
+  DGC_HD constexpr int flag() const { return 2 * nE + 2 * fE + Np; }
+  DGC_HD constexpr int tabBytes() const { return (flag() + 1 + 15) / 16 * 16; }
 };
 
 // FP64 instructions of a tile kernel per row (contraction to update), per
@@ -113,8 +122,9 @@ namespace dgc {
 
 // Node and face-node pair tables of order N, as the blob stores them:
 // 2 nE node indices, 2 fE face-node indices (f Nfp + d; the two members of an
-// unpaired entry are equal), then per node its pair | 128 for the second member.
-std::vector<uint8_t> eo_tables(int N);
+// unpaired entry are equal), then per node its pair | 128 for the second member
+// and the flag.
+std::vector<uint8_t> eo_tables(int N, bool rest = false);
 
 // Whether (Dr, Ds, L, M) have the reflection symmetry to rounding (1e-13 of
 // their largest entry); M may be null.  Operators a caller has replaced by ones
@@ -129,8 +139,9 @@ bool eo_symmetric(int N, const std::vector<double>& Dr, const std::vector<double
 bool eo_constants_cancel(int N, const std::vector<double>& Dr, const std::vector<double>& Ds,
                          const std::vector<double>& L);
 
-// The K, L and M parts of the blob (M left out when null), in FP64.
+// The K, L and M parts of the blob (M left out when null), in FP64; rest: the K and
+// L parts of the operators' rest (the mass matrix always has the symmetry).
 std::vector<double> eo_pack(int N, const std::vector<double>& Dr, const std::vector<double>& Ds,
-                            const std::vector<double>& L, const std::vector<double>* M);
+                            const std::vector<double>& L, const std::vector<double>* M, bool rest = false);
 
 }  // namespace dgc

@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(256) k_grad_eo(const IpdgParams p, const GradD
   }
   t.sum_diff(sU, ne);
   __syncthreads();
-  t.template grad_rows<true>(ne, k0, static_cast<double*>(p.qx), static_cast<double*>(p.qy));
+  t.template grad_rows<true>(p, ne, k0, static_cast<double*>(p.qx), static_cast<double*>(p.qy));
 }
 
 // divergence of (p.qx, p.qy) into p.out
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(256) k_div_eo(const IpdgParams p, const GradDi
   __syncthreads();
   const int e = tid / Np, r = tid - e * Np;
   const bool act = e < ne;
-  const double au = act ? t.div_row(e, r) : 0.0;
+  const double au = act ? t.div_row(p, e, r) : 0.0;
   __syncthreads();
   double* ro = t.in() + e * 2 * Np;
   if (act) ro[r] = au;

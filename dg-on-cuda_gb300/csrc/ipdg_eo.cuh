@@ -89,6 +89,11 @@ struct IpdgEoTile {
   __device__ const double* L() const { return K() + C::D.kK(); }
   __device__ const double* M() const { return L() + C::D.kL(); }
 
+  // operators without the symmetry: their rest's row r (eo.hpp), NULL without one
+  __device__ const double* rest(const IpdgParams& p, int r) const {
+    return smem[C::oTab + C::D.flag()] ? reinterpret_cast<const double*>(p.tab_eo + C::kTab) + r : nullptr;
+  }
+
   // set-up data of the elements k0 .. k0 + ne - 1; false if a wait expired
   __device__ bool setup(const IpdgParams& p, int k0, int ne, uint32_t ops, bool spd) const {
     if (threadIdx.x == 0) {
@@ -166,7 +171,7 @@ struct IpdgEoTile {
   // gradient rows of the tile from sum_diff's inputs and the x | y flux sums and
   // differences, then both components by node
   template <bool NEG = false>
-  __device__ void grad_rows(int ne, int k0, double* ox, double* oy) const {
+  __device__ void grad_rows(const IpdgParams& p, int ne, int k0, double* ox, double* oy) const {
     constexpr int Np = C::Np, nE = C::nE, nO = C::nO, fE = C::fE;
     const int e = (int)threadIdx.x / Np, r = (int)threadIdx.x - e * Np;
     const bool act = e < ne;
@@ -183,6 +188,11 @@ struct IpdgEoTile {
       x += nE;
 #pragma unroll 4
       for (int j = 0; j < nO; ++j) s2 = fma(k[j * Np], x[j], s2);
+      if (const double* k2 = rest(p, r)) {
+        x = in() + e * 2 * Np;
+#pragma unroll 1
+        for (int j = 0; j < Np; ++j) (j < nE ? s2 : s1) = fma(k2[j * Np], x[j], j < nE ? s2 : s1);
+      }
       const int ia = sum ? 0 : 1;  // D+ u is s1 in a sum row, s2 in a difference row
       qx = fma(c[IC_P1 + ia], s1, c[IC_P2 - ia] * s2);
       qy = fma(c[IC_Q1 + ia], s1, c[IC_Q2 - ia] * s2);
@@ -193,6 +203,14 @@ struct IpdgEoTile {
         const double ll = l[m * Np];
         qx = fma(ll, f[m], qx);
         qy = fma(ll, f[2 * fE + m], qy);
+      }
+      if (const double* l2 = rest(p, r)) {
+        f = flux() + e * C::FSTR + (sum ? fE : 0);
+#pragma unroll 1
+        for (int m = 0; m < (sum ? C::fO : fE); ++m) {
+          qx = fma(l2[C::D.kK() + m * Np], f[m], qx);
+          qy = fma(l2[C::D.kK() + m * Np], f[2 * fE + m], qy);
+        }
       }
     }
     __syncthreads();
@@ -209,7 +227,7 @@ struct IpdgEoTile {
     }
   }
   // divergence row r of element e from combine's inputs and the flux sums and differences
-  __device__ double div_row(int e, int r) const {
+  __device__ double div_row(const IpdgParams& p, int e, int r) const {
     constexpr int Np = C::Np, nE = C::nE, nO = C::nO, fE = C::fE;
     const bool sum = r < nE;
     const double* k = K() + r;
@@ -227,6 +245,14 @@ struct IpdgEoTile {
     const double* f = flux() + e * C::FSTR + (sum ? 0 : fE);
 #pragma unroll 4
     for (int m = 0; m < fE; ++m) s1 = fma(l[m * Np], f[m], s1);
+    if (const double* k2 = rest(p, r)) {
+      // sum rows: m's sums and p's differences, difference rows the others
+#pragma unroll 1
+      for (int j = 0; j < Np; ++j) s2 = fma(k2[j * Np], x[((j < nE) == sum ? Np : 0) + j], s2);
+      f = flux() + e * C::FSTR + (sum ? fE : 0);
+#pragma unroll 1
+      for (int m = 0; m < (sum ? C::fO : fE); ++m) s2 = fma(k2[C::D.kK() + m * Np], f[m], s2);
+    }
     return s1 + s2;
   }
 };
@@ -319,7 +345,7 @@ __global__ void __launch_bounds__(256) ipdg_grad_eo_kernel(const IpdgParams p) {
   }
   t.sum_diff(sU, ne);
   __syncthreads();
-  t.grad_rows(ne, k0, static_cast<double*>(p.qx), static_cast<double*>(p.qy));
+  t.grad_rows(p, ne, k0, static_cast<double*>(p.qx), static_cast<double*>(p.qy));
 }
 
 // ---------------------------------------------------------------- div pass
@@ -406,7 +432,7 @@ __global__ void __launch_bounds__(256) ipdg_div_eo_kernel(const IpdgParams p) {
   double au = 0.0;
   const bool sum = r < nE;
   if (act) {
-    au = t.div_row(e, r);
+    au = t.div_row(p, e, r);
     if (SPD && p.shift != 0.0) {  // (A - shift I) u, scaled by -J like the rest
       const int c = sum ? r : r - nE;
       const double ua = sU[e * NpP + t.nodes()[2 * c]], ub = sU[e * NpP + t.nodes()[2 * c + 1]];

@@ -152,11 +152,11 @@ int dgc_get_operator(dgc_handle h, int which, double* out);
 
 /* Replace the operator matrices by caller-supplied FP64 ones (e.g. the
  * reference's own m_Dr, m_Ds, m_L, which k_advection_2d.cu:60-62 copies to
- * __constant__ memory).  form 0 = weak (advection/Maxwell), 1 = strong.  FP64
- * kernels use the symmetry of the operators under the reflection r <-> s of the
- * reference triangle where it holds (to 1e-13), and other kernels where it does
- * not: capture a graph of your own again after replacing symmetric operators by
- * ones without it (replayed as it was, it returns NaN). */
+ * __constant__ memory).  form 0 = weak (advection/Maxwell), 1 = strong.  Kernels
+ * use the symmetry of the operators under the reflection r <-> s of the reference
+ * triangle where it holds (to 1e-13), and other kernels run where it does not.  A
+ * graph of your own, captured before, gives the new operators' results too, but
+ * slower than captured again if the symmetry has changed. */
 int dgc_set_operators(dgc_handle h, int form, const double* Dr, const double* Ds, const double* L);
 
 /* Layout conversion between the native layout and the reference's CPU or
