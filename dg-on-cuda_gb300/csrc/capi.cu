@@ -849,14 +849,20 @@ int refresh_rhs_info(dgc_handle h) {
   return DGC_OK;
 }
 
+// Version of the variant table: raised when a variant's number comes to mean
+// another kernel or its code changes, so that a cache file written before is not
+// taken for this one (2: 6, and 2 at orders 7, 8, are the even / odd kernel).
+constexpr int kVariantTable = 2;
+
+// eo_ok: which kernel variant 6 (2) runs
 std::string tune_key(dgc_handle h) {
   cudaDeviceProp prop{};
   cudaGetDeviceProperties(&prop, h->device);
   int kb = 0;
   while ((1 << (kb + 1)) <= h->K) ++kb;  // K bucket: floor(log2 K)
-  char buf[sizeof prop.name + 96];  // the device name can fill its 256 bytes
-  std::snprintf(buf, sizeof buf, "%s|sm%d|phys%d|prec%d|N%d|K2^%d", prop.name, prop.multiProcessorCount,
-                h->desc.physics, h->prec, h->N, kb);
+  char buf[sizeof prop.name + 128];  // the device name can fill its 256 bytes
+  std::snprintf(buf, sizeof buf, "%s|sm%d|phys%d|prec%d|N%d|K2^%d|eo%d|table%d", prop.name, prop.multiProcessorCount,
+                h->desc.physics, h->prec, h->N, kb, h->eo_ok[0] ? 1 : 0, kVariantTable);
   for (char* c = buf; *c; ++c)
     if (*c == ' ') *c = '_';
   return buf;
@@ -867,9 +873,9 @@ int cache_lookup(const std::string& key) {
   if (!path || !*path) return -1;
   FILE* f = std::fopen(path, "r");
   if (!f) return -1;
-  char k[300];
+  char k[400];
   int v, found = -1;
-  while (std::fscanf(f, "%299s %d", k, &v) == 2)
+  while (std::fscanf(f, "%399s %d", k, &v) == 2)
     if (key == k) found = v;  // last entry wins
   std::fclose(f);
   return found;

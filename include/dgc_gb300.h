@@ -594,8 +594,9 @@ int dgc_set_variant(dgc_handle h, int v);
  * times_ms (optional, dgc_num_variants entries) receives the median time per
  * launch.  When times_ms is NULL and the file named by the environment
  * variable DGC_TUNE_CACHE holds a choice for this (GPU, physics, precision,
- * order, log2 K) key, that choice is applied without timing; new choices are
- * appended to that file.  Synchronises the stream. */
+ * order, log2 K, symmetry of the operators, version of the variant table) key,
+ * that choice is applied without timing; new choices are appended to that file.
+ * Synchronises the stream. */
 int dgc_autotune(dgc_handle h, int reps, double* times_ms, int* chosen, void* stream);
 
 /* ---- host-only set-up queries (no GPU needed) ---------------------------- */
