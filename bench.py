@@ -959,6 +959,30 @@ def measure_equal_error(dg, meshes):
             "same_error_configs": same, "min_error": best, "time_to_error": frontier}
 
 
+# sections of the output line that are printed whole
+WHOLE = ("config", "e2e", "roofline", "cpu_baseline", "clocks", "accuracy")
+
+
+def brief(section, depth=0):
+    """A section's figures without its lists, long texts and what lies deeper than
+    two levels; floats to 6 digits."""
+    if isinstance(section, float):
+        return float("%.6g" % section)
+    if not isinstance(section, dict):
+        return section
+    return {k: brief(v, depth + 1) for k, v in section.items()
+            if not isinstance(v, list) and not (isinstance(v, str) and len(v) > 80)
+            and not (isinstance(v, dict) and depth == 2)}
+
+
+def print_result(line):
+    """The result as one JSON line on stdout, of a few KB (the whole sweep's rows made
+    it 23 KB, too long for readers that keep the end of the output); every section
+    whole as one JSON line on stderr."""
+    print(json.dumps({"details": line}), file=sys.stderr)
+    print(json.dumps({k: v if k in WHOLE or not isinstance(v, dict) else brief(v) for k, v in line.items()}))
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -1157,7 +1181,7 @@ def main():
                 "speedup_mixed_vs_fp64": (value / ws / fp64["value"]) if fp64 else None,
                 "accuracy": accuracy, "poisson": poisson, "batched": batched, "learned_precond": learned,
                 "stokes": stokes, "advection": advection, "equal_error": equal_error, "wall_s_timed_region": wall}
-        print(json.dumps(line))
+        print_result(line)
     if ws > 1:
         import torch.distributed as tdist
         tdist.destroy_process_group()
