@@ -47,9 +47,9 @@ STAGE_KERNELS = {
     2: "dgk::dg_rhs_v2_kernel<6,PHYS_TE,4,8>",
     3: "dgk::dg_rhs_v2_kernel<6,PHYS_TE,4,4>",
     4: "dgk::dg_rhs_tc_kernel<6,PHYS_TE> (tcgen05, split TF32)",
-    5: "dgk::dg_rhs_blk_kernel<6,PHYS_TE,1>",
+    5: "dgk::dg_rhs_blk_kernel<6,PHYS_TE>",
     6: "dgk::dg_rhs_sym_kernel<6,PHYS_TE> (even / odd operators, one element per lane)",
-    7: "dgk::dg_rhs_blk_kernel<6,PHYS_TE,1> (warp-uniform operator loads)",
+    7: "dgk::dg_rhs_blk_kernel<6,PHYS_TE> (warp-uniform operator loads)",
     8: "dgk::dg_rhs_tct_kernel<6,PHYS_TE> (tcgen05, A in TMEM, split TF32)",
     9: "dgk::dg_rhs_tcp_kernel<6,PHYS_TE> (tcgen05, A in TMEM, warp-specialized pipeline)",
 }

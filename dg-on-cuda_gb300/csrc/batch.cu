@@ -67,8 +67,8 @@ template <int N, int P>
 __device__ __noinline__ bool batch_item_blk(const RhsParams& p, unsigned char* smem, uint32_t* ph, int tile0,
                                             int ntile) {
   uint32_t loc[3] = {ph[0], ph[1], ph[2]};
-  const bool ok = blk_tiles<N, P, 1, 0, false>(p, smem, loc, tile0, 1, tile0 + ntile,
-                                               TileRun{p.K, BlkConfig<N, P, 1, 0>::TE});
+  const bool ok = blk_tiles<N, P, 0, false>(p, smem, loc, tile0, 1, tile0 + ntile,
+                                               TileRun{p.K, BlkConfig<N, P>::TE});
   ph[0] = loc[0];
   ph[1] = loc[1];
   ph[2] = loc[2];
@@ -79,9 +79,9 @@ __device__ __noinline__ bool batch_item_blk(const RhsParams& p, unsigned char* s
 constexpr uint32_t umax(uint32_t a, uint32_t b) { return a > b ? a : b; }
 template <int N>
 constexpr uint32_t batch_smem_upto() {
-  constexpr uint32_t a = umax(RhsConfig<float, N, PHYS_ADV>::kSmem, BlkConfig<N, PHYS_ADV, 1, 0>::kSmem),
-                     b = umax(RhsConfig<float, N, PHYS_TM>::kSmem, BlkConfig<N, PHYS_TM, 1, 0>::kSmem),
-                     c = umax(RhsConfig<float, N, PHYS_TE>::kSmem, BlkConfig<N, PHYS_TE, 1, 0>::kSmem);
+  constexpr uint32_t a = umax(RhsConfig<float, N, PHYS_ADV>::kSmem, BlkConfig<N, PHYS_ADV>::kSmem),
+                     b = umax(RhsConfig<float, N, PHYS_TM>::kSmem, BlkConfig<N, PHYS_TM>::kSmem),
+                     c = umax(RhsConfig<float, N, PHYS_TE>::kSmem, BlkConfig<N, PHYS_TE>::kSmem);
   constexpr uint32_t m = umax(a, umax(b, c));
   if constexpr (N == 1) {
     return m;

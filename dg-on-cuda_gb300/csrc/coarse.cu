@@ -100,14 +100,10 @@ __global__ void k_coarse_axpy(int64_t n, const double* x, double w, const double
   }
 }
 
-// FP32 copy of an FP64 vector, and back
+// FP32 copy of an FP64 vector
 __global__ void k_coarse_to_f32(int64_t n, const double* __restrict__ x, float* __restrict__ y) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     y[i] = (float)x[i];
-}
-__global__ void k_coarse_to_f64(int64_t n, const float* __restrict__ x, double* __restrict__ y) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    y[i] = (double)x[i];
 }
 
 // FP32 copy of an n x n matrix with rows padded to lda
@@ -363,16 +359,12 @@ __global__ void k_coarse_prolong32(int64_t nq, int npp, int np, const int32_t* _
   }
 }
 
-// z[k][j] (+)= xc[agg[k]] on the valid nodes
+// z[k][j] = xc[agg[k]] on the valid nodes, 0 on the others
 __global__ void k_coarse_prolong(int64_t n, int npp, int np, const int32_t* __restrict__ agg,
-                                 const double* __restrict__ xc, int add, double* __restrict__ z,
-                                 float* __restrict__ z32) {
+                                 const double* __restrict__ xc, double* __restrict__ z) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t k = i / npp;
-    const double v = (int)(i - k * npp) < np ? xc[agg[k]] : 0.0;
-    const double o = add ? z[i] + v : v;
-    z[i] = o;
-    if (z32) z32[i] = (float)o;  // the next FP32 operator apply's input
+    z[i] = (int)(i - k * npp) < np ? xc[agg[k]] : 0.0;
   }
 }
 
@@ -728,7 +720,7 @@ int dgc::coarse_apply(dgc_handle_s* h, const double* r, const double* binv_r, do
                                                                   nullptr, 0.0, c->d_rc, nullptr, nullptr);
   dgk::k_coarse_gemv<<<(c->nagg * 32 + 255) / 256, 256, 0, s>>>(c->nagg, c->d_ainv, c->d_rc, c->d_xc);
   // y = P0 x_c;  z (+)= y - w Binv S y
-  dgk::k_coarse_prolong<<<grid1(n), 256, 0, s>>>(n, h->NpP, h->Np, c->d_agg, c->d_xc, 0, w1, nullptr);
+  dgk::k_coarse_prolong<<<grid1(n), 256, 0, s>>>(n, h->NpP, h->Np, c->d_agg, c->d_xc, w1);
   CKC(cudaGetLastError(), "apply");
   if (int rc = dgc_laplace_spd_apply(h, w1, w2, s)) return rc;
   if (int rc = ipdg_block_jacobi_apply(h, w2, w0, s)) return rc;

@@ -7,15 +7,14 @@
 //   rhs_c[i] = sum_c' (Gr_cc' ur_c'[i] + Gs_cc' us_c'[i]) + sum_m LIFT[i][m] g_c[m],
 //   ur_c' = Dr q_c',  us_c' = Ds q_c',  g_c = -(faceJ / J) f*_c  (face flux),
 // with Gr, Gs the physics' combination of rx, ry, sx, sy.  Thread (slot s,
-// group g) owns nodes 4g .. 4g+3 of EPT elements of the tile (elements s and
-// s + NTE) and all their fields:
+// group g) owns nodes 4g .. 4g+3 of element s of the tile and all its fields:
 //   * the element's field values are read 4 columns at a time (float4), the
 //     operators as rows of the transposed matrices padded to NpP columns, so
 //     one float4 of Dr^T / Ds^T / LIFT^T row j covers the thread's 4 nodes;
 //   * Maxwell: the curl of the first two fields is accumulated as one
 //     product pair Dr u + Ds v, u and v their combination with the element's
 //     (constant) rx, ry, sx, sy, next to Dr q2 and Ds q2 for the gradient of
-//     the third field: 3 x 4 x EPT accumulators and 4 FMAs per node and
+//     the third field: 3 x 4 accumulators and 4 FMAs per node and
 //     column instead of 6 (advection: Dr q and Ds q);
 //   * the face fluxes are stored already scaled by -faceJ/J so LIFT
 //     accumulates straight into rhs;
@@ -35,27 +34,24 @@
 
 namespace dgk {
 
-template <int N, int P, int EPT_, int MAP_ = 0>
+template <int N, int P, int MAP_ = 0>
 struct BlkConfig {
   using O = Order<N>;
   static constexpr int Np = O::Np, NpP = O::NpP, NFACE = O::Nface;
-  static constexpr int EPT = EPT_, MAP = MAP_;
+  static constexpr int MAP = MAP_;
   static constexpr int NG = NpP / 4;                 // 4-node groups per element
   static constexpr int RW = (8 / NG) > 0 ? 8 / NG : 1;  // MAP 1: rows of 32 elements per CTA
   static constexpr int kThreads = MAP == 0 ? 256 : NG * 32 * RW;
-  static constexpr int kMinBlocks = EPT == 2 ? 2 : 3;
-  static constexpr int NTE = MAP == 0 ? kThreads / NG : 32 * RW;  // element slots per CTA
-  static constexpr int TE = NTE * EPT;               // elements per tile
+  static constexpr int kMinBlocks = 3;
+  static constexpr int TE = MAP == 0 ? kThreads / NG : 32 * RW;  // elements per tile
   static constexpr int Nf = PhysTraits<P>::Nf;
   static constexpr int ESTR = Nf * NpP;              // state stride per element
   static constexpr int FSTR = (NFACE + 3) / 4 * 4;   // padded face-flux row
   static constexpr int kFItems = (TE * O::Nfp + kThreads - 1) / kThreads;  // (element, face-node) items per thread
   static constexpr int KB = 2 * Np + NFACE;          // operator rows: Dr^T | Ds^T | LIFT^T
   static constexpr uint32_t kMat = KB * NpP * 4;
-  // the LSERK residual tile is prefetched with the state tile when the extra
-  // buffers keep the CTA count per SM (one element per thread)
-  static constexpr bool kAuxTile = EPT == 1;
-  static constexpr uint32_t kQ = TE * ESTR * 4, kA = kAuxTile ? kQ : 0, kG = TE * 16 * 4, kN = TE * 16;
+  // the LSERK residual tile is prefetched with the state tile
+  static constexpr uint32_t kQ = TE * ESTR * 4, kA = kQ, kG = TE * 16 * 4, kN = TE * 16;
   static constexpr uint32_t kBuf = kQ + kA + kG + kN;  // one tile buffer: state | residual | geometry | neighbours
   static constexpr uint32_t oBar = 0;
   static constexpr uint32_t oMats = 32;
@@ -87,12 +83,12 @@ __device__ __forceinline__ float f4c(const float4& v, int i) {
 // tile's faces and two barriers, in tiles without a boundary too: see rhs_blk for
 // where it pays; the batched launch has other work to run beside the exponentials
 // and lost up to 5 % by it (24 instances: 382 us per step with it, 367 without).
-template <int N, int P, int EPT_, int MAP_, bool LIST, typename Cut>
+template <int N, int P, int MAP_, bool LIST, typename Cut>
 __device__ __forceinline__ bool blk_tiles(const RhsParams& p, unsigned char* smem, uint32_t (&ph)[3], int t0,
                                           int tstep, int tend, const Cut& tiles) {
-  using C = BlkConfig<N, P, EPT_, MAP_>;
+  using C = BlkConfig<N, P, MAP_>;
   constexpr int Np = C::Np, NpP = C::NpP, NFACE = C::NFACE, Nfp = Order<N>::Nfp;
-  constexpr int EPT = C::EPT, NG = C::NG, NTE = C::NTE, TE = C::TE, NF = C::Nf, ESTR = C::ESTR;
+  constexpr int NG = C::NG, TE = C::TE, NF = C::Nf, ESTR = C::ESTR;
   constexpr int FSTR = C::FSTR, NT = C::kThreads;
 
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + C::oBar);  // [0], [1]: tile buffers, [2]: operators
@@ -104,7 +100,7 @@ __device__ __forceinline__ bool blk_tiles(const RhsParams& p, unsigned char* sme
   auto bufN = [&](int b) {
     return reinterpret_cast<int4*>(smem + C::oBuf + b * C::kBuf + C::kQ + C::kA + C::kG);
   };
-  const bool aux_tile = C::kAuxTile && p.mode == MODE_LSERK;
+  const bool aux_tile = p.mode == MODE_LSERK;
   int* bcount = reinterpret_cast<int*>(smem + C::oBnd);
   uint16_t* blist = reinterpret_cast<uint16_t*>(bcount + 4);
 
@@ -159,47 +155,37 @@ __device__ __forceinline__ bool blk_tiles(const RhsParams& p, unsigned char* sme
     const float* sG = bufG(b);
     const int4* sN = bufN(b);
 
-    // ---- volume: nodes 4 grp .. 4 grp + 3 of elements slot, slot + NTE.  It
-    //      needs no face data, so it runs first and the face phase's neighbour
-    //      gathers of some warps overlap the volume products of others.
-    float rh[EPT][NF][4];
-    if (slot < NTE) {
+    // ---- volume: nodes 4 grp .. 4 grp + 3 of element slot.  It needs no face data,
+    //      so it runs first and the face phase's neighbour gathers of some warps
+    //      overlap the volume products of others.
+    float rh[NF][4];
+    if (slot < TE) {
       const float* bR = sB + 4 * grp;           // Dr^T row j at bR + j NpP
       const float* bS = bR + Np * NpP;          // Ds^T
       if constexpr (P == PHYS_ADV) {
-        float ur[EPT][4], us[EPT][4];
+        float ur[4], us[4];
 #pragma unroll
-        for (int l = 0; l < EPT; ++l)
-#pragma unroll
-          for (int n = 0; n < 4; ++n) ur[l][n] = us[l][n] = 0.0f;
+        for (int n = 0; n < 4; ++n) ur[n] = us[n] = 0.0f;
 #pragma unroll
         for (int j0 = 0; j0 < Np; j0 += 4) {
-          float4 a[EPT];
-#pragma unroll
-          for (int l = 0; l < EPT; ++l) a[l] = *reinterpret_cast<const float4*>(sQ + (slot + l * NTE) * ESTR + j0);
+          const float4 a = *reinterpret_cast<const float4*>(sQ + slot * ESTR + j0);
 #pragma unroll
           for (int jj = 0; jj < 4; ++jj) {
             if (j0 + jj >= Np) break;
             const float4 br = *reinterpret_cast<const float4*>(bR + (j0 + jj) * NpP);
             const float4 bs = *reinterpret_cast<const float4*>(bS + (j0 + jj) * NpP);
-#pragma unroll
-            for (int l = 0; l < EPT; ++l) {
-              const float v = f4c(a[l], jj);
-              ur[l][0] = fmaf(br.x, v, ur[l][0]); us[l][0] = fmaf(bs.x, v, us[l][0]);
-              ur[l][1] = fmaf(br.y, v, ur[l][1]); us[l][1] = fmaf(bs.y, v, us[l][1]);
-              ur[l][2] = fmaf(br.z, v, ur[l][2]); us[l][2] = fmaf(bs.z, v, us[l][2]);
-              ur[l][3] = fmaf(br.w, v, ur[l][3]); us[l][3] = fmaf(bs.w, v, us[l][3]);
-            }
+            const float v = f4c(a, jj);
+            ur[0] = fmaf(br.x, v, ur[0]); us[0] = fmaf(bs.x, v, us[0]);
+            ur[1] = fmaf(br.y, v, ur[1]); us[1] = fmaf(bs.y, v, us[1]);
+            ur[2] = fmaf(br.z, v, ur[2]); us[2] = fmaf(bs.z, v, us[2]);
+            ur[3] = fmaf(br.w, v, ur[3]); us[3] = fmaf(bs.w, v, us[3]);
           }
         }
+        const float4 g0 = *reinterpret_cast<const float4*>(sG + slot * 16);  // rx ry sx sy
 #pragma unroll
-        for (int l = 0; l < EPT; ++l) {
-          const float4 g0 = *reinterpret_cast<const float4*>(sG + (slot + l * NTE) * 16);  // rx ry sx sy
-#pragma unroll
-          for (int n = 0; n < 4; ++n) {
-            const float dx = g0.x * ur[l][n] + g0.z * us[l][n], dy = g0.y * ur[l][n] + g0.w * us[l][n];
-            rh[l][0][n] = cax * dx + cay * dy;
-          }
+        for (int n = 0; n < 4; ++n) {
+          const float dx = g0.x * ur[n] + g0.z * us[n], dy = g0.y * ur[n] + g0.w * us[n];
+          rh[0][n] = cax * dx + cay * dy;
         }
       } else {
         // Maxwell: the curl term of the third field is one product pair,
@@ -208,57 +194,45 @@ __device__ __forceinline__ bool blk_tiles(const RhsParams& p, unsigned char* sme
         //   TE  Hz' = Dx Ey - Dy Ex = Dr (rx Ey - ry Ex) + Ds (sx Ey - sy Ex),
         //   TM  Ez' = Dy Hx - Dx Hy = Dr (ry Hx - rx Hy) + Ds (sy Hx - sx Hy);
         // the gradient of the third field needs Dr q2 and Ds q2.
-        float gr[EPT][4], gs[EPT][4], cu[EPT][4];
-        float4 g0[EPT];
+        float gr[4], gs[4], cu[4];
+        const float4 g0 = *reinterpret_cast<const float4*>(sG + slot * 16);  // rx ry sx sy
 #pragma unroll
-        for (int l = 0; l < EPT; ++l) {
-          g0[l] = *reinterpret_cast<const float4*>(sG + (slot + l * NTE) * 16);  // rx ry sx sy
-#pragma unroll
-          for (int n = 0; n < 4; ++n) gr[l][n] = gs[l][n] = cu[l][n] = 0.0f;
-        }
+        for (int n = 0; n < 4; ++n) gr[n] = gs[n] = cu[n] = 0.0f;
 #pragma unroll
         for (int j0 = 0; j0 < Np; j0 += 4) {
-          float4 a[EPT][NF];
+          float4 a[NF];
 #pragma unroll
-          for (int l = 0; l < EPT; ++l)
-#pragma unroll
-            for (int c = 0; c < NF; ++c)
-              a[l][c] = *reinterpret_cast<const float4*>(sQ + (slot + l * NTE) * ESTR + c * NpP + j0);
+          for (int c = 0; c < NF; ++c)
+            a[c] = *reinterpret_cast<const float4*>(sQ + slot * ESTR + c * NpP + j0);
 #pragma unroll
           for (int jj = 0; jj < 4; ++jj) {
             if (j0 + jj >= Np) break;
             const float4 br = *reinterpret_cast<const float4*>(bR + (j0 + jj) * NpP);
             const float4 bs = *reinterpret_cast<const float4*>(bS + (j0 + jj) * NpP);
-#pragma unroll
-            for (int l = 0; l < EPT; ++l) {
-              const float q0 = f4c(a[l][0], jj), q1 = f4c(a[l][1], jj), v = f4c(a[l][2], jj);
-              const float u = (P == PHYS_TE) ? g0[l].x * q1 - g0[l].y * q0 : g0[l].y * q0 - g0[l].x * q1;
-              const float w = (P == PHYS_TE) ? g0[l].z * q1 - g0[l].w * q0 : g0[l].w * q0 - g0[l].z * q1;
-              gr[l][0] = fmaf(br.x, v, gr[l][0]); gs[l][0] = fmaf(bs.x, v, gs[l][0]);
-              gr[l][1] = fmaf(br.y, v, gr[l][1]); gs[l][1] = fmaf(bs.y, v, gs[l][1]);
-              gr[l][2] = fmaf(br.z, v, gr[l][2]); gs[l][2] = fmaf(bs.z, v, gs[l][2]);
-              gr[l][3] = fmaf(br.w, v, gr[l][3]); gs[l][3] = fmaf(bs.w, v, gs[l][3]);
-              cu[l][0] = fmaf(br.x, u, fmaf(bs.x, w, cu[l][0]));
-              cu[l][1] = fmaf(br.y, u, fmaf(bs.y, w, cu[l][1]));
-              cu[l][2] = fmaf(br.z, u, fmaf(bs.z, w, cu[l][2]));
-              cu[l][3] = fmaf(br.w, u, fmaf(bs.w, w, cu[l][3]));
-            }
+            const float q0 = f4c(a[0], jj), q1 = f4c(a[1], jj), v = f4c(a[2], jj);
+            const float u = (P == PHYS_TE) ? g0.x * q1 - g0.y * q0 : g0.y * q0 - g0.x * q1;
+            const float w = (P == PHYS_TE) ? g0.z * q1 - g0.w * q0 : g0.w * q0 - g0.z * q1;
+            gr[0] = fmaf(br.x, v, gr[0]); gs[0] = fmaf(bs.x, v, gs[0]);
+            gr[1] = fmaf(br.y, v, gr[1]); gs[1] = fmaf(bs.y, v, gs[1]);
+            gr[2] = fmaf(br.z, v, gr[2]); gs[2] = fmaf(bs.z, v, gs[2]);
+            gr[3] = fmaf(br.w, v, gr[3]); gs[3] = fmaf(bs.w, v, gs[3]);
+            cu[0] = fmaf(br.x, u, fmaf(bs.x, w, cu[0]));
+            cu[1] = fmaf(br.y, u, fmaf(bs.y, w, cu[1]));
+            cu[2] = fmaf(br.z, u, fmaf(bs.z, w, cu[2]));
+            cu[3] = fmaf(br.w, u, fmaf(bs.w, w, cu[3]));
           }
         }
+        const float rx = g0.x, ry = g0.y, sx = g0.z, sy = g0.w;
 #pragma unroll
-        for (int l = 0; l < EPT; ++l) {
-          const float rx = g0[l].x, ry = g0[l].y, sx = g0[l].z, sy = g0[l].w;
-#pragma unroll
-          for (int n = 0; n < 4; ++n) {
-            if (P == PHYS_TM) {  // Hx' = Dy Ez, Hy' = -Dx Ez
-              rh[l][0][n] = ry * gr[l][n] + sy * gs[l][n];
-              rh[l][1][n] = -(rx * gr[l][n] + sx * gs[l][n]);
-            } else {             // Ex' = -Dy Hz, Ey' = Dx Hz
-              rh[l][0][n] = -(ry * gr[l][n] + sy * gs[l][n]);
-              rh[l][1][n] = rx * gr[l][n] + sx * gs[l][n];
-            }
-            rh[l][2][n] = cu[l][n];
+        for (int n = 0; n < 4; ++n) {
+          if (P == PHYS_TM) {  // Hx' = Dy Ez, Hy' = -Dx Ez
+            rh[0][n] = ry * gr[n] + sy * gs[n];
+            rh[1][n] = -(rx * gr[n] + sx * gs[n]);
+          } else {             // Ex' = -Dy Hz, Ey' = Dx Hz
+            rh[0][n] = -(ry * gr[n] + sy * gs[n]);
+            rh[1][n] = rx * gr[n] + sx * gs[n];
           }
+          rh[2][n] = cu[n];
         }
       }
     }
@@ -371,31 +345,27 @@ __device__ __forceinline__ bool blk_tiles(const RhsParams& p, unsigned char* sme
     if (P == PHYS_ADV && tid == 0) *bcount = 0;
 
     // ---- lift + epilogue
-    if (slot < NTE) {
+    if (slot < TE) {
       const float* bL = sB + 4 * grp + 2 * Np * NpP;  // LIFT^T row m at bL + m NpP
       // lift of the scaled face fluxes
 #pragma unroll
       for (int m0 = 0; m0 < NFACE; m0 += 4) {
-        float4 fv[EPT][NF];
+        float4 fv[NF];
 #pragma unroll
-        for (int l = 0; l < EPT; ++l)
-#pragma unroll
-          for (int c = 0; c < NF; ++c)
-            fv[l][c] = *reinterpret_cast<const float4*>(sF + (slot + l * NTE) * NF * FSTR + c * FSTR + m0);
+        for (int c = 0; c < NF; ++c)
+          fv[c] = *reinterpret_cast<const float4*>(sF + slot * NF * FSTR + c * FSTR + m0);
 #pragma unroll
         for (int mm = 0; mm < 4; ++mm) {
           if (m0 + mm >= NFACE) break;
           const float4 bl = *reinterpret_cast<const float4*>(bL + (m0 + mm) * NpP);
 #pragma unroll
-          for (int l = 0; l < EPT; ++l)
-#pragma unroll
-            for (int c = 0; c < NF; ++c) {
-              const float v = f4c(fv[l][c], mm);
-              rh[l][c][0] = fmaf(bl.x, v, rh[l][c][0]);
-              rh[l][c][1] = fmaf(bl.y, v, rh[l][c][1]);
-              rh[l][c][2] = fmaf(bl.z, v, rh[l][c][2]);
-              rh[l][c][3] = fmaf(bl.w, v, rh[l][c][3]);
-            }
+          for (int c = 0; c < NF; ++c) {
+            const float v = f4c(fv[c], mm);
+            rh[c][0] = fmaf(bl.x, v, rh[c][0]);
+            rh[c][1] = fmaf(bl.y, v, rh[c][1]);
+            rh[c][2] = fmaf(bl.z, v, rh[c][2]);
+            rh[c][3] = fmaf(bl.w, v, rh[c][3]);
+          }
         }
       }
       // ---- epilogue, 4 nodes of one element-field per float4
@@ -405,48 +375,43 @@ __device__ __forceinline__ bool blk_tiles(const RhsParams& p, unsigned char* sme
       // lanes of the last group past Np are padding: written as 0
       const int nvalid = Np - 4 * grp;
 #pragma unroll
-      for (int l = 0; l < EPT; ++l) {
-        const int e = slot + l * NTE;
-        if (e >= ne) break;
-#pragma unroll
-        for (int c = 0; c < NF; ++c) {
-          const size_t o = (size_t)(k0 + e) * ESTR + c * NpP + 4 * grp;
-          float4 r = make_float4(rh[l][c][0], rh[l][c][1], rh[l][c][2], rh[l][c][3]);
-          const float4 qv = *reinterpret_cast<const float4*>(sQ + e * ESTR + c * NpP + 4 * grp);
-          float4 w0 = r, w1 = r;  // values for out (w0) and aux / q0 (w1)
-          bool wr_aux = true, wr_q0 = false, wr_out = true;
-          if (p.mode == MODE_RHS) {
-            wr_aux = false;
-          } else if (p.mode == MODE_LSERK) {
-            const float4 av4 = aux_tile ? *reinterpret_cast<const float4*>(sA + e * ESTR + c * NpP + 4 * grp)
-                                        : *reinterpret_cast<const float4*>(aux + o);
-            w1 = make_float4(cca * av4.x + cdt * r.x, cca * av4.y + cdt * r.y, cca * av4.z + cdt * r.z,
-                             cca * av4.w + cdt * r.w);
-            w0 = make_float4(qv.x + ccb * w1.x, qv.y + ccb * w1.y, qv.z + ccb * w1.z, qv.w + ccb * w1.w);
-          } else if (p.stage == 0) {  // classical RK4, first stage
-            w1 = r;
-            w0 = make_float4(qv.x + cca * r.x, qv.y + cca * r.y, qv.z + cca * r.z, qv.w + cca * r.w);
-          } else if (p.stage < 3) {
-            const float4 av4 = *reinterpret_cast<const float4*>(aux + o);
-            const float4 b4 = *reinterpret_cast<const float4*>(q0 + o);
-            w1 = make_float4(av4.x + ccb * r.x, av4.y + ccb * r.y, av4.z + ccb * r.z, av4.w + ccb * r.w);
-            w0 = make_float4(b4.x + cca * r.x, b4.y + cca * r.y, b4.z + cca * r.z, b4.w + cca * r.w);
-          } else {                    // last stage updates the base state only
-            const float4 av4 = *reinterpret_cast<const float4*>(aux + o);
-            const float4 b4 = *reinterpret_cast<const float4*>(q0 + o);
-            w1 = make_float4(b4.x + cca * (av4.x + r.x), b4.y + cca * (av4.y + r.y), b4.z + cca * (av4.z + r.z),
-                             b4.w + cca * (av4.w + r.w));
-            wr_aux = false;
-            wr_q0 = true;
-            wr_out = false;
-          }
-          if (nvalid < 4) { w0.w = 0.0f; w1.w = 0.0f; }
-          if (nvalid < 3) { w0.z = 0.0f; w1.z = 0.0f; }
-          if (nvalid < 2) { w0.y = 0.0f; w1.y = 0.0f; }
-          if (wr_out) *reinterpret_cast<float4*>(out + o) = w0;
-          if (wr_aux) *reinterpret_cast<float4*>(aux + o) = w1;
-          if (wr_q0) *reinterpret_cast<float4*>(q0 + o) = w1;
+      for (int c = 0; c < NF; ++c) {
+        if (slot >= ne) break;
+        const size_t o = (size_t)(k0 + slot) * ESTR + c * NpP + 4 * grp;
+        float4 r = make_float4(rh[c][0], rh[c][1], rh[c][2], rh[c][3]);
+        const float4 qv = *reinterpret_cast<const float4*>(sQ + slot * ESTR + c * NpP + 4 * grp);
+        float4 w0 = r, w1 = r;  // values for out (w0) and aux / q0 (w1)
+        bool wr_aux = true, wr_q0 = false, wr_out = true;
+        if (p.mode == MODE_RHS) {
+          wr_aux = false;
+        } else if (p.mode == MODE_LSERK) {
+          const float4 av4 = *reinterpret_cast<const float4*>(sA + slot * ESTR + c * NpP + 4 * grp);
+          w1 = make_float4(cca * av4.x + cdt * r.x, cca * av4.y + cdt * r.y, cca * av4.z + cdt * r.z,
+                           cca * av4.w + cdt * r.w);
+          w0 = make_float4(qv.x + ccb * w1.x, qv.y + ccb * w1.y, qv.z + ccb * w1.z, qv.w + ccb * w1.w);
+        } else if (p.stage == 0) {  // classical RK4, first stage
+          w1 = r;
+          w0 = make_float4(qv.x + cca * r.x, qv.y + cca * r.y, qv.z + cca * r.z, qv.w + cca * r.w);
+        } else if (p.stage < 3) {
+          const float4 av4 = *reinterpret_cast<const float4*>(aux + o);
+          const float4 b4 = *reinterpret_cast<const float4*>(q0 + o);
+          w1 = make_float4(av4.x + ccb * r.x, av4.y + ccb * r.y, av4.z + ccb * r.z, av4.w + ccb * r.w);
+          w0 = make_float4(b4.x + cca * r.x, b4.y + cca * r.y, b4.z + cca * r.z, b4.w + cca * r.w);
+        } else {                    // last stage updates the base state only
+          const float4 av4 = *reinterpret_cast<const float4*>(aux + o);
+          const float4 b4 = *reinterpret_cast<const float4*>(q0 + o);
+          w1 = make_float4(b4.x + cca * (av4.x + r.x), b4.y + cca * (av4.y + r.y), b4.z + cca * (av4.z + r.z),
+                           b4.w + cca * (av4.w + r.w));
+          wr_aux = false;
+          wr_q0 = true;
+          wr_out = false;
         }
+        if (nvalid < 4) { w0.w = 0.0f; w1.w = 0.0f; }
+        if (nvalid < 3) { w0.z = 0.0f; w1.z = 0.0f; }
+        if (nvalid < 2) { w0.y = 0.0f; w1.y = 0.0f; }
+        if (wr_out) *reinterpret_cast<float4*>(out + o) = w0;
+        if (wr_aux) *reinterpret_cast<float4*>(aux + o) = w1;
+        if (wr_q0) *reinterpret_cast<float4*>(q0 + o) = w1;
       }
     }
     __syncthreads();
@@ -454,10 +419,10 @@ __device__ __forceinline__ bool blk_tiles(const RhsParams& p, unsigned char* sme
   return true;
 }
 
-template <int N, int P, int EPT_, int MAP_, bool LIST>
-__global__ void __launch_bounds__(BlkConfig<N, P, EPT_, MAP_>::kThreads, BlkConfig<N, P, EPT_, MAP_>::kMinBlocks)
+template <int N, int P, int MAP_, bool LIST>
+__global__ void __launch_bounds__(BlkConfig<N, P, MAP_>::kThreads, BlkConfig<N, P, MAP_>::kMinBlocks)
     dg_rhs_blk_kernel(const RhsParams p) {
-  using C = BlkConfig<N, P, EPT_, MAP_>;
+  using C = BlkConfig<N, P, MAP_>;
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + C::oBar);
   if (threadIdx.x == 0) {
@@ -468,7 +433,7 @@ __global__ void __launch_bounds__(BlkConfig<N, P, EPT_, MAP_>::kThreads, BlkConf
   }
   __syncthreads();
   uint32_t ph[3] = {0, 0, 0};
-  blk_tiles<N, P, EPT_, MAP_, LIST>(p, smem, ph, blockIdx.x, gridDim.x, p.ntiles, TileCut(p.K, p.ntiles));
+  blk_tiles<N, P, MAP_, LIST>(p, smem, ph, blockIdx.x, gridDim.x, p.ntiles, TileCut(p.K, p.ntiles));
 }
 
 }  // namespace dgk

@@ -275,10 +275,10 @@ cudaError_t rhs_sym(const RhsParams* p, cudaStream_t s, LaunchInfo* info) {
   return launch_stage(dg_rhs_sym_kernel<N, P>, (p->K + C::TE - 1) / C::TE, C::kThreads, C::kSmem, s, *p);
 }
 
-template <int N, int P, int EPT, int MAP, bool LIST = true>
+template <int N, int P, int MAP, bool LIST = true>
 cudaError_t rhs_blk(const RhsParams* p, int sm_count, cudaStream_t s, LaunchInfo* info) {
-  using C = BlkConfig<N, P, EPT, MAP>;
-  auto kern = dg_rhs_blk_kernel<N, P, EPT, MAP, LIST>;
+  using C = BlkConfig<N, P, MAP>;
+  auto kern = dg_rhs_blk_kernel<N, P, MAP, LIST>;
   static std::once_flag once;
   static cudaError_t st = cudaSuccess;
   static int bps = 0;
@@ -304,7 +304,7 @@ cudaError_t rhs_blk(const RhsParams* p, int sm_count, cudaStream_t s, LaunchInfo
   // K = 9800 64.9 / 68.0 / 70.4, but K = 29768 146.9 / 142.5 / 140.4; N = 6 60.1 / 61.3 /
   // 67.7 at K = 20000 and 104.0 / 104.7 / 106.5 at K = 45000, lower orders more)
   if constexpr (P == PHYS_ADV && N >= 7 && LIST)
-    if (grid < q.ntiles) return rhs_blk<N, P, EPT, MAP, false>(p, sm_count, s, info);
+    if (grid < q.ntiles) return rhs_blk<N, P, MAP, false>(p, sm_count, s, info);
   return launch_stage(kern, grid, C::kThreads, C::kSmem, s, q);
 }
 
@@ -325,7 +325,7 @@ constexpr int kF32VariantsHigh = 4;
 // blocked kernel
 template <int N, int P>
 cudaError_t rhs_sym_or_blk(const RhsParams* p, int sm, cudaStream_t s, LaunchInfo* info) {
-  return info || p->mats_sym ? rhs_sym<N, P>(p, s, info) : rhs_blk<N, P, 1, 0>(p, sm, s, info);
+  return info || p->mats_sym ? rhs_sym<N, P>(p, s, info) : rhs_blk<N, P, 0>(p, sm, s, info);
 }
 
 template <int N, int P>
@@ -334,15 +334,15 @@ cudaError_t rhs_f32_variant(int v, const RhsParams* p, int sm, cudaStream_t s, L
   if constexpr (N <= 6) {
     if (v >= 1 && v <= 3) return rhs_v2<N, P>(v - 1, p, sm, s, info);
     if (v == 4) return rhs_tc<N, P>(p, sm, s, info);
-    if (v == 5) return rhs_blk<N, P, 1, 0>(p, sm, s, info);
+    if (v == 5) return rhs_blk<N, P, 0>(p, sm, s, info);
     if (v == 6) return rhs_sym_or_blk<N, P>(p, sm, s, info);
-    if (v == 7) return rhs_blk<N, P, 1, 1>(p, sm, s, info);
+    if (v == 7) return rhs_blk<N, P, 1>(p, sm, s, info);
     if (v == 8) return rhs_tct<N, P>(p, sm, s, info);
     if (v == 9) return rhs_tcp<N, P>(p, sm, s, info);
   } else {
-    if (v == 1) return rhs_blk<N, P, 1, 0>(p, sm, s, info);
+    if (v == 1) return rhs_blk<N, P, 0>(p, sm, s, info);
     if (v == 2) return rhs_sym_or_blk<N, P>(p, sm, s, info);
-    if (v == 3) return rhs_blk<N, P, 1, 1>(p, sm, s, info);
+    if (v == 3) return rhs_blk<N, P, 1>(p, sm, s, info);
   }
   return cudaErrorInvalidValue;
 }
