@@ -822,7 +822,7 @@ int dgc::two_level_pcg(dgc_handle_s* h, double* x, double* r, double tol2, int m
   while (rr > tol2 && !stop && it < maxit) {
     const int cur = it & 1;
     if (int rc = apply()) return rc;
-    if (!op32)  // the FP32 apply forms p.q while it converts q
+    if (!op32)  // the FP32 apply forms p.q
       if (int rc = dots({{p, nullptr, nullptr}, {q, nullptr, nullptr}})) return rc;
     // x += alpha p, r -= alpha q, z = Binv r
     BjFused st;

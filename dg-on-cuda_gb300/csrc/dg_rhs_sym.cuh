@@ -2,8 +2,8 @@
 // r <-> s (eo.hpp), one element per lane: the operator, fluxes and epilogues of
 // dg_rhs_blk.cuh.
 //
-// What bounds it: shared-memory wavefronts (one per cycle and SM), as in
-// dg_rhs_blk.cuh, whose operator loads alone take 8 of the ~11 wavefronts per
+// What it saves: shared-memory wavefronts (one per cycle and SM).  In
+// dg_rhs_blk.cuh the operator loads alone take 8 of the ~11 wavefronts per
 // operator column and warp: with the node groups of an element in consecutive
 // lanes a 16-byte operator load serves 8 lanes per wavefront.  Here
 //   * D+ / D- and the half-sized LIFT (eo.hpp) halve the operator columns;
@@ -11,7 +11,9 @@
 //     uniform (2 wavefronts for 4 rows x 32 elements) and an input load is one
 //     word per lane at an odd element stride (1 wavefront);
 //   * rows are sums only or differences only within a group.
-// Wavefronts per element, Maxwell N = 6: volume and LIFT 37 instead of 99.
+// Wavefronts per element, Maxwell N = 6: volume and LIFT 37 instead of 99.  What
+// bounds it then is the chain of a tile's phases: half of the issue slots and 46 %
+// of the wavefronts are in use.
 //
 // A CTA takes one tile of TE elements: bulk copy of state, geometry and neighbours;
 // exterior face values into registers; fluxes of face-node pairs and inputs of
@@ -21,10 +23,10 @@
 // slower than dg_rhs_blk.cuh's, which the batch keeps.
 //
 // us per stage, graphed, against the blocked kernel: advection K = 32768, N = 6
-// 12.0 / 16.2, N = 4 8.1 / 13.1, K = 20000, N = 8 14.5 / 24.4, K = 2048, N = 4 5.0 / 8.2
-// (boundary values evaluated by consecutive threads); Maxwell K = 32768, N = 6
-// 17.5 / 18.7, K = 12800, N = 7 14.3 / 18.0, N = 8 14.3 / 19.4, but N = 3 8.2 / 7.8
-// and K = 2048, N = 6 5.4 / 4.5: the autotuner decides.
+// 12.2 / 15.1, N = 4 7.9 / 11.7, K = 24200, N = 8 15.8 / 28.2, but K = 2048, N = 4
+// 5.0 / 5.0; Maxwell K = 32768, N = 6 17.8 / 18.9, N = 4 11.5 / 11.6, K = 12800, N = 7
+// 14.4 / 18.1, N = 8 14.8 / 19.5, but N = 3 6.2 / 4.7 and K = 2048, N = 6 5.6 / 4.4: the
+// autotuner decides.
 #pragma once
 
 #include <type_traits>

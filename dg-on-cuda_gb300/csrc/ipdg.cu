@@ -916,7 +916,8 @@ int cg_iteration(dgc_handle_s* h, int cgi, int slot, int first, cudaStream_t s) 
   p.p_old = wv<R>(h, W_P + (slot + 2) % 3);
   p.qx = wv<R>(h, W_QX);
   p.qy = wv<R>(h, W_QY);
-  // FP32: the register-blocked kernels (ipdg_blk.cuh); FP64: the one-node-per-thread ones
+  // FP32: the register-blocked kernels (ipdg_blk.cuh); FP64: the even / odd passes
+  // (ipdg_eo.cuh) or the one-node-per-thread ones, and pcg_update_kernel
   auto run = [&](int kind_r, int kind_blk) -> int {
     if (sizeof(R) == 4) {
       const cudaError_t e = dgk::ipdg_blk_launch(h->N, kind_blk, p, h->sm_count, s, true);

@@ -18,10 +18,11 @@ struct LaunchInfo {
 };
 
 // Launch of a stage kernel that calls grid_dep_wait before it touches the
-// previous launch's data (dg_rhs_blk_kernel, dg_rhs_tcp_kernel,
-// dg_rhs_x2_kernel, dg_batch_kernel, the FP32 CG kernels): with programmatic stream serialization its CTAs are
-// scheduled, and run their set-up (barriers, operator copies, tensor memory),
-// while the previous kernel of the stream finishes.  DGC_STAGE_OVERLAP=0 in the
+// previous launch's data (dg_rhs_blk_kernel, dg_rhs_sym_kernel,
+// dg_rhs_tcp_kernel, dg_rhs_x2_kernel, dg_batch_kernel, the FP32 CG kernels, and on
+// meshes of at most one tile per SM the FP64 even / odd kernels): with programmatic
+// stream serialization its CTAs are scheduled, and run their set-up (barriers,
+// operator copies, tensor memory), while the previous kernel of the stream finishes.  DGC_STAGE_OVERLAP=0 in the
 // environment launches them without the attribute.
 inline bool stage_overlap_enabled() {
   static const bool on = [] {
