@@ -738,13 +738,13 @@ int dgc::two_level_pcg(dgc_handle_s* h, double* x, double* r, double tol2, int m
   if (!c->d_pcg[0]) {
     for (double*& v : c->d_pcg) {
       CKC(cudaMalloc(&v, n * 8), "allocation");
-      CKC(cudaMemset(v, 0, n * 8), "clear");
+      CKC(zero_fill(v, n * 8), "clear");
     }
     // [0..2] dot products, [3] sums of the singular system, [4] p.q of the FP32 operator
     CKC(cudaMalloc(&c->d_dots, 5 * 8), "allocation");
-    CKC(cudaMemset(c->d_dots, 0, 5 * 8), "clear");
+    CKC(zero_fill(c->d_dots, 5 * 8), "clear");
     CKC(cudaMalloc(&c->d_q32, n * 4), "allocation");
-    CKC(cudaMemset(c->d_q32, 0, n * 4), "clear");
+    CKC(zero_fill(c->d_q32, n * 4), "clear");
     CKC(cudaMalloc(&c->d_sc, 8 * 8), "allocation");
     CKC(cudaMallocHost(&c->h_sc, 8 * 8), "allocation");
   }

@@ -74,6 +74,12 @@ void ipdg_operators_changed(dgc_handle_s* h);
 // (FP64 vectors; the blocks and sums in FP32 with fp32)
 int ipdg_build_preconditioner(dgc_handle_s* h, cudaStream_t s);
 int ipdg_block_jacobi_apply(dgc_handle_s* h, const double* r, double* z, cudaStream_t s);
+// clear a new work buffer, done when the call returns: a caller's stream does not
+// wait for the default one
+inline cudaError_t zero_fill(void* p, size_t bytes) {
+  const cudaError_t e = cudaMemset(p, 0, bytes);
+  return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+}
 // z = Binv r with the FP32 blocks; z32, when non-null, receives an FP32 copy of z
 int ipdg_block_jacobi_apply_f32(dgc_handle_s* h, const double* r, double* z, float* z32, cudaStream_t s);
 // the same as part of the two-level cycle, fused with the vector updates around it

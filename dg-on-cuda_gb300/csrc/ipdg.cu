@@ -1252,7 +1252,7 @@ extern "C" int dgc_laplace_bc_rhs(dgc_handle h, const double* g, const double* h
   const size_t n = nvec(h), esz = h->prec == DGC_F64 ? 8 : 4;
   if (jump && !st->qd) {  // zero off the boundary cells for good: only those are ever written
     CKI(cudaMalloc(&st->qd, 2 * n * esz));
-    CKI(cudaMemset(st->qd, 0, 2 * n * esz));
+    CKI(zero_fill(st->qd, 2 * n * esz));
   }
   cudaError_t e;
   auto run = [&](auto zero, void* const* mats) {

@@ -596,7 +596,7 @@ size_t field_len(const dgc_mpnn_s* m) { return (size_t)m->h->K * m->h->NpP; }
 template <typename T>
 cudaError_t zalloc(T** p, size_t count) {
   cudaError_t e = cudaMalloc(p, count * sizeof(T));
-  return e == cudaSuccess ? cudaMemset(*p, 0, count * sizeof(T)) : e;
+  return e == cudaSuccess ? dgc::zero_fill(*p, count * sizeof(T)) : e;
 }
 
 // device scalars (and their pinned host copy) for at least `count` doubles
@@ -803,7 +803,9 @@ extern "C" int dgc_mpnn_create(dgc_handle h, int layers, uint64_t seed, dgc_mpnn
     e = cudaFuncSetAttribute(dgk::k_layer_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dgk::MpnnTc::kSmem);
   if (e != cudaSuccess) return fail(mcuda(e, "mpnn set-up"));
   dgk::k_to_bf16<<<grid_for(m, P, 256), 256>>>(P, m->w, m->w16);
-  if ((e = cudaGetLastError()) != cudaSuccess) return fail(mcuda(e, "mpnn set-up"));
+  // the caller's stream does not wait for the default one
+  if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaStreamSynchronize(cudaStreamLegacy)) != cudaSuccess)
+    return fail(mcuda(e, "mpnn set-up"));
   *out = m;
   return DGC_OK;
 }

@@ -183,12 +183,12 @@ extern "C" int dgc_stokes_create(int num_vertices, const double* vertex_xy, int 
   const size_t nb = std::max<size_t>(1, (size_t)st->vel->mesh.num_bfaces * st->vel->Nfp);
   double** bufs[7] = {&st->ut[0], &st->ut[1], &st->work, &st->b, &st->grad[0], &st->grad[1], &st->p};
   for (double** q : bufs) {
-    if (cudaMalloc(q, st->n * 8) != cudaSuccess || cudaMemset(*q, 0, st->n * 8) != cudaSuccess) {
+    if (cudaMalloc(q, st->n * 8) != cudaSuccess || dgc::zero_fill(*q, st->n * 8) != cudaSuccess) {
       dgc_stokes_destroy(st);
       return set_error(DGC_ERR_CUDA, "stokes workspace allocation");
     }
   }
-  if (cudaMalloc(&st->h2, nb * 8) != cudaSuccess || cudaMemset(st->h2, 0, nb * 8) != cudaSuccess) {
+  if (cudaMalloc(&st->h2, nb * 8) != cudaSuccess || dgc::zero_fill(st->h2, nb * 8) != cudaSuccess) {
     dgc_stokes_destroy(st);
     return set_error(DGC_ERR_CUDA, "stokes workspace allocation");
   }
